@@ -93,16 +93,15 @@ int akv_set_tuning(const char* key, int value) {
     else if (!strcmp(key, "k_wpc") && value >= 0 && value <= 16) t.k_wpc = value;
     else if (!strcmp(key, "v_impl") && (value == 0 || value == 1)) t.v_impl = value;
     else if (!strcmp(key, "v_nf") && value >= 0 && value <= 16) t.v_nf = value;
-    else if (!strcmp(key, "v_nside") && (value == 0 || value == 128 || value == 256 || value == 512))
-        t.v_nside = value;
-    else if (!strcmp(key, "v_cps") && value >= 0 && value <= 8) t.v_cps = value;
+    else if (!strcmp(key, "v_nside") && (value == 0 || value == 128 || value == 256 || value == 512)) {}   // (no effect)
+    else if (!strcmp(key, "v_cps") && value >= 0 && value <= 8) {}
     else if (!strcmp(key, "v_gqa_form") && value >= 0 && value <= 2) t.v_gqa_form = value;
-    else if (!strcmp(key, "v_npt") && value >= 0 && value <= 8) t.v_npt = value;
+    else if (!strcmp(key, "v_npt") && value >= 0 && value <= 8) {}
     else if (!strcmp(key, "v_split_impl") && (value == 0 || value == 1)) t.v_split_impl = value;
-    else if (!strcmp(key, "v_ndw") && (value == 0 || value == 2 || value == 4)) t.v_ndw = value;
+    else if (!strcmp(key, "v_ndw") && (value == 0 || value == 2 || value == 4)) {}
     else if (!strcmp(key, "v_split_nf") && (value == 0 || value == 4 || value == 8)) t.v_split_nf = value;
     else if (!strcmp(key, "v_split_cps") && value >= 0 && value <= 8) t.v_split_cps = value;
-    else if (!strcmp(key, "v_upc") && value >= 0 && value <= 2) t.v_upc = value;
+    else if (!strcmp(key, "v_upc") && value >= 0 && value <= 2) {}
     else {
         set_error("set_tuning: unknown key or value out of range (%s = %d)", key, value);
         return AKV_ERR_SHAPE;

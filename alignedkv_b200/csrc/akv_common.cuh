@@ -23,14 +23,9 @@ struct Tuning {
     int k_wpc = 0;      // cap on warps per CTA of the q.K^T kernel (0 = as many as shared memory allows)
     int pdl = 1;        // 1: the kernels of a decode step are chained with programmatic dependent launch
     int k_gqa_kch = 8;  // channels per stage of the q.K^T kernel when query heads share KV heads (8 or 16)
-    int v_impl = 0;     // exact P.V, multi-head, aligned mode: 0 = branch-free chain form, 1 = producer-transposed form
-    int v_nf = 0;       // exact P.V (form 0): cap on the ring depth in 64-token stages (0 = from the shared-memory budget)
-    int v_nside = 0;    // exact P.V (form 0): rows of the nibble side ring, a power of two >= 128 (0 = default)
-    int v_cps = 0;      // exact P.V (form 0): CTAs per SM the shared-memory budget is cut for (0 = one wave)
-    int v_upc = 0;      // exact P.V (form 0): (batch, head) units per CTA, 1 or 2 (0 = default)
+    int v_impl = 0;     // exact P.V, aligned mode, groups of 1, 2, 4: 0 = chain form, 1 = producer-transposed form
+    int v_nf = 0;       // exact P.V (form 0): cap on the ring depth in stages (0 = from the shared-memory budget)
     int v_gqa_form = 0;   // exact P.V, grouped queries (form 0): 0 = by size, 1 = one ring per query head, 2 = the group's heads share a ring
-    int v_npt = 0;      // exact P.V (form 0): low-byte tables per head, 2, 4, 6 or 8 (0 = default)
-    int v_ndw = 0;      // exact P.V (form 0), two rings of one head each: decision warps per head, 2 or 4 (0 = default)
     int v_split_impl = 0;   // order-free P.V, multi-head, aligned mode: 0 = staged through shared memory by bulk copies, 1 = direct loads
     int v_split_nf = 0;     // order-free P.V, streaming form: ring depth 4 or 8 (0 = default 8)
     int v_split_cps = 0;    // order-free P.V, streaming form: CTAs per SM the chunking aims at (0 = default 3)

@@ -1,42 +1,40 @@
-// Exact-order P.V, streaming form for multi-head attention: the kernel body behind v_cache_compute for head_dim 128.
+// Exact-order P.V: the kernel body behind v_cache_compute for head_dim 128.
 //
 // Replaces the reference's v_cache_compute_kernel (extension/csrc/V_cache.cu:178-308); bit-identical outputs: every
 // output channel is the fp16 fused-multiply-add chain over tokens 0..n-1 in order (V_cache.cu:203,304), skipped nibble
 // planes are replaced by the reference's constants (V_cache.cu:198-202,250-253).
 //
-// Design (B200).  The token order leaves one dependent chain per (batch, head, channel pair), and the V layout is
+// Design (B200).  The token order leaves one dependent chain per (batch, query head, channel pair), and the V layout is
 // token-major (a token's 128 high bytes are one row) while a chain thread wants "my channel pairs, next tokens".  That
 // transposition is done by the load instruction: ldmatrix.x4.trans over four token rows (one 8x8 matrix of 16-bit
 // words per token: its eight 16-byte chunks, 128 contiguous bytes, so no bank conflict) hands lane T, for each of
 // the four tokens, one register holding the high-byte pairs of channel pairs 16*(T%4) + T/4 and 16*(T%4) + 8 + T/4.
-// The LOW bytes come the same way from a table of the same shape that holds 0x80 for every channel of every token
-// (the reference's substitute when neither nibble plane is read: the rule, in aligned mode) except for the few tokens
-// whose probability lies within two binades of the threshold; their rows are built from the nibble planes.  So the
-// chain warp runs ONE branch-free instruction stream for every token: per 8 tokens four ldmatrix and one 16-byte load
-// of probabilities, per token two byte permutes (high + low bytes -> two fp16 pairs) and two FMAs - two independent
-// chains per thread, which hide the FMA latency.  That matters more than it seems: a warp whose steady loop carries
-// branches and rarely-run code, or does not fit the scheduler's instruction cache, was measured at a third of the
-// speed of the same arithmetic in a straight line.
-//   A unit = one (batch, query head).  A CTA holds UPC rings of high bytes; a ring serves GH heads - one, or the query
-//   heads of one KV head, which need the same high bytes - and every head has its own chain warp, decision warps,
-//   tables and barriers.  (With a ring per query head the heads of a KV head are neighbouring units that stream the same
-//   planes at the same pace: the first one's copies bring a stage into L2, the others' hit there.)
-//   chain warp: all 64 channel pairs of the head, one 64-token stage per loop iteration.
-//   copy warp (one per ring): stage i -> ring slot i % nf as soon as every chain of the ring has released the slot's
-//     previous stage: one 8 KB bulk asynchronous copy of the high bytes exactly as they lie in the plane.
-//   decision warps (NDW per head, stage i belongs to warp i % NDW): lane = tokens (lane, lane + 32) of a stage.  EARLY
-//     part, a ring ahead of its use: takes the probabilities from a buffer bulk-copied a chunk ahead, decides the read
-//     codes (V_cache.cu:211,250-251), reserves rows of a small side ring for the tokens that read a nibble plane and
-//     starts 64-byte copies of just those rows (one 4 KB copy when the whole stage reads a plane), counted on a barrier
-//     of their own.  LATE part, when the stage's ring slot is free: restores the table rows the slot's previous stage
-//     had patched, makes sure the nibble rows have landed (long ago), builds the flagged tokens' rows of the low-byte
-//     table, and arrives on the stage's barrier.  Requesting the nibble rows a ring ahead matters: issued together with
-//     the stage's high bytes, the few small copies completed late under load and held up every stage that had one.
-//     And the NUMBER of these warps matters: a stage with flagged tokens costs its warp three out-of-line calls, and
-//     two warps per head fell behind the chain on every such stage (34.9 us for batch 8 x 32 heads x 4096 tokens);
-//     four, on schedulers the chain warps do not use, keep up (28.5 us, with or without flagged tokens).
+// A token that reads no nibble plane - the rule - has the constant low byte 0x80, so its two fp16 words are two byte
+// permutes of that register, the same for every query head of the KV head: a chain warp runs the chains of GH heads, per
+// token two permutes and 2 GH FMAs.
+//   A unit = the query heads of one (batch, KV head), or one of them (while they are few the heads of a KV head do better
+//   with rings of their own: they stream the same planes at the same pace and meet in L2): a ring of 64-token stages in shared memory, W = NH / GH chain warps that drain it and HW
+//   helper warps that fill it (stage i belongs to helper i % HW).  A CTA holds UPC units (warps ordered so that the chain
+//   warps lie on different schedulers); with more units than fit at once a (helpers, chains) group walks through several
+//   of them without draining its ring.
+//   A stage = 8 KB of high bytes as they lie in the plane (one bulk copy), the probabilities of the unit's heads, and per
+//   head and token the place of the token's 128 LOW bytes: a constant row of 0x80, or, for a token that reads a nibble
+//   plane, a row of the helper's pool, built for the token's code.  Low bytes are fetched like the high ones - every
+//   lane of an ldmatrix names the row it loads, so a token's row can lie anywhere - which keeps the chain's instruction
+//   stream straight whatever the codes are.  Stages without a flagged token run a second copy of the body that does not
+//   fetch low bytes; that is the only branch.  It matters: a taken branch costs a lone warp tens of cycles, and forms
+//   that branched to other code for groups of 8 tokens with a flagged one lost more on the 1 % of flagged tokens than the
+//   rest gained.
+//   helper warp: lane = tokens (2 lane, 2 lane + 1) of its stage.  Waits for the slot to be released, starts the high
+//     bytes' copy, takes the heads' probabilities (loaded from global memory a stage of its own ahead) and decides the
+//     read codes (V_cache.cu:211,250-251); then it finishes its PREVIOUS stage (builds the rows from the nibble rows
+//     requested an iteration ago, arrives), hands out pool rows for this stage, stores probabilities and places and
+//     requests the nibble rows.  An iteration is a chain of latencies of 700 to 1500 cycles, several times what the chains
+//     need for a stage: hence several helpers.
+// What bounds it: with two units on every SM the high bytes' stream from HBM and the FMA pipe (an fp16x2 FMA issues every
+// other cycle: 4 heads are 16 cycles per token), with few units the chain: 6 to 7 cycles per token.
 // Every wait is bounded (about a second); a wait that runs out raises the device error flag, the chain stores NaN
-// instead of a result, and the producers give their copies in flight time to land before the CTA leaves.
+// instead of a result, and the helper gives its copies in flight time to land before the CTA leaves.
 #pragma once
 #include "akv_common.cuh"
 
@@ -57,10 +55,10 @@ struct VParams {
     uint16_t* o;            // [B, Hq, D]
     int max_seq_len, D, s_last_dim, n, reference;
     int group;              // query heads per KV head (1 = multi-head attention)
-    int nf, nside, sch;     // streaming form: ring depth (stages), side-ring rows (power of two), stages per chunk
-    int npt;                // streaming form: low-byte tables per head (even: half of them per decision warp)
-    int units;              // streaming form: number of ring units (heads / heads per ring)
-    // streaming form: res != nullptr adds the residual tokens' part of the output, [B, Hq, D] fp16 computed by the
+    int nf;                 // chain kernel: ring depth (stages)
+    int units;              // chain kernel: number of units
+    int share;              // chain kernel: units that read the planes of one KV head (group / heads per unit)
+    // chain kernel: res != nullptr adds the residual tokens' part of the output, [B, Hq, D] fp16 computed by the
     // softmax kernel: out = half(o + res) (extension/v_cache_file.py:189), which saves the tail launch
     const uint16_t* res;
 };
@@ -126,36 +124,37 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
 }
 
 namespace vch {
-constexpr int TOK = 64;            // tokens per stage
 constexpr int D = 128, HD = 64;    // head size, bytes of a nibble row
-constexpr int F_BYTES = TOK * D;   // high bytes of a stage (and its rows of the low-byte table)
-constexpr int REC = 16;            // record of a stage: {first side row, flagged tokens 0..31, 32..63, rows | (table + 1) << 8}
-
-// Shared-memory plan of a CTA (byte offsets), computed the same way on both sides.  A CTA holds `upc` rings, each
-// shared by `gh` heads (gh > 1: the query heads of one KV head read the same high bytes).
+constexpr int TOK = 64;            // tokens per stage
+// Helper warps per unit (the ring depth is a multiple: a slot's stages all belong to one helper).  Four, or two where the
+// pools of four would leave too little room for the ring.  (Stages of 128 tokens, prepared by two helpers, were faster in
+// back-to-back launches and slower in a decode step, where every plane byte comes from HBM: 96 against 85 us per step at
+// batch 8 x 32 heads x 4096 tokens.)
+__host__ __device__ constexpr int helpers(int upc, int heads) { return upc > (heads > 1 ? 1 : 2) ? 2 : 4; }
+// A ring slot: high bytes | probabilities [heads][TOK] | places of the low bytes [heads][8][8] (token 8 g + w of the
+// stage at [w][g]: what a lane needs for its rows of the groups lies together), in 2-byte units into the unit's pools |
+// how many tokens of the stage read a nibble plane
+__host__ __device__ constexpr int off_s() { return TOK * D; }
+__host__ __device__ constexpr int off_low(int heads) { return off_s() + heads * TOK * 2; }
+__host__ __device__ constexpr int off_any(int heads) { return off_low(heads) + heads * TOK * 2; }
+__host__ __device__ constexpr int slot_bytes(int heads) { return (off_any(heads) + 4 + 127) & ~127; }
+// Rows of a helper's pool: a token has one code with one head per unit, up to two (both planes; mid only) with several;
+// all tokens of a stage must fit at once.
+__host__ __device__ constexpr int rows_per_token(int heads) { return heads > 1 ? 2 : 1; }
+__host__ __device__ constexpr int pool_rows(int heads) { return TOK * rows_per_token(heads); }
+// A unit's share of the shared memory: nf slots | the helpers' pools and the constant row | per helper the list of a
+// stage's flagged tokens | pool position after each slot's stage | barriers full[nf], free[nf]
 struct Plan {
-    int ctab;                        // the constant low-byte table (0x80 everywhere), one per CTA
-    int ring0, ring_bytes, rbar;     // ring r at ring0 + r * ring_bytes: nf stages of high bytes, then full[nf], free[nf] at rbar
-    int head0, head_bytes;           // head u at head0 + u * head_bytes, inside it:
-    int lw, mid, low, sb, rec, thr, bar;
-    int bytes;
+    int pool, list, cum, bar, bytes;
 };
-__host__ __device__ inline Plan plan(int nf, int nside, int sch, int npt, int upc, int gh) {
-    Plan p;
-    p.ctab = 0;
-    p.ring0 = F_BYTES;
-    p.rbar = nf * F_BYTES;
-    p.ring_bytes = (nf * F_BYTES + 2 * nf * 8 + 127) & ~127;
-    p.head0 = p.ring0 + upc * p.ring_bytes;
-    p.lw = 0;                                  // npt low-byte tables, each of a stage's shape
-    p.mid = npt * F_BYTES;                     // side rings: rows of the mid / low nibble planes
-    p.low = p.mid + nside * HD;
-    p.sb = p.low + nside * HD;                 // three probability buffers of sch x 64 values
-    p.rec = p.sb + 3 * sch * TOK * 2;          // 2 nf records
-    p.thr = p.rec + 2 * nf * REC;              // threshold (already shifted)
-    p.bar = (p.thr + 4 + 7) & ~7;              // probability buffers[3], nibble rows[2 nf]
-    p.head_bytes = (p.bar + (2 * nf + 3) * 8 + 127) & ~127;
-    p.bytes = p.head0 + upc * gh * p.head_bytes;
+__host__ __device__ constexpr Plan plan(int nf, int upc, int heads) {
+    Plan p{};
+    const int hw = helpers(upc, heads);
+    p.pool = nf * slot_bytes(heads);
+    p.list = p.pool + (hw * pool_rows(heads) + 1) * D;
+    p.cum = p.list + hw * TOK * 2;
+    p.bar = (p.cum + nf * 4 + 7) & ~7;
+    p.bytes = (p.bar + 2 * nf * 8 + 127) & ~127;
     return p;
 }
 }  // namespace vch
@@ -177,480 +176,412 @@ __device__ __noinline__ void v_sleep_ms() {
     for (int k = 0; k < 1000; ++k) __nanosleep(1000);
 }
 
-// Starts the copies of the nibble rows of one stage into the side ring and announces their bytes on `bar` (one
-// arrival).  Out of line: it runs for the minority of stages in which some token reads a nibble plane, and the
-// decision warp's steady loop has to stay small.
-//   M, L: mid / low plane rows of the stage's token 0;  ma, la: side rings;  start: first side row;  wrap: rows - 1
-//   um0 / um1: tokens 0..31 / 32..63 that read the mid plane;  c0 / c1: this lane's codes of tokens lane / lane+32
-__device__ __noinline__ void v_issue_nibble_rows(const uint8_t* M, const uint8_t* L, uint32_t ma, uint32_t la, uint32_t bar,
-                                                 uint32_t start, uint32_t wrap, uint32_t um0, uint32_t um1, int c0, int c1,
-                                                 int lane) {
-    using namespace vch;
-    const uint32_t ul0 = __ballot_sync(0xFFFFFFFFu, c0 == 0), ul1 = __ballot_sync(0xFFFFFFFFu, c1 == 0);
-    const uint32_t rows = __popc(um0) + __popc(um1);
-    if (lane == 0) mbar_arrive_expect(bar, (uint32_t)HD * (rows + __popc(ul0) + __popc(ul1)));
-    __syncwarp();
-    const uint32_t lt = (1u << lane) - 1u;
-    if ((um0 & um1) == 0xFFFFFFFFu && start + TOK <= wrap + 1) {
-        // the whole stage reads the mid plane: one 4 KB copy (and one for the low plane when it is all read)
-        if (lane == 0) bulk_copy(ma + start * HD, M, TOK * HD, bar);
-        if ((ul0 & ul1) == 0xFFFFFFFFu) {
-            if (lane == 0) bulk_copy(la + start * HD, L, TOK * HD, bar);
-        } else {
-            if (c0 == 0) bulk_copy(la + ((start + lane) & wrap) * HD, L + (size_t)lane * HD, HD, bar);
-            if (c1 == 0) bulk_copy(la + ((start + 32 + lane) & wrap) * HD, L + (size_t)(lane + 32) * HD, HD, bar);
-        }
-    } else {
-        const uint32_t r0 = (start + __popc(um0 & lt)) & wrap;
-        const uint32_t r1 = (start + __popc(um0) + __popc(um1 & lt)) & wrap;
-        if (c0 < 2) bulk_copy(ma + r0 * HD, M + (size_t)lane * HD, HD, bar);
-        if (c0 == 0) bulk_copy(la + r0 * HD, L + (size_t)lane * HD, HD, bar);
-        if (c1 < 2) bulk_copy(ma + r1 * HD, M + (size_t)(lane + 32) * HD, HD, bar);
-        if (c1 == 0) bulk_copy(la + r1 * HD, L + (size_t)(lane + 32) * HD, HD, bar);
+__device__ __forceinline__ uint4 v_ldg128(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void sts128(uint32_t a, const uint4& v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts16(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(a), "h"((uint16_t)v) : "memory");
+}
+
+// 32 low bytes of a token (16 channel pairs) from 16 bytes of its mid and low plane rows.  A pair's byte holds the even
+// channel's nibble above the odd one's; the even channel's low byte is mid.hi:low.hi, the odd one's mid.lo:low.lo
+// (V_cache.cu:250-253).
+__device__ __forceinline__ void v_low_bytes(uint32_t dst, const uint4& m, const uint4& l) {
+    uint32_t o[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t mw = u4w(m, j), lw = u4w(l, j);
+        const uint32_t ev = (mw & 0xF0F0F0F0u) | ((lw >> 4) & 0x0F0F0F0Fu), od = ((mw << 4) & 0xF0F0F0F0u) | (lw & 0x0F0F0F0Fu);
+        o[2 * j] = __byte_perm(ev, od, 0x5140);
+        o[2 * j + 1] = __byte_perm(ev, od, 0x7362);
     }
+    sts128(dst, make_uint4(o[0], o[1], o[2], o[3]));
+    sts128(dst + 16, make_uint4(o[4], o[5], o[6], o[7]));
 }
 
-// Builds the rows of the low-byte table for the flagged tokens of one stage from the side ring (V_cache.cu:250-253):
-// channel pair p of a token has mid byte [even channel nibble | odd channel nibble] and low byte likewise; the low
-// byte of the even channel is (mid & 0xF0) | (low >> 4), of the odd one ((mid & 0x0F) << 4) | (low & 0x0F); a token
-// that reads only the mid plane takes 0x88 for the low-plane byte.  Lane l builds channel pairs 2l, 2l+1 (4 bytes).
-//   lw: the stage's rows of the table;  ma, la: side rings;  rec: {first side row, flagged 0..31, 32..63, rows}
-//   s_a: the stage's probabilities;  thr: shifted threshold
-__device__ __noinline__ void v_build_low_rows(uint32_t lw, uint32_t ma, uint32_t la, uint4 rec, uint32_t wrap, uint32_t s_a,
-                                              uint32_t thr, int reference, int lane) {
-    using namespace vch;
-    uint32_t rank = 0;
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-#pragma unroll 1
-        for (uint32_t bits = half ? rec.z : rec.y; bits; bits &= bits - 1, ++rank) {
-            const int t = half * 32 + __ffs(bits) - 1;
-            const uint32_t sb = lds16(s_a + t * 2);
-            const int diff = (int)(int16_t)(uint16_t)(thr - sb);
-            const bool low_too = reference || diff < 0x0400;             // (the token reads the mid plane: it is flagged)
-            const uint32_t row = ((rec.x + rank) & wrap) * HD + 2 * lane;
-            const uint32_t mb = lds16(ma + row);                          // pairs 2l, 2l+1
-            const uint32_t lb = low_too ? lds16(la + row) : 0x8888u;
-            const uint32_t even = (mb & 0xF0F0u) | ((lb >> 4) & 0x0F0Fu);     // [pair 2l, pair 2l+1] even channels
-            const uint32_t odd = ((mb & 0x0F0Fu) << 4) | (lb & 0x0F0Fu);
-            // bytes: [even(2l), odd(2l), even(2l+1), odd(2l+1)]
-            const uint32_t w = (even & 0xFFu) | ((odd & 0xFFu) << 8) | ((even & 0xFF00u) << 8) | ((odd & 0xFF00u) << 16);
-            asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(lw + (uint32_t)t * D + lane * 4), "r"(w) : "memory");
-        }
-    }
-}
-
-// Puts the constant 0x80 back into the table rows of the tokens flagged in (m0, m1).
-__device__ __noinline__ void v_restore_low_rows(uint32_t lw, uint32_t m0, uint32_t m1, int lane) {
-    using namespace vch;
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half)
-#pragma unroll 1
-        for (uint32_t bits = half ? m1 : m0; bits; bits &= bits - 1)
-            asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(lw + (uint32_t)(half * 32 + __ffs(bits) - 1) * D + lane * 4),
-                         "r"(0x80808080u) : "memory");
-}
-
-// UPC rings per CTA, GH heads per ring, NDW decision warps per head (2, or 4 with two rings of one head each).
-template <int UPC, int GH, int NDW>
-__global__ void __launch_bounds__(NDW == 2 ? ((1 + NDW) * UPC * GH + UPC) * 32 : 512, 1) v_chain_kernel(const VParams p) {
-    static_assert(NDW == 2 || (NDW == 4 && UPC == 2 && GH == 1), "decision warps per head");
+// NH query heads per unit, GH of them per chain warp, UPC units per CTA at a time.
+template <int NH, int GH, int UPC>
+__global__ void __launch_bounds__(UPC * (2 * NH / GH + vch::helpers(UPC, NH)) * 32, 1) v_chain_kernel(const VParams p) {
     using namespace vch;
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int NU = UPC * GH;                   // heads of the CTA
-    // Low-byte tables.  One head per ring: a table per ring slot (npt == nf), patched for the slot's stage and restored
-    // when the slot is released - a stage without flagged tokens finds the constant there, and the chain needs neither
-    // the record nor a select.  Several heads per ring: there is no room for that, so each decision warp has a few
-    // tables it hands to its stages with flagged tokens, and the other stages read the CTA's constant table.
-    constexpr bool SLOT_TABLES = GH == 1;
-    const int tid = threadIdx.x, lane = tid & 31, wcta = tid >> 5;
-    // Warp roles: per head a chain warp and two decision warps (even / odd stages: one warp's serial walk through a
-    // stage takes longer than the chain needs to consume it), per ring a copy warp.  Order in the CTA: the chain warps,
-    // the even-stage decision warps, the copy warps, the odd-stage decision warps.  The warps are spread over the SM's
-    // four schedulers by index, so with two rings of one head each chain warp shares its scheduler only with its copy
-    // warp (a handful of instructions per stage) and the four decision warps have the other two; with four heads on
-    // one ring every scheduler has one chain warp.
-    int role, hu, dw = 0;                          // 0: chain, 1: decision (warp dw of its head), 3: copy, -1: none; head of the CTA
-    if (NDW == 2) {
-        if (wcta < NU) { role = 0; hu = wcta; }
-        else if (wcta < 2 * NU) { role = 1; hu = wcta - NU; }
-        else if (wcta < 2 * NU + UPC) { role = 3; hu = (wcta - 2 * NU) * GH; }
-        else { role = 1; dw = 1; hu = wcta - 2 * NU - UPC; }
-    } else {
-        // sixteen warps in groups of four (one per scheduler): schedulers 0, 1 get [chain, copy, -, -] of ring 0 / 1,
-        // schedulers 2, 3 the four decision warps of head 0 / 1 - a chain warp never shares its scheduler with a
-        // decision warp, whose bursts of work would take issue slots from it
-        const int q4 = wcta >> 2, r4 = wcta & 3;
-        if (r4 < 2) { hu = r4; role = q4 == 0 ? 0 : (q4 == 1 ? 3 : -1); }
-        else { hu = r4 - 2; role = 1; dw = q4; }
-    }
-    const int ring = hu / GH, hg = hu - ring * GH;
-    const long long ru = (long long)blockIdx.x * UPC + ring;   // ring unit
-    const long long bh = ru * GH + hg;                         // (batch, query head)
-    const long long kv = (ru * GH) / p.group;                  // (batch, KV head) whose planes the ring streams
-    const int n = p.n, nf = p.nf, nside = p.nside, sch = p.sch;
-    const int nst = (n + TOK - 1) / TOK;
-    const Plan pl = plan(nf, nside, sch, p.npt, UPC, GH);
-    const uint32_t cta = smem_u32(smem);
-    const uint32_t rbase = cta + pl.ring0 + (uint32_t)ring * pl.ring_bytes;    // the ring's stages of high bytes
-    const uint32_t base = cta + pl.head0 + (uint32_t)hu * pl.head_bytes;       // everything of this head
-    const uint32_t bar_full = rbase + pl.rbar, bar_free = bar_full + nf * 8;
-    const uint32_t bar_sb = base + pl.bar, bar_nib = bar_sb + 3 * 8;
-    const uint32_t ctab = cta + pl.ctab;
-
-    pdl_enter();
-    if (!SLOT_TABLES)
-        for (int i = tid; i < F_BYTES / 16; i += blockDim.x)
-            asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(ctab + i * 16), "r"(0x80808080u) : "memory");
-    if (role == 0) {
-        if (lane == 0) {
-            if (hg == 0)
-                for (int s = 0; s < nf; ++s) {
-                    mbar_init(bar_full + s * 8, 1 + GH);   // the copy warp's arrival (+ the high bytes) and one decision warp's per head
-                    mbar_init(bar_free + s * 8, GH);       // the chain warps' arrivals
-                }
-            for (int s = 0; s < 3; ++s) mbar_init(bar_sb + s * 8, 1);
-            for (int s = 0; s < 2 * nf; ++s) mbar_init(bar_nib + s * 8, 1);
+    constexpr int W = 2 * NH / GH, HW = helpers(UPC, NH), NG = TOK / 8;
+    constexpr int SLOT = slot_bytes(NH), RPT = rows_per_token(NH), NP = pool_rows(NH);
+    constexpr int OFF_S = off_s(), OFF_LOW = off_low(NH), OFF_ANY = off_any(NH);
+    constexpr uint32_t CONST_ROW = HW * NP * D;    // place of the constant low bytes
+    const int lane = threadIdx.x & 31, wcta = threadIdx.x >> 5;
+    // warps: the chain warps of all units first (consecutive warps go to different schedulers), then the helpers
+    const bool helper = wcta >= UPC * W;
+    const int uc = helper ? (wcta - UPC * W) / HW : wcta / W;
+    const int wi = helper ? wcta - UPC * W - uc * HW : wcta - uc * W;      // warp inside the unit's helpers / chains
+    const int nf = p.nf, n = p.n, nst = (n + TOK - 1) / TOK;
+    const Plan pl = plan(nf, UPC, NH);
+    const uint32_t ring = smem_u32(smem) + (uint32_t)(uc * pl.bytes);
+    const uint32_t pool = ring + pl.pool, bar_full = ring + pl.bar, bar_free = bar_full + nf * 8;
+    if (helper) {
+        if (wi == 0 && lane == 0) {
+            for (int s = 0; s < nf; ++s) {
+                mbar_init(bar_full + s * 8, 2);    // the high bytes' copy and the helper's arrival
+                mbar_init(bar_free + s * 8, W);    // the chain warps
+            }
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
-        // the head's own low-byte tables start as the constant too: 0x80 for every channel of every token
-        for (int i = lane; i < p.npt * F_BYTES / 16; i += 32)
-            asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(base + pl.lw + i * 16), "r"(0x80808080u) : "memory");
+        sts32(pool + CONST_ROW + lane * 4, 0x80808080u);
+        // (a chain warp loads low bytes from the places of a stage without flagged tokens too, or of a slot that has no stage
+        // yet, without using them: they have to lie inside the pools)
+        for (int s = wi; s < nf; s += HW)
+            for (int i = lane; i < NH * TOK / 2; i += 32) sts32(ring + (uint32_t)s * SLOT + OFF_LOW + i * 4, 0u);
     }
+    pdl_enter();
     __syncthreads();
-    if (role < 0 || ru >= p.units) return;         // (odd number of ring units: the last CTA's second ring has none)
+    // units are dealt out a grid apart, so that every SM gets its share
+    const int first_unit = uc * gridDim.x + blockIdx.x, stride = UPC * gridDim.x;
+    const int nunits = first_unit < p.units ? (p.units - first_unit + stride - 1) / stride : 0;   // of this group
 
-    if (role == 3) {
-        // ------------------------------------------------------------------ copy warp: the high bytes
-        const uint8_t* F = p.first8 + (size_t)kv * p.max_seq_len * D;
-        int slot = 0;
-        uint32_t parity = 0;                       // of the release being waited for: (i / nf - 1) & 1
+    if (helper) {
+        // ------------------------------------------------------------------ helper warp
+        // Its stages are q = wi, wi + HW, ... of the group's stages 0 .. nunits * nst - 1; stage q uses slot q % nf.
+        const uint32_t list = ring + pl.list + wi * TOK * 2, cum = ring + pl.cum;
+        const uint32_t mine = (uint32_t)wi * NP * D;                       // place of the pool
+        const long long total = (long long)nunits * nst;
         bool alive = true;
-        // The decision warp's first loads (probe result, exponent maxima) go out before this warp floods the memory
-        // system with the first ring of copies - behind that flood they would take several times as long, and the
-        // first stage cannot be consumed before the threshold is known.
-        asm volatile("bar.sync %0, %1;\n" ::"r"(1 + ring), "r"((NDW * GH + 1) * 32) : "memory");
+        int slot = wi;                             // of stage q (nf is a multiple of HW)
+        int rel = wi, out = 0;                     // slot of its oldest stage whose release has not been consumed; stages since
+        uint32_t rel_par = 0;                      // parity of that release
+        uint32_t head = 0, tail = 0;               // pool rows handed out / taken back so far
+        // consume the release of its oldest stage: the slot and the stage's pool rows are free again
+        auto reclaim = [&]() {
+            alive = mbar_wait(bar_free + rel * 8, rel_par);
+            tail = lds32(cum + rel * 4);
+            --out;
+            if ((rel += HW) >= nf) { rel -= nf; rel_par ^= 1u; }
+        };
+        const int lim_m = p.reference ? 0x8000 : 0x0800, lim_l = p.reference ? 0x8000 : 0x0400;    // (0x8000: always)
+        auto plane_row = [&](int unit) { return (size_t)(NH > 1 ? unit : unit / p.share) * p.max_seq_len; };   // of its token 0
+        auto copy_high = [&](size_t row, int i, int sl) {
+            const uint32_t bytes = (uint32_t)min(TOK, n - i * TOK) * D;
+            mbar_arrive_expect(bar_full + sl * 8, bytes);
+            bulk_copy(ring + (uint32_t)sl * SLOT, p.first8 + (row + (size_t)i * TOK) * D, bytes,
+                      bar_full + sl * 8);
+        };
+        // the first ring's high bytes depend on nothing but the planes: under way before the thresholds are known
+        const int early = min(nf, nst);
+        if (nunits > 0 && wi + HW * lane < early) copy_high(plane_row(first_unit), wi + HW * lane, wi + HW * lane);
+        // the unit's thresholds; probabilities of this lane's two tokens of its next stage
+        uint32_t A[NH], nxt[NH];
+        auto load_s = [&](int unit, int i) {       // (rows are padded to a multiple of 8 values)
+            const int t = i * TOK + 2 * lane;
+#pragma unroll
+            for (int g = 0; g < NH; ++g)
+                nxt[g] = t < n ? *reinterpret_cast<const uint32_t*>(p.s + ((size_t)unit * NH + g) * p.s_last_dim + t) : 0u;
+        };
+        // the previous stage: its slot (-1: none), flagged tokens and their first pool row
+        int pslot = -1, pcnt = 0;
+        size_t ptok = 0;                           // plane row of its first token
+        uint32_t prow = 0;
+        // Nibble rows of eight flagged tokens, lane = (token lane/4, 16 bytes lane%4).  The stage's first eight are requested
+        // when it is prepared and turned into pool rows an iteration later, more of them NBT batches at a time.
+        struct Batch {
+            uint4 m, l;
+            uint32_t t;                            // list entry: token | some head reads both planes << 8 | mid only << 9
+        };
+        auto request = [&](Batch& b, int k) {
+            b.t = 0xFFFFu;
+            if (8 * k + (lane >> 2) < pcnt) {
+                b.t = lds16(list + (8 * k + (lane >> 2)) * 2);
+                const size_t at = (ptok + (b.t & 0xFFu)) * HD + (lane & 3) * 16;
+                b.m = v_ldg128(p.mid4 + at);
+                if (b.t & 0x100u) b.l = v_ldg128(p.last4 + at);
+            }
+        };
+        auto build = [&](const Batch& b, int k) {
+            if (b.t == 0xFFFFu) return;
+            const uint32_t r = (prow + (uint32_t)(8 * k + (lane >> 2)) * RPT) % NP;
+            const uint32_t dst = pool + mine + r * D + (lane & 3) * 32;
+            const uint4 c88 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);
+            if (RPT == 1) {
+                v_low_bytes(dst, b.m, b.t & 0x100u ? b.l : c88);
+            } else {
+                if (b.t & 0x100u) v_low_bytes(dst, b.m, b.l);
+                if (b.t & 0x200u) v_low_bytes(dst + D, b.m, c88);    // (NP is even: the second row follows the first)
+            }
+        };
+        constexpr int NBT = NH > 4 ? 4 : 8;        // (registers)
+        Batch first;
+        first.m = first.l = make_uint4(0, 0, 0, 0);
+        first.t = 0xFFFFu;
+        const int slots = nf / HW;                 // its share of the ring
+        int unit = first_unit, i = wi;             // of stage q
+        while (i >= nst && nst > 0 && unit < p.units) { i -= nst; unit += stride; }
+        int aunit = -1;                            // the unit whose thresholds are in A
+        size_t row = 0;                            // ... and the plane row of its token 0
+        if (wi < total) load_s(unit, i);
 #pragma unroll 1
-        for (int i = 0; i < nst; ++i) {
-            if (i >= nf) {
-                alive = mbar_wait(bar_free + slot * 8, parity);
+        for (long long q = wi; q < total + HW && alive; q += HW) {
+            const bool now = q < total;            // (else: only the previous stage is left)
+            uint32_t cur[NH], code[NH], u0[2] = {0, 0}, u1[2] = {0, 0};   // even / odd tokens that read both planes / mid only for some head
+            int nunit = unit, ni = i + HW;
+            if (now) {
+                const bool entered = aunit != unit;
+                if (entered) {
+                    aunit = unit;
+                    row = plane_row(unit);
+                }
+                if (q >= early) {
+                    while (alive && out >= slots) reclaim();
+                    if (!alive) break;
+                    if (lane == 0) copy_high(row, i, slot);
+                }
+                ++out;
+                if (entered) {
+#pragma unroll
+                    for (int g = 0; g < NH; ++g) {
+                        const long long bh = (long long)unit * NH + g;
+                        uint32_t a;
+                        if (p.test_o) {
+                            a = v_threshold_warp(p.test_o, p.v_exp, bh, p.H, p.group, D, lane);
+                            if (i == 0 && lane == 0) p.amin_out[bh] = (uint8_t)a;
+                        } else {
+                            a = p.amin[bh];
+                        }
+                        A[g] = (a << 10) & 0xFFFFu;
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < NH; ++g) cur[g] = nxt[g];
+                while (ni >= nst) { ni -= nst; nunit += stride; }
+                if (q + HW < total) load_s(nunit, ni);
+                // read codes of this lane's tokens for every head: 16-bit wrap-around, signed compare
+                // (V_cache.cu:211,250-251); a code is 0 when the token reads both planes, 1 mid only, 2 neither
+                const int left = n - i * TOK - 2 * lane;     // of this lane's two tokens
+                uint32_t r0 = 0, r1 = 0;                     // bit h: some head reads both planes / mid only
+#pragma unroll
+                for (int g = 0; g < NH; ++g) {
+                    const int d0 = (int)(int16_t)(uint16_t)(A[g] - cur[g]), d1 = (int)(int16_t)(uint16_t)(A[g] - (cur[g] >> 16));
+                    const uint32_t c0 = left < 1 || d0 >= lim_m ? 2u : d0 >= lim_l ? 1u : 0u;
+                    const uint32_t c1 = left < 2 || d1 >= lim_m ? 2u : d1 >= lim_l ? 1u : 0u;
+                    code[g] = c0 | c1 << 16;
+                    r0 |= (c0 == 0 ? 1u : 0u) | (c1 == 0 ? 2u : 0u);
+                    r1 |= (c0 == 1 ? 1u : 0u) | (c1 == 1 ? 2u : 0u);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    u0[h] = __ballot_sync(0xFFFFFFFFu, (r0 >> h) & 1u);
+                    u1[h] = __ballot_sync(0xFFFFFFFFu, (r1 >> h) & 1u);
+                }
+            }
+            // finish the previous stage
+            if (pslot >= 0) {
+                if (pcnt > 0) {
+                    build(first, 0);
+#pragma unroll 1
+                    for (int k = 1; 8 * k < pcnt; k += NBT) {
+                        Batch b[NBT];
+#pragma unroll
+                        for (int j = 0; j < NBT; ++j) request(b[j], k + j);
+#pragma unroll
+                        for (int j = 0; j < NBT; ++j) build(b[j], k + j);
+                    }
+                }
+                __syncwarp();                      // (everything the lanes stored for this stage comes before the arrival)
+                if (lane == 0) mbar_arrive(bar_full + pslot * 8);
+            }
+            if (!now) break;
+            pslot = slot;
+            ptok = row + (size_t)i * TOK;
+            // pool rows and places of this stage
+            const uint32_t sl = ring + (uint32_t)slot * SLOT;
+            uint32_t place[2] = {CONST_ROW, CONST_ROW};
+            pcnt = __popc(u0[0] | u1[0]) + __popc(u0[1] | u1[1]);
+            if (pcnt != 0) {                       // (warp-uniform)
+                // (its older stages have been armed, and the chains let go of them once the stage behind them - another
+                // helper's - is there)
+                while (alive && head + pcnt * RPT - tail > (uint32_t)NP) reclaim();
                 if (!alive) break;
+                prow = head % NP;
+                head += pcnt * RPT;
+                const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t f = u0[h] | u1[h];
+                    const int rank = (h ? __popc(u0[0] | u1[0]) : 0) + __popc(f & lt);
+                    place[h] = mine + (prow + (uint32_t)rank * RPT) % NP * D;
+                    if ((f >> lane) & 1u)
+                        sts16(list + rank * 2, (2 * lane + h) | ((u0[h] >> lane) & 1u) << 8 | ((u1[h] >> lane) & 1u) << 9);
+                }
+                __syncwarp();
+                request(first, 0);
+            }
+#pragma unroll
+            for (int g = 0; g < NH; ++g) sts32(sl + OFF_S + g * (TOK * 2) + lane * 4, cur[g]);
+            if (pcnt != 0) {                       // (the places of other stages are not looked at)
+#pragma unroll
+                for (int g = 0; g < NH; ++g)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t c = h ? code[g] >> 16 : code[g] & 0xFFFFu, t = 2 * lane + h;
+                        const uint32_t at = c == 2 ? CONST_ROW : place[h] + (RPT == 2 && c == 1 ? D : 0);
+                        sts16(sl + OFF_LOW + (g * TOK + (t & 7) * NG + (t >> 3)) * 2, at >> 1);
+                    }
             }
             if (lane == 0) {
-                const int cnt = (n - i * TOK) < TOK ? (n - i * TOK) : TOK;
-                const uint32_t bar = bar_full + slot * 8;
-                mbar_arrive_expect(bar, (uint32_t)cnt * D);
-                bulk_copy(rbase + (uint32_t)slot * F_BYTES, F + (size_t)i * TOK * D, (uint32_t)cnt * D, bar);
+                sts32(sl + OFF_ANY, (uint32_t)pcnt);
+                sts32(cum + slot * 4, head);
             }
-            if (++slot == nf) { slot = 0; if (i >= nf) parity ^= 1u; }
-        }
-        if (!alive) v_sleep_ms();
-        return;
-    }
-    if (role == 1) {
-        // ------------------------------------------------------------------ decision warps
-        // Warp w (0 .. NDW-1) owns the stages i with i % NDW == w.  The ring depth nf is a multiple of NDW, so the
-        // previous stage of a ring slot belongs to the same warp, and each warp has its own part of the side ring: the
-        // warps never share state.
-        const int w = dw;
-        const uint8_t* M = p.mid4 + (size_t)kv * p.max_seq_len * HD;
-        const uint8_t* L = p.last4 + (size_t)kv * p.max_seq_len * HD;
-        const uint16_t* s_row = p.s + (size_t)bh * p.s_last_dim;
-        bool alive = true;
-        // probability chunk c (stages c*sch ..) -> buffer `buf` = c % 3; issued by one thread of warp 0
-        auto request_s = [&](int c, int buf) {
-            const int t0 = c * sch * TOK;
-            int cnt = n - t0;
-            cnt = cnt > sch * TOK ? sch * TOK : cnt;
-            const uint32_t bytes = (uint32_t)((cnt + 7) & ~7) * 2;     // rows are padded to a multiple of 8 values
-            mbar_arrive_expect(bar_sb + buf * 8, bytes);
-            bulk_copy(base + pl.sb + (uint32_t)buf * (sch * TOK * 2), s_row + t0, bytes, bar_sb + buf * 8);
-        };
-        if (w == 0 && lane == 0 && nst > 0) request_s(0, 0);
-        // threshold: from the probe result (decode step) or as given
-        uint32_t a;
-        if (p.test_o) {
-            a = v_threshold_warp(p.test_o, p.v_exp, bh, p.H, p.group, D, lane);
-            if (w == 0 && lane == 0) p.amin_out[bh] = (uint8_t)a;
-        } else {
-            a = p.amin[bh];
-        }
-        const uint32_t A = (a << 10) & 0xFFFFu;
-        asm volatile("bar.sync %0, %1;\n" ::"r"(1 + ring), "r"((NDW * GH + 1) * 32) : "memory");
-        const int hside = nside / NDW;                     // rows of this warp's part of the side ring
-        const uint32_t ma = base + pl.mid + (uint32_t)w * hside * HD, la = base + pl.low + (uint32_t)w * hside * HD;
-        const uint32_t wrap = (uint32_t)(hside - 1);
-        uint32_t side_head = 0, side_tail = 0;    // side rows handed out / taken back so far
-        const int nrec = 2 * nf;
-        int freed = w, freed_slot = w, freed_rec = w;   // next own stage whose release is to be consumed; % nf, % 2nf
-        uint32_t freed_parity = 0;                      // (freed / nf) & 1
-        uint32_t nib_par = 0;                           // bit r: parity of the NEXT phase of nibble barrier r
-        // low-byte tables of this warp, used in turn by its stages with flagged tokens; t_out = tables in use (built
-        // and not yet restored)
-        const int npw = p.npt / NDW;
-        int t_next = 0, t_out = 0;
-        // consume the release of own stage `freed`: its side rows are free again, its patched table rows become 0x80 again
-        auto reclaim = [&]() {
-            alive = mbar_wait(bar_free + freed_slot * 8, freed_parity);
-            const uint4 rec = lds128(base + pl.rec + freed_rec * REC);
-            if (__builtin_expect(rec.w != 0, 0)) {
-                side_tail += rec.w & 0xFFu;
-                if (alive && (rec.w >> 8) != 0) {           // (a stage that was prepared but never armed has no table)
-                    v_restore_low_rows(base + pl.lw + ((rec.w >> 8) - 1u) * F_BYTES, rec.y, rec.z, lane);
-                    --t_out;
-                }
-            }
-            freed += NDW;
-            if ((freed_slot += NDW) >= nf) { freed_slot -= nf; freed_parity ^= 1u; }
-            if ((freed_rec += NDW) >= nrec) freed_rec -= nrec;
-        };
-        // EARLY part for own stage j (position state advances with j).  armed = next own stage to be armed: side rows
-        // can only be waited for while an armed own stage is still unreleased; otherwise the stage is prepared later
-        // (returns false).
-        int e_rec = w, e_sic = w, e_c = 0, e_buf = 0;   // of stage j: j % 2nf, j % sch, j / sch, (j / sch) % 3
-        uint32_t e_par = 0;                             // ((j / sch) / 3) & 1
-        bool e_chunk = false;                           // the chunk of stage j has been entered
-        auto early = [&](int j, int armed) -> bool {
-            if (e_sic < NDW && !e_chunk) {    // entering chunk c: ask for the next one (warp 0), make sure this one has landed
-                if (w == 0 && (e_c + 1) * sch < nst && lane == 0) request_s(e_c + 1, e_buf == 2 ? 0 : e_buf + 1);
-                alive = mbar_wait(bar_sb + e_buf * 8, e_par);
-                if (!alive) return false;
-                e_chunk = true;
-            }
-            const int t0 = j * TOK;
-            const int cnt = (n - t0) < TOK ? (n - t0) : TOK;
-            // read codes of tokens `lane` and `lane + 32` from the bit patterns (V_cache.cu:211,250-251): 16-bit
-            // wrap-around, signed compare  (beyond the last token the buffer holds stale but readable bytes)
-            const uint32_t sa = base + pl.sb + (uint32_t)e_buf * (sch * TOK * 2) + (uint32_t)e_sic * (TOK * 2) + lane * 2;
-            const uint32_t s0 = lds16(sa), s1 = lds16(sa + 64);
-            const int d0 = (int)(int16_t)(uint16_t)(A - s0), d1 = (int)(int16_t)(uint16_t)(A - s1);
-            int c0 = p.reference ? 0 : (d0 >= 0x0800 ? 2 : (d0 >= 0x0400 ? 1 : 0));
-            int c1 = p.reference ? 0 : (d1 >= 0x0800 ? 2 : (d1 >= 0x0400 ? 1 : 0));
-            if (lane >= cnt) c0 = 2;
-            if (lane + 32 >= cnt) c1 = 2;
-            const uint32_t um0 = __ballot_sync(0xFFFFFFFFu, c0 < 2), um1 = __ballot_sync(0xFFFFFFFFu, c1 < 2);
-            uint32_t rows = 0, start = 0;
-            if (__builtin_expect((um0 | um1) != 0, 0)) {    // (warp-uniform)
-                rows = __popc(um0) + __popc(um1);
-                // rows of the side ring, taken in token order; wait for older stages to hand theirs back if it is full
-                while (alive && side_head + rows - side_tail > (uint32_t)hside) {
-                    if (freed >= armed) return false;       // nothing armed is outstanding: prepare this stage later
-                    reclaim();
-                }
-                if (!alive) return false;
-                start = side_head & wrap;
-                side_head += rows;
-                nib_par ^= 1u << e_rec;
-                v_issue_nibble_rows(M + (size_t)t0 * HD, L + (size_t)t0 * HD, ma, la, bar_nib + e_rec * 8, start, wrap, um0,
-                                    um1, c0, c1, lane);
-            }
-            if (lane == 0)
-                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(base + pl.rec + e_rec * REC), "r"(start), "r"(um0),
-                             "r"(um1), "r"(rows) : "memory");
-            __syncwarp();               // (the record is read back by every lane in the late part)
-            if ((e_rec += NDW) >= nrec) e_rec -= nrec;
-            e_chunk = false;
-            if ((e_sic += NDW) >= sch) {
-                e_sic -= sch;
-                ++e_c;
-                if (++e_buf == 3) { e_buf = 0; e_par ^= 1u; }
-            }
-            return true;
-        };
-        int slot = w, rec = w, j = w;             // of stage i: i % nf, i % 2nf; j: next own stage to prepare
-        int l_sic = w, l_buf = 0;                 // of stage i: i % sch, (i / sch) % 3
-#pragma unroll 1
-        for (int i = w; i < nst && alive; i += NDW) {
-            while (alive && freed <= i - nf) reclaim();
-            // phase 0: stage i must be prepared (it normally is, a ring ago), then it is armed; phase 1: run ahead, up
-            // to a ring's length (one call site of the early part for both)
-#pragma unroll 1
-            for (int phase = 0; phase < 2 && alive; ++phase) {
-                const int lim = phase == 0 ? i : i + nf;
-#pragma unroll 1
-                while (alive && j <= lim && j < nst) {
-                    if (!early(j, i + NDW * phase)) break;
-                    j += NDW;
-                }
-                if (phase == 0 && alive) {
-                    // LATE part of stage i: its nibble rows (requested long ago) must have landed and its rows of the
-                    // low-byte table be built; then it is armed
-                    const uint4 r = lds128(base + pl.rec + rec * REC);
-                    if (__builtin_expect(r.w != 0, 0)) {
-                        // a table of this warp: the oldest one in use is handed back when its (armed) stage is released
-                        while (!SLOT_TABLES && alive && t_out >= npw) reclaim();
-                        if (alive) alive = mbar_wait(bar_nib + rec * 8, ((nib_par >> rec) & 1u) ^ 1u);
-                        if (alive) {
-                            const uint32_t tbl = SLOT_TABLES ? (uint32_t)slot : (uint32_t)(w * npw + t_next);
-                            v_build_low_rows(base + pl.lw + tbl * F_BYTES, ma, la, r, wrap,
-                                             base + pl.sb + (uint32_t)l_buf * (sch * TOK * 2) + (uint32_t)l_sic * (TOK * 2), A,
-                                             p.reference, lane);
-                            if (lane == 0)
-                                asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(base + pl.rec + rec * REC + 12),
-                                             "r"(r.w | ((tbl + 1u) << 8)) : "memory");
-                            t_next = t_next + 1 == npw ? 0 : t_next + 1;
-                            ++t_out;
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0 && alive) mbar_arrive(bar_full + slot * 8);   // publishes the table rows; the copy warp adds the bytes
-                    if ((slot += NDW) >= nf) slot -= nf;
-                    if ((rec += NDW) >= nrec) rec -= nrec;
-                    if ((l_sic += NDW) >= sch) { l_sic -= sch; l_buf = l_buf == 2 ? 0 : l_buf + 1; }
-                }
-            }
+            if ((slot += HW) >= nf) slot -= nf;
+            unit = nunit;
+            i = ni;
         }
         if (!alive) v_sleep_ms();
         return;
     }
 
     // ---------------------------------------------------------------------- chain warp
-    const int pairA = 16 * (lane & 3) + (lane >> 2), pairB = pairA + 8;   // this lane's channel pairs
-    // ldmatrix row address of this lane inside four token rows: matrix lane/8 = token, row lane%8 = 16-byte chunk
-    const uint32_t lm_off = (uint32_t)((lane >> 3) * D + (lane & 7) * 16);
-    uint32_t accA = 0, accB = 0;
-    bool alive = true;
-    const int nsf = n / TOK;                                           // full stages
-    const int nrec = 2 * nf;                                           // records: one per stage, a ring of two ring lengths
-    // Registers of one group of 8 tokens: per token [pair A even, odd | pair B even, odd] high bytes and low bytes, and
-    // the 8 probabilities.
+    constexpr int NB = GH <= 2 ? 4 : 2;            // groups of 8 tokens in flight
+    const int half = wi & 1, h0 = (wi >> 1) * GH;                          // its channels and its first head
+    const int pair = 32 * half + 8 * (lane & 3) + (lane >> 2);             // this lane's channel pair
+    // row this lane names in an ldmatrix over a group of 8 tokens: matrix lane/8 = tokens 2 (lane/8) and the next, row
+    // lane%8 = chunk (lane%8)/2 of the half, token (lane%8)%2
+    const uint32_t lm_tok = 2 * (lane >> 3) + (lane & 1), lm_chunk = (4 * half + ((lane >> 1) & 3)) * 16;
+    const uint32_t lm_off = lm_tok * D + lm_chunk, lm_low = pool + lm_chunk;
+    const uint32_t s_off = OFF_S + h0 * TOK * 2, low_off = OFF_LOW + h0 * TOK * 2 + lm_tok * (NG * 2);
+    // Registers of one group of 8 tokens: high bytes [even token's pair | odd token's pair], the heads' low bytes likewise,
+    // and the heads' probabilities
     struct Grp {
-        uint32_t h[8], l[8];
-        uint4 s;
+        uint32_t h[4], l[GH][4];
+        uint4 s[GH];
     };
-    auto ldm = [](uint32_t (&r)[8], int o, uint32_t a) {
+    auto ldm = [](uint32_t* r, uint32_t a) {
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                     : "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]) : "r"(a));
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
     };
-    // A stage without flagged tokens (most of them) has the constant low byte 0x80 everywhere: it is consumed by a
-    // second copy of the stage body that neither loads the table nor holds its words (LEAN).  la: the low-byte table of
-    // a stage WITH flagged tokens (0 for the others): the table of its ring slot, or one of the head's own tables.
-    auto fetch_high = [&](Grp& r, uint32_t fa, uint32_t sa, int grp) {
-        const uint32_t a = (uint32_t)grp * (8 * D) + lm_off;
-        ldm(r.h, 0, fa + a);
-        ldm(r.h, 4, fa + a + 4 * D);
-        r.s = lds128(sa + grp * 16);
-    };
-    auto fetch_low = [&](Grp& r, uint32_t la, int grp) {
-        const uint32_t a = (uint32_t)grp * (8 * D) + lm_off;
-        ldm(r.l, 0, la + a);
-        ldm(r.l, 4, la + a + 4 * D);
-    };
-    auto consume = [&](const Grp& r, auto lean) {
+    auto fetch = [&](Grp& r, uint32_t sl, int grp) {
+        ldm(r.h, sl + (uint32_t)grp * (8 * D) + lm_off);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const __half2 sd = v_dup(u4w(r.s, u >> 1), u & 1);
-            if (decltype(lean)::value) {
-                accA = v_fma(__byte_perm(r.h[u], 0x80808080u, 0x1404), sd, accA);
-                accB = v_fma(__byte_perm(r.h[u], 0x80808080u, 0x3424), sd, accB);
-            } else {
-                accA = v_fma(__byte_perm(r.h[u], r.l[u], 0x1504), sd, accA);
-                accB = v_fma(__byte_perm(r.h[u], r.l[u], 0x3726), sd, accB);
-            }
+        for (int g = 0; g < GH; ++g) r.s[g] = lds128(sl + s_off + g * (TOK * 2) + grp * 16);
+    };
+    uint4 low[GH];                                 // places of the low bytes of this lane's token of the stage's groups
+    auto places = [&](uint32_t sl) {
+#pragma unroll
+        for (int g = 0; g < GH; ++g) low[g] = lds128(sl + low_off + g * (TOK * 2));
+    };
+    auto fetch_low = [&](Grp& r, int grp) {
+#pragma unroll
+        for (int g = 0; g < GH; ++g) {
+            const uint32_t w = u4w(low[g], grp >> 1);
+            ldm(r.l[g], lm_low + 2 * (grp & 1 ? w >> 16 : w & 0xFFFFu));
         }
     };
-    int slot = 0, sic = 0, buf = 0, crec = 0;                          // of the current stage: % nf, % sch, chunk % 3, % 2 nf
+    uint32_t acc[GH];
+    auto token = [&](const Grp& r, int u, bool with_low) {
+        uint32_t k = 0;
+        if (!with_low) k = __byte_perm(r.h[u >> 1], 0x80808080u, u & 1 ? 0x3424 : 0x1404);
+#pragma unroll
+        for (int g = 0; g < GH; ++g) {
+            if (with_low) k = __byte_perm(r.h[u >> 1], r.l[g][u >> 1], u & 1 ? 0x3726 : 0x1504);
+            acc[g] = v_fma(k, v_dup(u4w(r.s[g], u >> 1), u & 1), acc[g]);
+        }
+    };
+    bool alive = true;
+    int slot = 0;
     uint32_t parity = 0;
-    auto f_addr = [&]() { return rbase + (uint32_t)slot * F_BYTES; };
-    auto s_addr = [&]() { return base + pl.sb + (uint32_t)buf * (sch * TOK * 2) + (uint32_t)sic * (TOK * 2); };
-    // the stage's table: the one of its ring slot (which holds the constant for a stage without flagged tokens, so
-    // that form runs one copy of the stage body only: the second copy costs it more in instruction fetch than the
-    // skipped loads save - 31.8 against 29.0 us), or from its record (word 3: flagged rows | (table + 1) << 8;
-    // 0 = no flagged token -> 0)
-    auto l_addr = [&]() -> uint32_t {
-        if (SLOT_TABLES) return base + pl.lw + (uint32_t)slot * F_BYTES;
-        const uint32_t w = lds32(base + pl.rec + (uint32_t)crec * REC + 12);
-        return w ? base + pl.lw + ((w >> 8) - 1u) * F_BYTES : 0u;
-    };
-    Grp ra, rb;
-    uint32_t fa = f_addr(), sa = s_addr(), la = 0;
-    if (nst > 0) {
-        alive = mbar_wait(bar_full, 0);
-        if (alive) la = l_addr();
-        if (alive && nsf > 0) {
-            fetch_high(ra, fa, sa, 0);
-            if (la) fetch_low(ra, la, 0);
-        }
-    }
-    // One full stage per iteration, straight-line: groups alternate between ra and rb, the group after next is
-    // fetched while one is consumed; on entry ra holds group 0 of the stage.
+    const int nsf = n / TOK, rest = n - nsf * TOK;
 #pragma unroll 1
-    for (int left = nsf; left > 0 && alive; --left) {
-        const int cslot = slot;
-        if (++slot == nf) { slot = 0; parity ^= 1u; }
-        if (++sic == sch) { sic = 0; buf = buf == 2 ? 0 : buf + 1; }
-        if (++crec == nrec) crec = 0;
-        const uint32_t nfa = f_addr(), nsa = s_addr();
-        uint32_t nla = 0;
-        auto stage = [&](auto lean) {
-            uint32_t landed = 0;
+    for (int unit = first_unit; unit < p.units; unit += stride) {
 #pragma unroll
-            for (int ga = 0; ga < 8; ga += 2) {
-                fetch_high(rb, fa, sa, ga + 1);
-                if (!decltype(lean)::value) fetch_low(rb, la, ga + 1);
-                consume(ra, lean);
-                if (ga < 6) {
-                    fetch_high(ra, fa, sa, ga + 2);
-                    if (!decltype(lean)::value) fetch_low(ra, la, ga + 2);
-                    // the next stage has normally landed long ago (the ring is several stages deep): probe its barrier
-                    // two groups before the answer is needed, so that the probe's latency is hidden; then its record
-                    if (ga == 2 && left > 1) landed = mbar_test(bar_full + slot * 8, parity);
-                    if (ga == 4 && left > 1) nla = l_addr();          // (valid only if it had landed)
-                } else if (left > 1) {
-                    if (__builtin_expect(!landed, 0)) {
-                        alive = mbar_wait(bar_full + slot * 8, parity);
-                        nla = l_addr();
+        for (int g = 0; g < GH; ++g) acc[g] = 0;
+        Grp r[NB];
+        uint32_t sl = ring + (uint32_t)slot * SLOT, any = 0;
+        if (alive && nst > 0) {
+            alive = mbar_wait(bar_full + slot * 8, parity);
+            any = lds32(sl + OFF_ANY);
+#pragma unroll
+            for (int j = 0; j < NB; ++j) fetch(r[j], sl, j);
+        }
+        // One full stage per iteration, straight-line; on entry r holds the bytes of its first NB groups.
+#pragma unroll 1
+        for (int left = nsf; left > 0 && alive; --left) {
+            const int cslot = slot;
+            if (++slot == nf) { slot = 0; parity ^= 1u; }
+            const uint32_t nsl = ring + (uint32_t)slot * SLOT, nbar = bar_full + slot * 8;
+            const bool more = left > 1 || rest > 0;
+            uint32_t nany = 0;
+            auto stage = [&](auto with_low) {
+                constexpr bool LOW = decltype(with_low)::value;
+#pragma unroll
+                for (int j = 0; j < NG; ++j) {
+                    if (j + NB == NG) {
+                        // the next stage (when there is none: stale bytes, unused)
+                        if (more) alive = mbar_wait(nbar, parity);
+                        nany = lds32(nsl + OFF_ANY);
                     }
-                    if (alive) {                                      // first group of the next stage
-                        fetch_high(ra, nfa, nsa, 0);
-                        if (nla) fetch_low(ra, nla, 0);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) token(r[j % NB], u, LOW);
+                    if (j + NB < NG) {
+                        fetch(r[j % NB], sl, j + NB);
+                        if (LOW) fetch_low(r[j % NB], j + NB);
+                    } else {
+                        fetch(r[j % NB], nsl, j + NB - NG);
                     }
                 }
-                consume(rb, lean);
+            };
+            if (__builtin_expect(any == 0, 1)) {
+                stage(std::false_type{});
+            } else {
+                places(sl);
+#pragma unroll
+                for (int j = 0; j < NB; ++j) fetch_low(r[j], j);
+                stage(std::true_type{});
             }
-        };
-        if constexpr (SLOT_TABLES) {
-            stage(std::false_type{});               // (the only copy of the stage body in this instantiation)
-        } else {
-            if (la) stage(std::false_type{});
-            else stage(std::true_type{});
+            // the stage is consumed: hand back its ring slot
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_free + cslot * 8);
+            sl = nsl;
+            any = nany;
         }
-        // the stage is consumed: hand back its ring slot
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_free + cslot * 8);
-        fa = nfa; sa = nsa; la = nla;
-    }
-    const int tail = n - nsf * TOK;
-    if (tail > 0 && alive) {
-        // last, partial stage, token by token (rows of the slot beyond the last token hold stale bytes, never used)
-        if (nsf > 0) alive = mbar_wait(bar_full + slot * 8, parity);
-        if (alive) {
-            if (nsf > 0) la = l_addr();
-#pragma unroll 1
-            for (int t = 0; t < tail; ++t) {
-                const uint32_t hw = lds16(fa + (uint32_t)t * D + pairA * 2) | (lds16(fa + (uint32_t)t * D + pairB * 2) << 16);
-                const uint32_t lw = la ? lds16(la + (uint32_t)t * D + pairA * 2) | (lds16(la + (uint32_t)t * D + pairB * 2) << 16)
-                                       : 0x80808080u;
-                const uint32_t sb = lds16(sa + t * 2);
-                accA = hfma2_bits(__byte_perm(hw, lw, 0x1504), sb | (sb << 16), accA);
-                accB = hfma2_bits(__byte_perm(hw, lw, 0x3726), sb | (sb << 16), accB);
+        if (rest > 0) {
+            // last, partial stage (rows beyond the last token hold stale bytes: not accumulated)
+            if (alive) {
+                if (any != 0) places(sl);
+#pragma unroll
+                for (int k = 0; k < NG; ++k) {
+                    if (8 * k >= rest) break;
+                    fetch(r[0], sl, k);
+                    if (any != 0) {
+                        fetch_low(r[0], k);
+                    } else {
+#pragma unroll
+                        for (int g = 0; g < GH; ++g)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) r[0].l[g][e] = 0x80808080u;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (8 * k + u < rest) token(r[0], u, true);
+                }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_free + slot * 8);
+            if (++slot == nf) { slot = 0; parity ^= 1u; }
+        }
+#pragma unroll
+        for (int g = 0; g < GH; ++g) {
+            const size_t at = ((size_t)unit * NH + h0 + g) * 64 + pair;
+            if (p.res) {
+                const uint32_t t = reinterpret_cast<const uint32_t*>(p.res)[at];
+                const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&acc[g]));
+                const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&t));
+                const __half2 c = __floats2half2_rn(a.x + b.x, a.y + b.y);
+                acc[g] = *reinterpret_cast<const uint32_t*>(&c);
+            }
+            reinterpret_cast<uint32_t*>(p.o)[at] = alive ? acc[g] : 0x7E007E00u;
         }
     }
-    if (p.res) {
-        const uint32_t* r = reinterpret_cast<const uint32_t*>(p.res) + (size_t)bh * 64;
-        auto add = [](uint32_t acc, uint32_t t) {
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&acc));
-            const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&t));
-            const __half2 c = __floats2half2_rn(a.x + b.x, a.y + b.y);
-            return *reinterpret_cast<const uint32_t*>(&c);
-        };
-        accA = add(accA, r[pairA]);
-        accB = add(accB, r[pairB]);
-    }
-    uint32_t* o = reinterpret_cast<uint32_t*>(p.o) + (size_t)bh * 64;
-    o[pairA] = alive ? accA : 0x7E007E00u;
-    o[pairB] = alive ? accB : 0x7E007E00u;
 }
 
 }  // namespace akv

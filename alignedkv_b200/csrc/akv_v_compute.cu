@@ -474,71 +474,56 @@ static int launch_v_fast(const VParams& p, int BH, cudaStream_t st) {
     return cuda_status(cudaGetLastError(), "v_cache_compute launch");
 }
 
-// ---- launch of the branch-free streaming form for multi-head attention (v_chain_kernel)
-// Ring sizes follow from how many units ((batch, head) pairs) have to share an SM so that the whole grid is resident
-// at once (the kernel is a pure stream: a second wave would start with cold rings): shared memory per unit = SM
-// capacity / units per SM, of which the probability buffers and the side ring take a fixed part and the two rings
-// (high bytes, low-byte table: 16 KB per stage) the rest.
-struct VChainCfg {
-    int upc, gh, ndw, nf, nside, sch, npt, smem;
-};
-// heads: (batch, query head) rows; gh: heads that share a ring (1, or the group size: the query heads of a KV head)
-static VChainCfg v_chain_config(long long heads, int gh, int reference) {
-    const Tuning& t = tuning();
-    VChainCfg c;
-    c.gh = gh;
-    // one head per ring: two rings per CTA, whose eight warps put the chain and decision warps on different schedulers
-    c.upc = (gh == 1 && heads >= 2) ? 2 : 1;
-    if (gh == 1 && t.v_upc > 0) c.upc = t.v_upc;
-    const int budget = max_dyn_smem();
-    // decision warps per head: a stage with flagged tokens costs its warp three out-of-line calls (copy issue, row
-    // build, row restore), and two warps per head fell behind the chain on them; four have the time.  They need
-    // schedulers of their own, which two rings of one head each can give them.
-    c.ndw = (c.upc == 2 && gh == 1 && tuning().v_ndw != 2) ? 4 : 2;
-    c.nside = (reference ? 128 : 64) * c.ndw;              // (each decision warp owns a part: at least a stage's 64 rows)
-    c.sch = 16;
-    if (t.v_nside >= 64 * c.ndw) c.nside = t.v_nside;
-    // low-byte tables per head: two per decision warp where they fit (a third stage with flagged tokens among a warp's
-    // stages in flight is rare and only makes that warp wait for the oldest one), one with four heads on a ring
-    c.npt = c.upc * gh >= 4 ? 2 : 4;
-    if (t.v_npt == 2 || t.v_npt == 4 || t.v_npt == 6 || t.v_npt == 8) c.npt = t.v_npt;
-    // ring depth: the decision warp runs a ring ahead, 2 nf stages <= a chunk; one head per ring gains nothing beyond
-    // four stages (measured: 4, 6 and 8 alike), heads that share a ring wait for each other and use what fits
-    int nf = gh == 1 ? 4 : c.sch / 2;
-    if (t.v_nf > 0 && t.v_nf < nf) nf = t.v_nf;
-    nf -= nf % c.ndw;                                      // a ring slot's stages all belong to one decision warp
-    if (nf < c.ndw) nf = c.ndw;
-    // (one head per ring: a table per ring slot)
-    while (nf > c.ndw && vch::plan(nf, c.nside, c.sch, gh == 1 ? nf : c.npt, c.upc, gh).bytes > budget) nf -= c.ndw;
-    c.nf = nf;
-    if (gh == 1) c.npt = nf;
-    c.smem = vch::plan(c.nf, c.nside, c.sch, c.npt, c.upc, gh).bytes;
-    return c;
-}
-
-template <int UPC, int GH, int NDW>
-static int launch_v_chain_u(VParams& p, const VChainCfg& c, long long heads, cudaStream_t st) {
+// ---- launch of the chain kernel (akv_v_chain.cuh)
+// NH query heads per unit, GH of them per chain warp, UPC units per CTA at a time (one CTA per SM).
+template <int NH, int GH, int UPC>
+static int launch_v_chain_u(VParams& p, long long units, cudaStream_t st) {
     static bool configured[64] = {false};   // the attribute is per device (one array per instantiation)
+    const int budget = max_dyn_smem();
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(v_chain_kernel<UPC, GH, NDW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             max_dyn_smem());
+        cudaError_t e = cudaFuncSetAttribute(v_chain_kernel<NH, GH, UPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
         if (e != cudaSuccess) return cuda_status(e, "v_cache_compute smem attribute");
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    AKV_REQUIRE(c.smem <= max_dyn_smem(), AKV_ERR_CUDA, "v_cache_compute: %d bytes of shared memory are too many", c.smem);
-    p.nf = c.nf; p.nside = c.nside; p.sch = c.sch; p.npt = c.npt;
-    p.units = (int)(heads / GH);
-    const int grid = (p.units + UPC - 1) / UPC;
-    launch_chained(v_chain_kernel<UPC, GH, NDW>, dim3(grid), dim3(NDW == 2 ? ((1 + NDW) * UPC * GH + UPC) * 32 : 512), (size_t)c.smem, st, p);
+    constexpr int HW = vch::helpers(UPC, NH);
+    int nf = 16;
+    if (tuning().v_nf > 0 && tuning().v_nf < nf) nf = tuning().v_nf;
+    nf = nf < 2 * HW ? 2 * HW : nf - nf % HW;      // (a helper arms a stage while it prepares its next one: at least two each)
+    while (nf > 2 * HW && UPC * vch::plan(nf, UPC, NH).bytes > budget) nf -= HW;
+    const int smem = UPC * vch::plan(nf, UPC, NH).bytes;
+    AKV_REQUIRE(smem <= budget, AKV_ERR_CUDA, "v_cache_compute: %d bytes of shared memory are too many", smem);
+    p.nf = nf;
+    p.units = (int)units;
+    p.share = p.group / NH;
+    const int grid = units < sm_count() ? (int)units : sm_count();
+    launch_chained(v_chain_kernel<NH, GH, UPC>, dim3(grid), dim3(UPC * (2 * NH / GH + HW) * 32), (size_t)smem, st, p);
     return cuda_status(cudaGetLastError(), "v_cache_compute launch");
+}
+
+static int launch_v_chain(VParams& p, long long BH, cudaStream_t st) {
+    // One unit per SM while there are no more units than SMs, else two; with still more units of one head four (batch 16 x
+    // 32 heads x 4096 tokens, two against four: 46 us both while few tokens are flagged, 286 against 186 us when all are),
+    // units of several heads stay at two: their pools are twice as large.
+    // Grouped queries: a unit per query head while the heads fit one wave (8 KV heads x 4, batch 8 x 8192 tokens: 50 us
+    // against 67 with the group in one unit; 4 x 8, batch 4 x 2048: 12 against 32), else a unit per KV head, its heads on
+    // four chain warps while every unit has an SM to itself (batch 64: 200 us against 320 with a chain warp pair per head).
+    const long long sms = sm_count(), heads = BH * p.group;
+    const int form = tuning().v_gqa_form;
+    if (p.group == 1 || form == 1 || (form == 0 && heads <= 2 * sms)) {
+        if (heads <= sms) return launch_v_chain_u<1, 1, 1>(p, heads, st);
+        return heads <= 2 * sms ? launch_v_chain_u<1, 1, 2>(p, heads, st) : launch_v_chain_u<1, 1, 4>(p, heads, st);
+    }
+    if (p.group == 2) return launch_v_chain_u<2, 2, 2>(p, BH, st);
+    if (p.group == 4) return BH <= sms ? launch_v_chain_u<4, 2, 1>(p, BH, st) : launch_v_chain_u<4, 4, 2>(p, BH, st);
+    return BH <= sms ? launch_v_chain_u<8, 4, 1>(p, BH, st) : launch_v_chain_u<8, 4, 2>(p, BH, st);
 }
 
 // true when launch_v_compute_probe runs the streaming kernel, which can compute the threshold bytes itself
 bool v_compute_takes_probe(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* s,
                            const uint8_t* o, int group, int D, int s_last_dim, int n) {
-    return D == 128 && (group == 1 || group == 2 || group == 4) &&
+    return D == 128 && (group == 1 || group == 2 || group == 4 || group == 8) &&
            aligned16(first8) && aligned16(mid4) &&
            aligned16(last4) && (n == 0 || (aligned16(s) && s_last_dim % 8 == 0 && ((n + 7) & ~7) <= s_last_dim)) &&
            ((reinterpret_cast<uintptr_t>(o) & 3u) == 0);
@@ -562,27 +547,16 @@ int launch_v_compute_res(const uint8_t* first8, const uint8_t* mid4, const uint8
     p.o = reinterpret_cast<uint16_t*>(o);
     p.max_seq_len = max_seq_len; p.D = D; p.s_last_dim = s_last_dim; p.n = n; p.reference = reference;
     p.group = group;
-    p.nf = p.nside = p.sch = p.units = 0;
+    p.nf = p.units = 0;
+    p.share = 1;
     const int BH = bsz * H;
     const bool fast = v_compute_takes_probe(first8, mid4, last4, s, o, group, D, s_last_dim, n);
     AKV_REQUIRE(fast || !test_o, AKV_ERR_SHAPE, "v_cache_compute: the probe form needs the streaming kernel");
-    const long long heads = (long long)BH * group;
-    const bool chain = fast && !reference && tuning().v_impl == 0 && heads < (1ll << 30);
+    // (all planes read: the producer-transposed kernel is faster, 68 against 148 us at batch 8 x 32 heads x 4096 tokens,
+    // but has no form for eight heads per KV head)
+    const bool chain = fast && (group == 8 || (!reference && tuning().v_impl == 0)) && (long long)BH * group < (1ll << 30);
     AKV_REQUIRE(chain || !p.res, AKV_ERR_SHAPE, "v_cache_compute: the residual form needs the chain kernel");
-    if (chain) {
-        // grouped queries: the heads of a KV head share one ring of high bytes in a CTA (gh = group); the form with
-        // one ring per query head, whose heads meet in L2, stays selectable for measurements
-        // (measured at 8192 tokens, 8 KV heads x 4: batch 8: 98 us grouped kernel, 84 shared ring, 65 ring per head;
-        // batch 16: 117 / 102 / 125): a ring per head while the heads fit one wave of CTAs, else the shared ring
-        const int w = tuning().v_gqa_form;
-        const bool per_head = group == 1 || w == 1 || (w == 0 && heads <= 2ll * sm_count());
-        const int gh = per_head ? 1 : group;
-        const VChainCfg c = v_chain_config(heads, gh, reference);
-        if (gh == 4) return launch_v_chain_u<1, 4, 2>(p, c, heads, st);
-        if (gh == 2) return launch_v_chain_u<1, 2, 2>(p, c, heads, st);
-        if (c.upc == 2) return c.ndw == 4 ? launch_v_chain_u<2, 1, 4>(p, c, heads, st) : launch_v_chain_u<2, 1, 2>(p, c, heads, st);
-        return launch_v_chain_u<1, 1, 2>(p, c, heads, st);
-    }
+    if (chain) return launch_v_chain(p, BH, st);
     if (fast && group == 1) return launch_v_fast<1, 6, 2, 1>(p, BH, st);
     if (fast && group == 2) return launch_v_fast<2, 6, 2, 2>(p, BH, st);
     if (fast && group == 4) return launch_v_fast<4, 6, 2, 2>(p, BH, st);
@@ -606,7 +580,7 @@ int launch_v_compute_probe(const uint8_t* first8, const uint8_t* mid4, const uin
 bool v_compute_adds_residual(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* s,
                              const uint8_t* o, int bsz, int H, int group, int D, int s_last_dim, int n, int reference) {
     return v_compute_takes_probe(first8, mid4, last4, s, o, group, D, s_last_dim, n) && !reference &&
-           tuning().v_impl == 0 && (long long)bsz * H * group < (1ll << 30);
+           (tuning().v_impl == 0 || group == 8) && (long long)bsz * H * group < (1ll << 30);
 }
 
 int launch_v_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* s,
