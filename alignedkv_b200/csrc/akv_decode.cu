@@ -179,15 +179,7 @@ append_flush_kernel(uint32_t* __restrict__ restk, uint32_t* __restrict__ restv, 
 }
 
 // ------------------------------------------------------------------ softmax (+ residual scores, class maxima, probe)
-// grid B*Hq, block 256.  Row = [0, qn) aligned scores | [qn, qn+rest) residual scores | -inf up to R.
-// CACHED: the row has at most 256*SM_REGS scores and every thread keeps its share in registers, so the row is read
-// from memory once instead of three times.  The per-thread and cross-thread summation order is the same either way.
-// PROBE (and first8 != nullptr): the magnitude probe (V_cache.cu:104-119; see v_probe_kernel) of this row follows in
-// the same CTA from the class maxima it has just found, and lands in test_o.  Both forms pay when the grid is a wave
-// or two and the step is bound by the latency of its kernel chain; with many rows the plain form plus a separate
-// probe launch keeps more CTAs per SM and is faster.
-constexpr int SM_REGS = 32;
-constexpr int SM_REGS_512 = 34;   // with 512 threads: rows of up to 17408 scores (16384 cached tokens plus residual blocks)
+// Row = [0, qn) aligned scores | [qn, qn+rest) residual scores | -inf up to R.
 // Score t of a row as the fp32 softmax sees it: the fp16 score, plus (optional) the additive fp16 mask of its batch
 // row, added in fp16 as the reference's in-place `scores += mask` on fp16 tensors does (model/KVCache_AlignedKV.py:119-120).
 __device__ __forceinline__ float masked_score(const uint16_t* __restrict__ row, const __half* __restrict__ mrow, int t) {
@@ -195,50 +187,295 @@ __device__ __forceinline__ float masked_score(const uint16_t* __restrict__ row, 
     if (mrow) s = __hadd(s, mrow[t]);
     return __half2float(s);
 }
-// Scores of the residual tokens of one (batch, query head) row, by a CTA of 256 threads: thread = (token tid / 4,
+// Scores of the residual tokens of one (batch, query head) row, by 256 threads: thread = (token tid / 4,
 // quarter tid % 4 of the channels in 16-byte pieces), all loads of a row in flight at once, fp32 dot product rounded to
 // fp16, then divided by sqrt(D) and rounded again, which is what `matmul(q, restk^T) / sqrt(D)` on fp16 tensors
-// produces (k_cache_file.py:156-157).  Only tokens with t_lo <= qn + r < t_hi are written (a row split across CTAs).
+// produces (k_cache_file.py:156-157).  Returned by the first thread of each token's four, 0 <= tid / 4 < rest < 64.
+__device__ __forceinline__ __half residual_score(const __half* __restrict__ qr, const __half* __restrict__ restk, int b, int h,
+                                                 int H, int D, int rest, float sqrt_d, bool wanted) {
+    const int r = threadIdx.x >> 2, c = threadIdx.x & 3;
+    float acc = 0.f;
+    if (wanted && r < rest) {
+        const __half* kr = restk + (((size_t)b * BLK + r) * H + h) * D;
+#pragma unroll 4
+        for (int d = c * 8; d < D; d += 32) {
+            const uint4 kv = *reinterpret_cast<const uint4*>(kr + d), qv = *reinterpret_cast<const uint4*>(qr + d);
+            const __half2* k2 = reinterpret_cast<const __half2*>(&kv);
+            const __half2* q2 = reinterpret_cast<const __half2*>(&qv);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 kf = __half22float2(k2[i]), qf = __half22float2(q2[i]);
+                acc = fmaf(qf.x, kf.x, acc);
+                acc = fmaf(qf.y, kf.y, acc);
+            }
+        }
+    }
+    acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
+    acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
+    return __float2half_rn(__half2float(__float2half_rn(acc)) / sqrt_d);
+}
+// The same for a CTA of 256 threads, written into the row; only tokens with t_lo <= qn + r < t_hi (a row split across CTAs).
 __device__ __forceinline__ void residual_scores(uint16_t* __restrict__ row, const __half* __restrict__ qr,
                                                 const __half* __restrict__ restk, int b, int h, int H, int D, int qn,
                                                 int rest, float sqrt_d, int t_lo, int t_hi) {
-    const int tid = threadIdx.x;
-    for (int r0 = 0; r0 < rest; r0 += 64) {       // (the residual buffer holds at most 64 tokens: one round)
-        const int r = r0 + (tid >> 2), c = tid & 3;
-        const bool mine = r < rest && qn + r >= t_lo && qn + r < t_hi;
-        float acc = 0.f;
-        if (mine) {
-            const __half* kr = restk + (((size_t)b * BLK + r) * H + h) * D;
-            for (int d = c * 8; d < D; d += 32) {
-                const uint4 kv = *reinterpret_cast<const uint4*>(kr + d), qv = *reinterpret_cast<const uint4*>(qr + d);
-                const __half2* k2 = reinterpret_cast<const __half2*>(&kv);
-                const __half2* q2 = reinterpret_cast<const __half2*>(&qv);
+    const int r = threadIdx.x >> 2;
+    const bool mine = r < rest && qn + r >= t_lo && qn + r < t_hi;
+    const __half v = residual_score(qr, restk, b, h, H, D, rest, sqrt_d, mine);
+    if (mine && (threadIdx.x & 3) == 0) row[qn + r] = __half_as_ushort(v);
+}
+
+// One CTA per row, which stays in registers: thread = vectors tid, tid + NT, ... of 8 consecutive scores, VPT of them.
+// One 16-byte load and store per vector; the residual tokens' scores go straight from their dot products to the vectors
+// that hold them.  A thread's vectors all have the same eight residue classes (token index mod 32: 8 (tid % 4) + 0..7), so
+// the classes' largest probabilities and first positions are running maxima of (probability bits << 16 | 65535 - position)
+// per element, reduced over the CTA at the end.  Then, in the same CTA: the magnitude probe of the row (V_cache.cu:104-119;
+// see v_probe_kernel), its chain by the first D/2 threads, and, beside it, the residual tokens' part of the output
+// half(sum_r p[qn + r] * restv[r]) (extension/v_cache_file.py:189) by the others, for the P.V kernel to add.
+// The residual values come into shared memory by asynchronous copies started first, so that the sum at the end waits for
+// nothing.  With few rows the chain of loads, three reductions and the probe's gathers counts, with many the instructions
+// per score: about 14, of which the division takes three - quotient by the reciprocal of the sum, then one residual
+// correction (Markstein 1990: correctly rounded, as the division it replaces).  MINB: CTAs per SM.
+// Measured (cold, one launch): 256 rows of 4160 scores 8.9 us, 512 rows of 1088 with 48 residual tokens 11.0, 32 rows of
+// 16448 9.7, 2048 rows of 8192 43.4.  The form before it - scores one at a time, 17 to 34 a thread, exponential, division
+// and checks at 105 instructions per score; for the last, probe and residual part in launches of their own - took 11.2,
+// 21.9, 12.6 and 45.9 + 14.1 + 25.5.
+template <int NT, int VPT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __half* __restrict__ restk,
+                   uint16_t* __restrict__ pval, int32_t* __restrict__ pidx, float* __restrict__ stats,
+                   const uint8_t* __restrict__ first8, uint16_t* __restrict__ test_o, int max_seq_len, int H, int G, int D,
+                   int R, int qn, int rest, float sqrt_d, const __half* __restrict__ mask, long long mask_stride,
+                   const __half* __restrict__ restv, uint16_t* __restrict__ res) {
+    constexpr int NW = NT / 32, PARTS = 4;
+    __shared__ float red[2][NW];
+    __shared__ __align__(16) uint32_t key[NW][TOPK];
+    __shared__ __align__(16) uint16_t rs[BLK];                   // residual scores, then their probabilities
+    __shared__ float part[PARTS][256];
+    __shared__ __align__(16) uint8_t rows[TOPK][256];            // the probe's rows
+    extern __shared__ __align__(16) uint8_t dyn[];               // residual values [rest][D] (res), then exponentials [R] (NT 1024)
+    pdl_enter();
+    const int bhq = blockIdx.x, Hq = H * G, b = bhq / Hq, h = (bhq - b * Hq) / G;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint16_t* row = s + (size_t)bhq * R;
+    const int nv = R >> 3, qv = qn >> 3, len = qn + rest;
+    constexpr uint32_t NEG = 0xFC00FC00u;                        // two -inf
+    const bool with_res = res != nullptr && rest > 0;
+    if (with_res) {
+        const int per = D >> 3;                                  // 16-byte pieces of a row
+        for (int i = tid; i < rest * per; i += NT) {
+            const int r = i / per, c = i - r * per;
+            cp_async16(smem_u32(dyn) + i * 16, restv + (((size_t)b * BLK + r) * H + h) * D + c * 8);
+        }
+        cp_async_commit();
+    }
+    uint4 w[VPT];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 kf = __half22float2(k2[i]), qf = __half22float2(q2[i]);
-                    acc = fmaf(qf.x, kf.x, acc);
-                    acc = fmaf(qf.y, kf.y, acc);
-                }
+    for (int i = 0; i < VPT; ++i) {
+        const int v = tid + NT * i;
+        w[i] = v < qv ? reinterpret_cast<const uint4*>(row)[v] : make_uint4(NEG, NEG, NEG, NEG);
+    }
+    if (tid < 256) {
+        const __half v = residual_score(q + (size_t)bhq * D, restk, b, h, H, D, rest, sqrt_d, true);
+        if ((tid & 3) == 0) rs[tid >> 2] = (tid >> 2) < rest ? __half_as_ushort(v) : (uint16_t)0xFC00u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int v = tid + NT * i;
+        if (v >= qv && v < nv) w[i] = reinterpret_cast<const uint4*>(rs)[v - qv];
+    }
+    if (mask) {     // additive fp16 mask, added in fp16 as the reference's in-place `scores += mask` does (KVCache_AlignedKV.py:119-120)
+        const __half* mrow = mask + (size_t)b * mask_stride;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const int t = 8 * (tid + NT * i);
+            __half2* x = reinterpret_cast<__half2*>(&w[i]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __half m0 = t + 2 * j < len ? mrow[t + 2 * j] : __half(0.f), m1 = t + 2 * j + 1 < len ? mrow[t + 2 * j + 1] : __half(0.f);
+                x[j] = __hadd2(x[j], __halves2half2(m0, m1));
             }
         }
-        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
-        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
-        if (mine && c == 0) row[qn + r] = __half_as_ushort(__float2half_rn(__half2float(__float2half_rn(acc)) / sqrt_d));
+    }
+    // maximum
+    __half2 m2 = __halves2half2(__ushort_as_half((unsigned short)0xFC00u), __ushort_as_half((unsigned short)0xFC00u));
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m2 = __hmax2(m2, reinterpret_cast<const __half2*>(&w[i])[j]);
+    float m = fmaxf(__low2float(m2), __high2float(m2));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+    if (lane == 0) red[0][warp] = m;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NW; ++k) m = fmaxf(m, red[0][k]);
+    // sum of exponentials (fp32, as F.softmax(scores.float()) does; model/KVCache_AlignedKV.py:121)
+    float sum = 0.f;
+    // Rows beyond 12288 scores also exist as shards of a sequence, whose probabilities agree bit for bit with one device's as
+    // far as the sums do: their order of additions stays that of a 512-thread CTA that owns every 512th score.
+    float* ex = reinterpret_cast<float*>(dyn + (with_res ? (size_t)rest * D * 2 : 0));
+    float x[VPT][8];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int v = tid + NT * i;
+        const bool in = v < nv;                                  // (scores beyond `len` are -inf: exactly 0 unless all are)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(reinterpret_cast<const __half2*>(&w[i])[j]);
+            x[i][2 * j] = in ? expf(f.x - m) : 0.f;
+            x[i][2 * j + 1] = in ? expf(f.y - m) : 0.f;
+        }
+        if (NT == 1024) {
+            if (in) {
+                reinterpret_cast<float4*>(ex)[2 * v] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
+                reinterpret_cast<float4*>(ex)[2 * v + 1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sum += x[i][j];
+        }
+    }
+    if (NT == 1024) {
+        __syncthreads();
+        if (tid < 512)
+#pragma unroll 8
+            for (int t = tid; t < len; t += 512) sum += ex[t];
+    }
+    constexpr int SW = NT == 1024 ? 16 : NW;                     // warps that hold sums
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) red[1][warp] = sum;
+    __syncthreads();
+    sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < SW; ++k) sum += red[1][k];
+    if (tid == 0) {
+        stats[(size_t)bhq * 2] = m;
+        stats[(size_t)bhq * 2 + 1] = sum;
+    }
+    // probabilities and class maxima over the quantized tokens (torch.max over the group axis keeps the first maximum,
+    // v_cache_file.py:128-130; probabilities are non-negative: bit patterns order like values)
+    const float inv = 1.f / sum;
+    uint32_t best[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) best[j] = 0;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int v = tid + NT * i;
+        if (v >= nv) break;
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float p[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float y = x[i][2 * j + k] * inv;
+                p[k] = fmaf(fmaf(-y, sum, x[i][2 * j + k]), inv, y);
+            }
+            const __half2 h2 = __floats2half2_rn(p[0], p[1]);
+            o[j] = *reinterpret_cast<const uint32_t*>(&h2);
+        }
+        if (v < qv) {
+            const uint32_t at = 0xFFFFu - (uint32_t)(v >> 2);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                best[2 * j] = max(best[2 * j], __byte_perm(o[j], at, 0x1054));
+                best[2 * j + 1] = max(best[2 * j + 1], __byte_perm(o[j], at, 0x3254));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (8 * v + 2 * j >= len) o[j] = 0u;
+                else if (8 * v + 2 * j + 1 >= len) o[j] &= 0xFFFFu;
+            }
+            reinterpret_cast<uint4*>(rs)[v - qv] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        reinterpret_cast<uint4*>(row)[v] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) best[j] = max(best[j], __shfl_xor_sync(0xFFFFFFFFu, best[j], o));
+    if (lane < 4) {
+        *reinterpret_cast<uint4*>(&key[warp][8 * lane]) = make_uint4(best[0], best[1], best[2], best[3]);
+        *reinterpret_cast<uint4*>(&key[warp][8 * lane + 4]) = make_uint4(best[4], best[5], best[6], best[7]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (tid < TOPK) {
+        uint32_t k = key[0][tid];
+        for (int i = 1; i < NW; ++i) k = max(k, key[i][tid]);
+        const int32_t at = k ? (int32_t)(0xFFFFu - (k & 0xFFFFu)) : 0;
+        pval[(size_t)bhq * TOPK + tid] = (uint16_t)(k >> 16);
+        pidx[(size_t)bhq * TOPK + tid] = at;
+        key[0][tid] = k >> 16;
+        key[1][tid] = (uint32_t)at;
+    }
+    if (qn == 0) return;                                         // (uniform)
+    __syncthreads();
+    const int hd = D >> 1;
+    // probe: o_test[d] = sum_j |half((first_8[row_j][d] << 8) + 0x80)| * p_j over the class maxima, rows
+    // row_j = class position * 32 + j, accumulated in fp16 in j order.  The rows are gathered by the whole CTA, 16 bytes a
+    // thread (all 32 rows of 128 bytes in one load), 256 channels at a time.
+    const uint8_t* F = first8 + (size_t)(bhq / G) * max_seq_len * D;
+    const bool vec = (reinterpret_cast<uintptr_t>(F) & 15u) == 0;
+    for (int d0 = 0; d0 < D; d0 += 256) {
+        const int dn = min(256, D - d0);
+        if (d0 > 0) __syncthreads();
+        auto src = [&](int j) { return F + (size_t)min((int)key[1][j] * TOPK + j, max_seq_len - 1) * D + d0; };
+        if (vec) {
+            const int per = dn >> 4;                             // 16-byte pieces of a row (D is a multiple of 64)
+            for (int i = tid; i < TOPK * per; i += NT)
+                *reinterpret_cast<uint4*>(&rows[i / per][16 * (i % per)]) = __ldg(reinterpret_cast<const uint4*>(src(i / per)) + i % per);
+        } else {
+            const int per = dn >> 1;
+            for (int i = tid; i < TOPK * per; i += NT)
+                *reinterpret_cast<uint16_t*>(&rows[i / per][2 * (i % per)]) = __ldg(reinterpret_cast<const uint16_t*>(src(i / per)) + i % per);
+        }
+        __syncthreads();
+        for (int c = tid; 2 * c < dn; c += NT) {
+            uint32_t acc = 0;
+#pragma unroll 8
+            for (int j = 0; j < TOPK; ++j) {
+                const uint32_t f = *reinterpret_cast<const uint16_t*>(&rows[j][2 * c]);
+                acc = hfma2_bits(__byte_perm(f, 0x80u, 0x1404) & 0x7FFF7FFFu, key[0][j] | (key[0][j] << 16), acc);
+            }
+            reinterpret_cast<uint32_t*>(test_o)[(size_t)bhq * hd + (d0 >> 1) + c] = acc;
+        }
+    }
+    if (!with_res) return;                                       // (uniform)
+    // residual part (D <= 256): item = (channel pair, share g of the tokens), fp32 sums, the shares added in order
+    const int first = NT >= 2 * hd ? hd : 0;                     // (beside the probe's chain where there are threads left)
+    const int parts = min(PARTS, (NT - first) / hd);
+    if (tid >= first && tid < first + parts * hd) {
+        const int i = tid - first, g = i / hd, c = i - g * hd;
+        const __half2* vr = reinterpret_cast<const __half2*>(dyn) + c;
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll 4
+        for (int r = g; r < rest; r += parts) {
+            const float2 f = __half22float2(vr[r * hd]);
+            const float pv = __half2float(__ushort_as_half(rs[r]));
+            a0 = fmaf(pv, f.x, a0);
+            a1 = fmaf(pv, f.y, a1);
+        }
+        part[g][2 * c] = a0;
+        part[g][2 * c + 1] = a1;
+    }
+    __syncthreads();
+    for (int d = tid; d < D; d += NT) {
+        float v = part[0][d];
+        for (int g = 1; g < parts; ++g) v += part[g][d];
+        res[(size_t)bhq * D + d] = __half_as_ushort(__float2half_rn(v));
     }
 }
 
-// NT threads per CTA (256, or 512 for rows of up to 512*SM_REGS scores that one CTA keeps in registers).
-// RG: scores a thread keeps in registers (CACHED): SM_REGS, or fewer for short rows - with 17 (rows of up to 4352
-// scores) two CTAs of 256 threads fit an SM instead of one, and 256 rows run as one wave.
-template <bool CACHED, bool PROBE, int NT, int RG = (NT == 512 ? SM_REGS_512 : SM_REGS)>
-__global__ void __launch_bounds__(NT, (RG <= 17 && NT == 256) ? 2 : 0)
+// Rows too long for one CTA's registers, and many of them: three passes over the row, the probe in a launch of its own.
+__global__ void __launch_bounds__(256)
 softmax_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __half* __restrict__ restk,
-               uint16_t* __restrict__ pval, int32_t* __restrict__ pidx, float* __restrict__ stats,
-               const uint8_t* __restrict__ first8, uint16_t* __restrict__ test_o, int max_seq_len, int H, int G, int D,
-               int R, int qn, int rest, float sqrt_d, const __half* __restrict__ mask, long long mask_stride,
-               const __half* __restrict__ restv, uint16_t* __restrict__ res) {
-    constexpr int NW = NT / 32;
-    constexpr int REGS = RG;                                     // scores a thread keeps (CACHED)
+               uint16_t* __restrict__ pval, int32_t* __restrict__ pidx, float* __restrict__ stats, int H, int G, int D, int R,
+               int qn, int rest, float sqrt_d, const __half* __restrict__ mask, long long mask_stride) {
+    constexpr int NT = 256, NW = NT / 32;
     __shared__ float redf[NW];
     __shared__ uint32_t cand_v[NT];
     __shared__ int32_t cand_i[NT];
@@ -250,19 +487,9 @@ softmax_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __h
     const int len = qn + rest;
     residual_scores(row, q + (size_t)bhq * D, restk, b, h, H, D, qn, rest, sqrt_d, 0, len);
     __syncthreads();
-    float x[CACHED ? REGS : 1];
     // pass 1: maximum
     float m = -INFINITY;
-    if (CACHED) {
-#pragma unroll
-        for (int i = 0; i < REGS; ++i) {
-            const int t = tid + NT * i;
-            x[i] = t < len ? masked_score(row, mrow, t) : -INFINITY;
-            m = fmaxf(m, x[i]);
-        }
-    } else {
-        for (int t = tid; t < len; t += NT) m = fmaxf(m, masked_score(row, mrow, t));
-    }
+    for (int t = tid; t < len; t += NT) m = fmaxf(m, masked_score(row, mrow, t));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
     if (lane == 0) redf[warp] = m;
@@ -271,19 +498,9 @@ softmax_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __h
 #pragma unroll
     for (int w = 1; w < NW; ++w) m = fmaxf(m, redf[w]);
     __syncthreads();
-    // pass 2: sum of exponentials (fp32, as F.softmax(scores.float()) does; model/KVCache_AlignedKV.py:121)
+    // pass 2: sum of exponentials
     float sum = 0.f;
-    if (CACHED) {
-#pragma unroll
-        for (int i = 0; i < REGS; ++i) {
-            if (tid + NT * i < len) {
-                x[i] = expf(x[i] - m);
-                sum += x[i];
-            }
-        }
-    } else {
-        for (int t = tid; t < len; t += NT) sum += expf(masked_score(row, mrow, t) - m);
-    }
+    for (int t = tid; t < len; t += NT) sum += expf(masked_score(row, mrow, t) - m);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     if (lane == 0) redf[warp] = sum;
@@ -296,32 +513,16 @@ softmax_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __h
         stats[(size_t)bhq * 2 + 1] = sum;
     }
     // pass 3: probabilities, and this thread's residue class (tid % 32): largest probability over the quantized
-    // tokens with its first position (torch.max over the group axis keeps the first maximum; v_cache_file.py:128-130)
+    // tokens with its first position
     uint32_t best = 0;
     int32_t best_g = 0;
-    if (CACHED) {
-#pragma unroll
-        for (int i = 0; i < REGS; ++i) {
-            const int t = tid + NT * i;
-            if (t < R) {
-                uint16_t pb = 0;   // exp(-inf - m) = 0
-                if (t < len) pb = __half_as_ushort(__float2half_rn(x[i] / sum));
-                row[t] = pb;
-                if (t < qn && pb > best) {   // probabilities are non-negative: bit patterns order like values
-                    best = pb;
-                    best_g = t >> 5;
-                }
-            }
-        }
-    } else {
-        for (int t = tid; t < R; t += NT) {
-            uint16_t pb = 0;
-            if (t < len) pb = __half_as_ushort(__float2half_rn(expf(masked_score(row, mrow, t) - m) / sum));
-            row[t] = pb;
-            if (t < qn && pb > best) {
-                best = pb;
-                best_g = t >> 5;
-            }
+    for (int t = tid; t < R; t += NT) {
+        uint16_t pb = 0;
+        if (t < len) pb = __half_as_ushort(__float2half_rn(expf(masked_score(row, mrow, t) - m) / sum));
+        row[t] = pb;
+        if (t < qn && pb > best) {
+            best = pb;
+            best_g = t >> 5;
         }
     }
     cand_v[tid] = best;
@@ -337,68 +538,7 @@ softmax_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __h
         }
         pval[(size_t)bhq * TOPK + tid] = (uint16_t)bv;
         pidx[(size_t)bhq * TOPK + tid] = bi;
-        if (PROBE) {
-            cand_v[tid] = bv;
-            cand_i[tid] = bi;
-        }
     }
-    if (!PROBE || first8 == nullptr || qn == 0) return;   // (uniform)
-    __syncthreads();
-    // probe: o_test[d] = sum_j |half((first_8[row_j][d] << 8) + 0x80)| * p_j over the class maxima, rows
-    // row_j = class position * 32 + j, accumulated in fp16 in j order; all row gathers go out before the chain starts
-    const uint8_t* F = first8 + (size_t)(bhq / G) * max_seq_len * D;
-    for (int c = tid; c < (D >> 1); c += NT) {
-        uint32_t f[TOPK];
-#pragma unroll
-        for (int j = 0; j < TOPK; ++j) {
-            long long r = (long long)cand_i[j] * TOPK + j;
-            r = r >= max_seq_len ? max_seq_len - 1 : r;
-            f[j] = __ldg(reinterpret_cast<const uint16_t*>(F + (size_t)r * D + 2 * c));
-        }
-        uint32_t acc = 0;
-#pragma unroll
-        for (int j = 0; j < TOPK; ++j) {
-            const uint32_t v = __byte_perm(f[j], 0x80u, 0x1404) & 0x7FFF7FFFu;
-            acc = hfma2_bits(v, cand_v[j] | (cand_v[j] << 16), acc);
-        }
-        reinterpret_cast<uint32_t*>(test_o)[(size_t)bhq * (D >> 1) + c] = acc;
-    }
-    if (res == nullptr || rest <= 0) return;              // (uniform)
-    // The residual tokens' part of the output, half(sum_r p[qn + r] * restv[r]) (extension/v_cache_file.py:189), for the
-    // P.V kernel to add in its epilogue - computed here by the threads the probe leaves idle (it occupies D/2 of them),
-    // so that no tail launch is needed.  Item = (channel pair, third of the tokens); fp32 sums, added in a fixed order.
-    __shared__ float part[3][256];
-    {
-        const int hd = D >> 1, idle0 = hd < NT ? hd : 0, nidle = NT - idle0;
-        if (tid >= idle0) {
-            for (int i = tid - idle0; i < 3 * hd; i += nidle) {
-                const int g = i / hd, c = i - g * hd;
-                const __half* vr = restv + ((size_t)b * BLK * H + h) * D + 2 * c;
-                const size_t vs = (size_t)H * D;
-                float pv[22];
-                __half2 vv[22];
-#pragma unroll
-                for (int j = 0; j < 22; ++j) {
-                    const int r = g + 3 * j;
-                    const bool on = r < rest;
-                    pv[j] = on ? __half2float(__ushort_as_half(row[qn + r])) : 0.f;
-                    vv[j] = on ? *reinterpret_cast<const __half2*>(vr + (size_t)r * vs) : __half2(__half(0.f), __half(0.f));
-                }
-                float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-                for (int j = 0; j < 22; ++j) {
-                    const float2 f = __half22float2(vv[j]);
-                    a0 = fmaf(pv[j], f.x, a0);
-                    a1 = fmaf(pv[j], f.y, a1);
-                }
-                part[g][2 * c] = a0;
-                part[g][2 * c + 1] = a1;
-            }
-        }
-    }
-    __syncthreads();
-    for (int d = tid; d < D; d += NT)
-        res[(size_t)bhq * D + d] = __half_as_ushort(__float2half_rn((part[0][d] + part[1][d]) + part[2][d]));
 }
 
 // ------------------------------------------------------------------ softmax over long rows, split across CTAs
@@ -924,31 +1064,45 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
         if (ev) cudaEventRecord(ev[1], st);
         if (rc != AKV_OK) return rc;
     }
-    // one CTA per row while there are enough rows to fill the GPU or the rows are short (three launches cost more
-    // than they save below ~16k scores); else the split form
+    // Rows split across CTAs when they are few and long (softmax_chunk_*); one CTA per row, held in registers, when it has at
+    // most 24576 scores; else one CTA in three passes.  (The split form's chunk grid is part of the sequence-sharded
+    // protocol: the line between it and the others stays where it is.)
     const int sm_chunks = (R + SM_CHUNK - 1) / SM_CHUNK;
-    bool probed = false;
     const int rows = B * H * G;
-    const bool one_cta_512 = R > 256 * SM_REGS && R <= 512 * SM_REGS_512 && rows <= 2 * sm_count();
-    const bool one_cta_256 = !one_cta_512 && !(sm_chunks >= 4 && rows < 2 * sm_count()) && R <= 256 * SM_REGS &&
-                             rows <= 4 * sm_count();
+    const bool split = R > 17408 && rows < 2 * sm_count();
+    const bool probed = !split && R <= 1024 * 24;
     // The residual tokens' part of the output without a launch of its own: the softmax CTA of a row computes it beside
     // its probe (into o_main, as fp16), and the exact-order chain kernel adds it in its epilogue.
-    const bool fuse_tail = !order_free && !packed_out && qn > 0 && rest > 0 && D <= 256 && (one_cta_512 || one_cta_256) &&
+    const bool fuse_tail = !order_free && !packed_out && qn > 0 && rest > 0 && D <= 256 && probed &&
         v_compute_adds_residual(static_cast<const uint8_t*>(v_first_8), static_cast<const uint8_t*>(v_mid_4),
                                 static_cast<const uint8_t*>(v_last_4), reinterpret_cast<const uint8_t*>(sc.s),
                                 static_cast<const uint8_t*>(out), B, H, G, D, R, qn, reference);
     const __half* res_v = fuse_tail ? static_cast<const __half*>(restv) : nullptr;
     uint16_t* res_o = fuse_tail ? sc.o_main : nullptr;
-    if (one_cta_512) {
-        // few rows of up to 17408 scores: one CTA of 512 threads keeps the row in registers - one launch instead of the
-        // four of the split form (statistics, probabilities, class reduction, probe)
-        launch_chained(softmax_kernel<true, true, 512>, dim3(rows), dim3(512), 0, st, sc.s,
-                       static_cast<const __half*>(q), static_cast<const __half*>(restk), sc.pval, sc.pidx, sc.stats,
-                       static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn, rest,
-                       sqrtf((float)D), mk, mask_stride, res_v, res_o);
-        probed = true;
-    } else if (sm_chunks >= 4 && B * H * G < 2 * sm_count()) {
+    if (probed) {
+        // Few rows: many threads per row, for its latency.  Many rows: few, for rows in flight.
+        const size_t vals = res_v ? (size_t)rest * D * 2 : 0;
+        auto go = [&](auto kern, int nt, size_t smem) -> int {
+            if (smem > 32 * 1024) {
+                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (e != cudaSuccess) return cuda_status(e, "decode_step softmax smem attribute");
+            }
+            launch_chained(kern, dim3(rows), dim3(nt), smem, st, sc.s, static_cast<const __half*>(q),
+                           static_cast<const __half*>(restk), sc.pval, sc.pidx, sc.stats,
+                           static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn, rest,
+                           sqrtf((float)D), mk, mask_stride, res_v, res_o);
+            return AKV_OK;
+        };
+        const bool many = rows > 2 * sm_count();
+        if (R <= 256 * 8) rc = go(softmax_row_kernel<256, 1, 4>, 256, vals);
+        else if (many && R <= 256 * 16) rc = go(softmax_row_kernel<256, 2, 4>, 256, vals);
+        else if (many && R <= 256 * 40) rc = go(softmax_row_kernel<256, 5, 3>, 256, vals);
+        else if (R <= 512 * 8) rc = go(softmax_row_kernel<512, 1, 2>, 512, vals);
+        else if (R <= 512 * 16) rc = go(softmax_row_kernel<512, 2, 2>, 512, vals);
+        else if (R <= 512 * 24) rc = go(softmax_row_kernel<512, 3, 2>, 512, vals);
+        else rc = go(softmax_row_kernel<1024, 3, 1>, 1024, vals + (size_t)R * sizeof(float));
+        if (rc != AKV_OK) return rc;
+    } else if (split) {
         dim3 grid(sm_chunks, B * H * G);
         count_launch();
         softmax_chunk_stats_kernel<<<grid, 256, 0, st>>>(sc.s, static_cast<const __half*>(q),
@@ -961,25 +1115,9 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
         softmax_class_reduce_kernel<<<B * H * G, 32, 0, st>>>(sc.cstat, sc.cand_val, sc.cand_idx, sc.pval, sc.pidx,
                                                              sc.stats, sm_chunks, 1);
     } else {
-        if (R <= 256 * SM_REGS && B * H * G <= 4 * sm_count()) {
-            // few rows: one pass over the row, and the probe runs inside the softmax CTA of its row
-            if (R <= 256 * 17)
-                launch_chained(softmax_kernel<true, true, 256, 17>, dim3(B * H * G), dim3(256), 0, st, sc.s,
-                               static_cast<const __half*>(q), static_cast<const __half*>(restk), sc.pval, sc.pidx,
-                               sc.stats, static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn,
-                               rest, sqrtf((float)D), mk, mask_stride, res_v, res_o);
-            else
-                launch_chained(softmax_kernel<true, true, 256>, dim3(B * H * G), dim3(256), 0, st, sc.s,
-                               static_cast<const __half*>(q), static_cast<const __half*>(restk), sc.pval, sc.pidx,
-                               sc.stats, static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn,
-                               rest, sqrtf((float)D), mk, mask_stride, res_v, res_o);
-            probed = true;
-        } else {
-            launch_chained(softmax_kernel<false, false, 256>, dim3(B * H * G), dim3(256), 0, st, sc.s,
-                           static_cast<const __half*>(q), static_cast<const __half*>(restk), sc.pval, sc.pidx, sc.stats,
-                           (const uint8_t*)nullptr, (uint16_t*)nullptr, max_seq_len, H, G, D, R, qn, rest,
-                           sqrtf((float)D), mk, mask_stride, (const __half*)nullptr, (uint16_t*)nullptr);
-        }
+        launch_chained(softmax_kernel, dim3(rows), dim3(256), 0, st, sc.s, static_cast<const __half*>(q),
+                       static_cast<const __half*>(restk), sc.pval, sc.pidx, sc.stats, H, G, D, R, qn, rest,
+                       sqrtf((float)D), mk, mask_stride);
     }
     if ((rc = cuda_status(cudaGetLastError(), "decode_step softmax launch")) != AKV_OK) return rc;
     const bool need_tail = (rest > 0 && !fuse_tail) || qn == 0 || packed_out != nullptr || order_free;
