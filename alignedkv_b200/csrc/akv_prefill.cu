@@ -4,11 +4,10 @@
 // extension/csrc/V_cache.cu:17-41), the remaining tokens copied to the fp16 residual buffers - reading every input
 // byte once.  The reference makes three passes per tensor (max reduction, plane writer, tail copy).
 //
-// prefill_kernel: grid (ceil(S/64), H, B), 128 threads.  The CTA stages its 64-token tile of K and of V in shared
-// memory (16-byte loads), emits the K block (thread = channel: gathers 64 tokens, 16-byte plane stores) and the V
-// rows (thread = 32 channels of a token) and records per channel the signed maximum of the tile; a partial last tile
-// goes to the residual buffers instead of the planes.  exp_reduce_kernel then takes the maximum over tiles and stores
-// its exponent field.
+// prefill128_kernel (head_dim 128): grid (ceil(S/64), H, B), 256 threads, one 64-token tile of K and of V per CTA.
+// Every plane piece of a tile - a K block's three planes, 64 V rows' three planes - is contiguous in memory: the results
+// are put together in shared memory, over the input tile, and leave by six bulk stores.  prefill_kernel: any other head
+// size, and the same partial maxima.  exp_reduce_kernel takes the maximum over tiles and stores its exponent field.
 #include "akv_save.cuh"
 
 namespace akv {
@@ -70,19 +69,201 @@ prefill_kernel(uint8_t* __restrict__ k_first_8, uint8_t* __restrict__ k_mid_4, u
     }
 }
 
-// exponent field of the signed maximum over the tiles -> [B,1,H,D] bytes
-__global__ void __launch_bounds__(128)
-exp_reduce_kernel(const uint16_t* __restrict__ kmax_part, const uint16_t* __restrict__ vmax_part,
-                  uint8_t* __restrict__ k_exp, uint8_t* __restrict__ v_exp, int D, int tiles) {
-    const long long bh = blockIdx.x;
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        float km = -INFINITY, vm = -INFINITY;
-        for (int z = 0; z < tiles; ++z) {
-            km = fmaxf(km, __half2float(__ushort_as_half(kmax_part[(bh * tiles + z) * D + d])));
-            vm = fmaxf(vm, __half2float(__ushort_as_half(vmax_part[(bh * tiles + z) * D + d])));
+// ---- head_dim 128
+namespace pf {
+constexpr int D = 128, NT = 256, IN_BYTES = PF_BLK * 2 * D;          // one tile as it arrives
+// Row t of a staged tile: 256 bytes, 32 bytes further after every 16 tokens - four threads that read the same channels of
+// tokens 16 apart then hit different banks.
+constexpr int BUF_BYTES = IN_BYTES + 128;
+__device__ __forceinline__ int row_at(int t) { return t * 2 * D + (t >> 4) * 32; }
+}  // namespace pf
+
+__device__ __forceinline__ uint32_t hmax2_bits(uint32_t a, uint32_t b) {
+    const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+// Four tokens' low bytes of a channel [t0, t1, t2, t3] -> two bytes of a nibble plane (in bytes 0 and 2), the even token's
+// nibble above the odd one's (extension/csrc/K_cache.cu:49-56)
+__device__ __forceinline__ uint32_t mid_nibbles(uint32_t x) { return (x & 0x00F000F0u) | ((x >> 12) & 0x000F000Fu); }
+__device__ __forceinline__ uint32_t low_nibbles(uint32_t x) { return ((x << 4) & 0x00F000F0u) | ((x >> 8) & 0x000F000Fu); }
+
+// Bound by HBM: 32 KB in, 32 KB out and 8 KB of nibble planes read per tile (the K nibbles are added onto what the planes
+// hold).  Thread = (channel pair c = tid / 4, 16 tokens q = tid % 4): 16 four-byte shared loads of a tile give 2 x (16 high
+// bytes, 8 mid, 8 low bytes) of the K planes, all transposition by byte permutes; for V = (token, 32 channels).  About 4
+// integer instructions per value where the form before it (thread = channel, one 2-byte load per value, results stored 16
+// bytes at a time straight to the planes) took 10 and half-filled every sector it wrote: batch 8 x 32 heads x
+// 4096 tokens 182.5 us (1.21 GB: 6.6 TB/s) against 356.4.
+__global__ void __launch_bounds__(pf::NT, 4)
+prefill128_kernel(uint8_t* __restrict__ k_first_8, uint8_t* __restrict__ k_mid_4, uint8_t* __restrict__ k_last_4,
+                  uint8_t* __restrict__ v_first_8, uint8_t* __restrict__ v_mid_4, uint8_t* __restrict__ v_last_4,
+                  uint8_t* __restrict__ restk, uint8_t* __restrict__ restv, const uint8_t* __restrict__ k,
+                  const uint8_t* __restrict__ v, uint32_t* __restrict__ kmax_part, uint32_t* __restrict__ vmax_part, int H,
+                  int S, int nmb, int max_seq_len, int tiles) {
+    using namespace pf;
+    __shared__ __align__(128) uint8_t ks[BUF_BYTES], vs[BUF_BYTES];
+    const int tid = threadIdx.x, z = blockIdx.x, h = blockIdx.y;
+    const long long b = blockIdx.z, bh = b * H + h;
+    const int t0 = z * PF_BLK, cnt = min(PF_BLK, S - t0);
+    const size_t in0 = ((size_t)(b * S + t0) * H + h) * (2 * D), in_step = (size_t)H * 2 * D;
+    const uint32_t ka = smem_u32(ks), va = smem_u32(vs);
+#pragma unroll
+    for (int j = 0; j < IN_BYTES / 16 / NT; ++j) {
+        const int i = tid + j * NT, t = i >> 4, o = (i & 15) * 16;
+        if (t < cnt) {
+            cp_async16(ka + row_at(t) + o, k + in0 + t * in_step + o);
+            cp_async16(va + row_at(t) + o, v + in0 + t * in_step + o);
         }
-        k_exp[bh * D + d] = (uint8_t)((__half_as_ushort(__float2half_rn(km)) >> 10) & 0x1Fu);
-        v_exp[bh * D + d] = (uint8_t)((__half_as_ushort(__float2half_rn(vm)) >> 10) & 0x1Fu);
+    }
+    cp_async_commit();
+    const int c = tid >> 2, q = tid & 3;                             // channel pair, tokens 16 q .. 16 q + 15
+    const size_t tile = (size_t)(bh * nmb + z) * D;                  // plane row of channel 0
+    uint8_t* mid = k_mid_4 + (tile + 2 * c) * 32 + q * 8;
+    uint8_t* low = k_last_4 + (tile + 2 * c) * 32 + q * 8;
+    uint2 om[2], ol[2];                                              // the nibble bytes this thread adds onto
+    if (cnt == PF_BLK) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            om[e] = *reinterpret_cast<const uint2*>(mid + e * 32);
+            ol[e] = *reinterpret_cast<const uint2*>(low + e * 32);
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // signed maxima of this thread's channel pair over its tokens (extension/k_cache_file.py:77-78), as fp16x2
+    uint32_t km = 0xFC00FC00u, vm = 0xFC00FC00u;
+    uint32_t kw[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        const int a = row_at(16 * q + t) + 4 * c;
+        kw[t] = *reinterpret_cast<const uint32_t*>(ks + a);
+        const uint32_t vw = *reinterpret_cast<const uint32_t*>(vs + a);
+        if (16 * q + t < cnt) {
+            km = hmax2_bits(km, kw[t]);
+            vm = hmax2_bits(vm, vw);
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        km = hmax2_bits(km, __shfl_xor_sync(0xFFFFFFFFu, km, o));
+        vm = hmax2_bits(vm, __shfl_xor_sync(0xFFFFFFFFu, vm, o));
+    }
+    if (q == 0) {
+        const size_t at = (size_t)(bh * tiles + z) * (D / 2) + c;
+        kmax_part[at] = km;
+        vmax_part[at] = vm;
+    }
+    if (cnt < PF_BLK) {
+        // the prompt's last, partial tile stays in fp16 (residual buffers [B,64,H,D], rows 0..cnt-1)
+        for (int i = tid; i < cnt * 16; i += NT) {
+            const int t = i >> 4, o = (i & 15) * 16;
+            const size_t dst = ((size_t)(b * PF_BLK + t) * H + h) * (2 * D) + o;
+            *reinterpret_cast<uint4*>(restk + dst) = *reinterpret_cast<const uint4*>(ks + row_at(t) + o);
+            *reinterpret_cast<uint4*>(restv + dst) = *reinterpret_cast<const uint4*>(vs + row_at(t) + o);
+        }
+        return;
+    }
+    // K: per 4 tokens, words [lo a, hi a, lo b, hi b] of channels a, b -> high bytes and low bytes of each channel
+    uint32_t f[2][4], m[2][2], l[2][2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {                                    // 8 tokens
+        uint32_t lo[2][2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {                                // 4 tokens
+            const uint32_t* w = kw + 8 * g + 4 * p;
+            const uint32_t h01 = __byte_perm(w[0], w[1], 0x7531), h23 = __byte_perm(w[2], w[3], 0x7531);
+            const uint32_t l01 = __byte_perm(w[0], w[1], 0x6420), l23 = __byte_perm(w[2], w[3], 0x6420);
+            f[0][2 * g + p] = __byte_perm(h01, h23, 0x6420);
+            f[1][2 * g + p] = __byte_perm(h01, h23, 0x7531);
+            lo[0][p] = __byte_perm(l01, l23, 0x6420);
+            lo[1][p] = __byte_perm(l01, l23, 0x7531);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            m[e][g] = __byte_perm(mid_nibbles(lo[e][0]), mid_nibbles(lo[e][1]), 0x6420);
+            l[e][g] = __byte_perm(low_nibbles(lo[e][0]), low_nibbles(lo[e][1]), 0x6420);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {                                    // bytewise, modulo 256
+        m[e][0] = __vadd4(m[e][0], om[e].x);
+        m[e][1] = __vadd4(m[e][1], om[e].y);
+        l[e][0] = __vadd4(l[e][0], ol[e].x);
+        l[e][1] = __vadd4(l[e][1], ol[e].y);
+    }
+    // V: token t, 32 channels
+    const int t = tid >> 2;
+    uint4 vf0, vf1, vmid, vlow;
+    {
+        const uint4* src = reinterpret_cast<const uint4*>(vs + row_at(t) + q * 64);
+        const uint4 a0 = src[0], a1 = src[1], a2 = src[2], a3 = src[3];
+        v_split4(a0.x, a0.y, a0.z, a0.w, vf0.x, vf0.y, vmid.x, vlow.x);
+        v_split4(a1.x, a1.y, a1.z, a1.w, vf0.z, vf0.w, vmid.y, vlow.y);
+        v_split4(a2.x, a2.y, a2.z, a2.w, vf1.x, vf1.y, vmid.z, vlow.z);
+        v_split4(a3.x, a3.y, a3.z, a3.w, vf1.z, vf1.w, vmid.w, vlow.w);
+    }
+    __syncthreads();                                                 // (the tiles have been read)
+    // planes in the order of memory: high [0, 8 KB), mid, low (4 KB each).  Threads next to each other write different
+    // halves of a row first, so that a warp's stores spread over the banks.
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int e = s ^ (c & 1), n = s ^ ((c >> 1) & 1);
+        const uint32_t x = e ? f[1][0] : f[0][0], y = e ? f[1][1] : f[0][1], zz = e ? f[1][2] : f[0][2], w = e ? f[1][3] : f[0][3];
+        *reinterpret_cast<uint4*>(ks + (2 * c + e) * 64 + q * 16) = make_uint4(x, y, zz, w);
+        *reinterpret_cast<uint2*>(ks + 8192 + (2 * c + n) * 32 + q * 8) = n ? make_uint2(m[1][0], m[1][1]) : make_uint2(m[0][0], m[0][1]);
+        *reinterpret_cast<uint2*>(ks + 12288 + (2 * c + n) * 32 + q * 8) = n ? make_uint2(l[1][0], l[1][1]) : make_uint2(l[0][0], l[0][1]);
+    }
+    *reinterpret_cast<uint4*>(vs + t * 128 + q * 32) = vf0;
+    *reinterpret_cast<uint4*>(vs + t * 128 + q * 32 + 16) = vf1;
+    *reinterpret_cast<uint4*>(vs + 8192 + t * 64 + q * 16) = vmid;
+    *reinterpret_cast<uint4*>(vs + 12288 + t * 64 + q * 16) = vlow;
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+        const size_t vrow = (size_t)bh * max_seq_len + t0;
+        bulk_store(k_first_8 + tile * 64, ka, 8192);
+        bulk_store(k_mid_4 + tile * 32, ka + 8192, 4096);
+        bulk_store(k_last_4 + tile * 32, ka + 12288, 4096);
+        bulk_store(v_first_8 + vrow * D, va, 8192);
+        bulk_store(v_mid_4 + vrow * (D / 2), va + 8192, 4096);
+        bulk_store(v_last_4 + vrow * (D / 2), va + 12288, 4096);
+        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // (shared memory is read, and the planes are written)
+    }
+}
+
+// exponent field of the signed maximum over the tiles -> [B,1,H,D] bytes.  Thread = (channel pair, share of the tiles).
+__global__ void __launch_bounds__(256)
+exp_reduce_kernel(const uint32_t* __restrict__ kmax_part, const uint32_t* __restrict__ vmax_part,
+                  uint8_t* __restrict__ k_exp, uint8_t* __restrict__ v_exp, int hd, int tiles) {
+    __shared__ uint32_t red[2][256];
+    const long long bh = blockIdx.x;
+    const int shares = hd <= 128 ? 256 / hd : 1;                     // (hd <= 128: head_dim is at most 256)
+    const int c = threadIdx.x % hd, g = threadIdx.x / hd;
+    uint32_t km = 0xFC00FC00u, vm = 0xFC00FC00u;
+    if (g < shares) {
+        const size_t at = (size_t)bh * tiles * hd + c;
+#pragma unroll 8
+        for (int z = g; z < tiles; z += shares) {
+            km = hmax2_bits(km, kmax_part[at + (size_t)z * hd]);
+            vm = hmax2_bits(vm, vmax_part[at + (size_t)z * hd]);
+        }
+    }
+    red[0][threadIdx.x] = km;
+    red[1][threadIdx.x] = vm;
+    __syncthreads();
+    if (g == 0) {
+        for (int s = 1; s < shares; ++s) {
+            km = hmax2_bits(km, red[0][c + s * hd]);
+            vm = hmax2_bits(vm, red[1][c + s * hd]);
+        }
+        const size_t at = 2 * ((size_t)bh * hd + c);                 // (the exponent tensors may lie at any address)
+        k_exp[at] = (uint8_t)((km >> 10) & 0x1Fu);
+        k_exp[at + 1] = (uint8_t)((km >> 26) & 0x1Fu);
+        v_exp[at] = (uint8_t)((vm >> 10) & 0x1Fu);
+        v_exp[at + 1] = (uint8_t)((vm >> 26) & 0x1Fu);
     }
 }
 
@@ -119,22 +300,31 @@ int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8,
     const int nmb = (max_seq_len + PF_BLK - 1) / PF_BLK;
     uint16_t* kmax_part = static_cast<uint16_t*>(scratch);
     uint16_t* vmax_part = kmax_part + (size_t)B * H * tiles * D;
-    const size_t smem = (size_t)2 * PF_BLK * 2 * D;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return cuda_status(e, "prefill smem attribute");
-    }
     dim3 grid(tiles, H, B);
     count_launch(2);
-    prefill_kernel<<<grid, 128, smem, st>>>(
-        static_cast<uint8_t*>(k_first_8), static_cast<uint8_t*>(k_mid_4), static_cast<uint8_t*>(k_last_4),
-        static_cast<uint8_t*>(v_first_8), static_cast<uint8_t*>(v_mid_4), static_cast<uint8_t*>(v_last_4),
-        static_cast<uint8_t*>(restk), static_cast<uint8_t*>(restv), static_cast<const uint8_t*>(k),
-        static_cast<const uint8_t*>(v), kmax_part, vmax_part, H, D, S, nmb, max_seq_len, tiles);
+    if (D == pf::D) {
+        prefill128_kernel<<<grid, pf::NT, 0, st>>>(
+            static_cast<uint8_t*>(k_first_8), static_cast<uint8_t*>(k_mid_4), static_cast<uint8_t*>(k_last_4),
+            static_cast<uint8_t*>(v_first_8), static_cast<uint8_t*>(v_mid_4), static_cast<uint8_t*>(v_last_4),
+            static_cast<uint8_t*>(restk), static_cast<uint8_t*>(restv), static_cast<const uint8_t*>(k),
+            static_cast<const uint8_t*>(v), reinterpret_cast<uint32_t*>(kmax_part), reinterpret_cast<uint32_t*>(vmax_part), H,
+            S, nmb, max_seq_len, tiles);
+    } else {
+        const size_t smem = (size_t)2 * PF_BLK * 2 * D;
+        if (smem > 48 * 1024) {
+            cudaError_t e = cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return cuda_status(e, "prefill smem attribute");
+        }
+        prefill_kernel<<<grid, 128, smem, st>>>(
+            static_cast<uint8_t*>(k_first_8), static_cast<uint8_t*>(k_mid_4), static_cast<uint8_t*>(k_last_4),
+            static_cast<uint8_t*>(v_first_8), static_cast<uint8_t*>(v_mid_4), static_cast<uint8_t*>(v_last_4),
+            static_cast<uint8_t*>(restk), static_cast<uint8_t*>(restv), static_cast<const uint8_t*>(k),
+            static_cast<const uint8_t*>(v), kmax_part, vmax_part, H, D, S, nmb, max_seq_len, tiles);
+    }
     int rc = cuda_status(cudaGetLastError(), "prefill launch");
     if (rc != AKV_OK) return rc;
-    exp_reduce_kernel<<<B * H, 128, 0, st>>>(kmax_part, vmax_part, static_cast<uint8_t*>(k_exp_max),
-                                            static_cast<uint8_t*>(v_exp_max), D, tiles);
+    exp_reduce_kernel<<<B * H, 256, 0, st>>>(reinterpret_cast<const uint32_t*>(kmax_part), reinterpret_cast<const uint32_t*>(vmax_part),
+                                            static_cast<uint8_t*>(k_exp_max), static_cast<uint8_t*>(v_exp_max), D / 2, tiles);
     return cuda_status(cudaGetLastError(), "prefill reduce launch");
 }
 
