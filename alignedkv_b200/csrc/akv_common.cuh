@@ -22,7 +22,6 @@ struct Tuning {
     int timing = 0;     // 1: akv_decode_step records CUDA events around its two streaming kernels
     int k_wpc = 0;      // cap on warps per CTA of the q.K^T kernel (0 = as many as shared memory allows)
     int pdl = 1;        // 1: the kernels of a decode step are chained with programmatic dependent launch
-    int k_gqa_kch = 8;  // channels per stage of the q.K^T kernel when query heads share KV heads (8 or 16)
     int v_impl = 0;     // exact P.V, aligned mode, groups of 1, 2, 4: 0 = chain form, 1 = producer-transposed form
     int v_nf = 0;       // exact P.V (form 0): cap on the ring depth in stages (0 = from the shared-memory budget)
     int v_gqa_form = 0;   // exact P.V, grouped queries (form 0): 0 = by size, 1 = one ring per query head, 2 = the group's heads share a ring

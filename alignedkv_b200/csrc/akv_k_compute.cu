@@ -16,15 +16,16 @@
 // Grouped-query attention (G query heads per KV head): a row is fetched when ANY head of the group needs it, every
 // staged row is read from shared memory once and applied to the G heads in turn, each head substituting the
 // reference's constants where its own code skips the plane - so plane bytes cross HBM once per group and the
-// results equal G independent multi-head passes.  The byte shuffles that assemble a token's low byte from the
-// nibble planes run on the half-rate integer pipe, and with them done per head the kernel was bound by that pipe
-// (2.1 TB/s at G = 4).  So per row each lane assembles the low bytes once per alignment code (mid only / both planes;
-// "neither" is a constant) and parks them in a private 8-byte slot per code of a small per-warp scratch; a head then
-// fetches the pair of its own code with one 8-byte load whose offset (code x 256) was tabulated per (head, channel)
-// when the (batch, KV head) started: one add and one load per head and row instead of selects and shuffles.  The
-// rows are software-pipelined by one (two scratch buffers), so the store -> load round trip of a row overlaps the
-// arithmetic of the previous one.  With G == 1 the producer writes the constants into the skipped rows' slots
-// instead, and the consumer has neither selects nor scratch.
+// results equal G independent multi-head passes.  A row's four fp16x2 words are assembled once, with all planes; a head's
+// words are (word & mask) | constant, mask and constant by the head's code on the channel: ONE logic operation per FMA (whatever
+// lies in a plane's slot that the union did not fetch is masked away).  Mask, constant and query of a (head, channel) are
+// tabulated when the (batch, KV head) starts.  Per row of four 64-token tiles that is 24 operations on the half-rate
+// integer pipe and 16 FMAs for four heads; parking the low bytes of each code in shared memory and fetching them back per
+// head, which this replaces, took 80 instructions: groups of eight 253 against
+// 177 us at batch 64 x 4 KV heads x 8192 tokens, of two 56 against 46 at batch 16 x 16 x 4096, of four 41.5 against 35.5 at
+// batch 8 x 8 x 8192 but 228 against 223 at batch 64, where the copies are what is left (a stage's issue stalls for 450 to
+// 770 cycles on the load unit; neither bulk copies nor TMA boxes, built and bit-exact, moved these pieces faster).
+// With G == 1 the producer writes the constants into the skipped rows' slots instead.
 #include "akv_common.cuh"
 
 namespace akv {
@@ -32,23 +33,25 @@ namespace akv {
 namespace kc {
 constexpr int TILES = 4;                         // 64-token blocks per warp unit
 constexpr int MAX_D = 256;
-// Metadata slots per warp: the producer runs at most STAGES - 1 stages ahead of the consumer, which is less than one
-// unit's stages, so it is at most one (batch, KV head) ahead: two slots.  (A third is kept for multi-head attention,
-// whose slots are small and whose 16-channel stages make a unit only D/16 stages long.)
-__host__ __device__ constexpr int nmeta(int G) { return G > 1 ? 2 : 3; }
 __host__ __device__ constexpr int f_tile(int kch) { return kch * 64 + 64; }   // +64: tiles land on distinct banks
 __host__ __device__ constexpr int n_tile(int kch) { return kch * 32 + 32; }
 __host__ __device__ constexpr int stage_bytes(int kch) { return TILES * f_tile(kch) + 2 * TILES * n_tile(kch); }
 }  // namespace kc
 
 namespace kc {
-// per (batch, KV head) metadata slot: union masks (16 words), then per query head D offset words (code x 256: which
-// scratch slot holds the low bytes of the head's alignment code on that channel; used when G > 1) + D q words
-__host__ __device__ constexpr int head_meta(int D) { return 8 * D; }
-__host__ __device__ constexpr int meta_bytes(int D, int G) { return 64 + G * head_meta(D); }
-// per-warp scratch of the grouped-query consumer: 2 row buffers x 3 codes x 32 lanes x 8 bytes
-constexpr int SCR_CODE = 256, SCR_ROW = 3 * SCR_CODE, SCR_BYTES = 2 * SCR_ROW;
-__host__ __device__ constexpr int scratch_bytes(int G) { return G > 1 ? SCR_BYTES : 0; }
+// Per warp: two sets of union masks (16 words) - the producer is at most STAGES - 1 stages ahead of the consumer, less than a
+// unit's stages, so at most one (batch, KV head) ahead - and the consumer's tables.  G == 1: D words q (both halves equal), two
+// sets that come and go with the masks.  G > 1, one set, loaded when the consumer enters a (batch, KV head): per query head
+// D words mask and D words constant (of the head's alignment code on the channel), D fp16 q.
+constexpr int MASK_BYTES = 64;
+__host__ __device__ constexpr int head_meta(int D, int G) { return G > 1 ? 10 * D : 4 * D; }
+__host__ __device__ constexpr int meta_bytes(int D, int G) { return 2 * MASK_BYTES + (G > 1 ? G : 2) * head_meta(D, G); }
+// Channels per stage and ring depth with grouped queries, warps a CTA is compiled for.  Three stages of 16 channels; groups of
+// eight, whose tables are large, four of 8 (for them 177 us against 226 at batch 64 x 4 KV heads x 8 x 8192 tokens; groups
+// of two 46 against 51 at batch 16 x 16 x 4096, groups of four alike at batch 64 and 35.5 against 38.6 at batch 8).
+__host__ __device__ constexpr int gqa_kch(int G) { return G == 8 ? 8 : 16; }
+__host__ __device__ constexpr int gqa_stages(int G) { return G == 8 ? 4 : 3; }
+__host__ __device__ constexpr int max_warps(int G) { return G == 1 ? 16 : 8; }
 }  // namespace kc
 
 struct KParams {
@@ -69,15 +72,25 @@ __device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t v) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(a), "r"(v) : "memory");
 }
 
+// Both halves of the result = half `hi` of w, and the fp16x2 multiply-add with it (the selection is part of the instruction).
+__device__ __forceinline__ __half2 kc_dup(uint32_t w, int hi) {
+    const __half2 h = *reinterpret_cast<const __half2*>(&w);
+    return hi ? __high2half2(h) : __low2half2(h);
+}
+__device__ __forceinline__ uint32_t kc_fma(uint32_t k, __half2 q, uint32_t acc) {
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&k), q, *reinterpret_cast<const __half2*>(&acc));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
 // Position of a stream of stages (unit, channel chunk) inside one warp's run of units.
 struct KCursor {
     int u, g, bh, c;          // absolute unit, block group inside (batch, KV head), (batch, KV head), channel chunk
-    int slot;                 // metadata slot of the current (batch, KV head)
+    int slot;                 // set of union masks of the current (batch, KV head)
     size_t row;               // plane row index of (tile 0 of the unit, first channel of the chunk)
 };
 
 template <int KCH, int STAGES, int G>
-__global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const KParams p) {
+__global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(const KParams p) {
     using namespace kc;
     constexpr int F_TILE = f_tile(KCH), N_TILE = n_tile(KCH);
     constexpr int F_BYTES = TILES * F_TILE, N_BYTES = TILES * N_TILE, STAGE = F_BYTES + 2 * N_BYTES;
@@ -96,11 +109,11 @@ __global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const K
     const int nch = p.D / KCH;
     const int total = (u_end - u_begin) * nch;
     const size_t tile_f = (size_t)p.D * 64, tile_n = (size_t)p.D * 32;
-    const int META = meta_bytes(p.D, G), HMETA = head_meta(p.D);
+    const int META = meta_bytes(p.D, G), HMETA = head_meta(p.D, G);
 
-    constexpr int NMETA = nmeta(G);
-    uint8_t* ring = smem + (size_t)warp * (STAGES * STAGE + NMETA * META + scratch_bytes(G));
+    uint8_t* ring = smem + (size_t)warp * (STAGES * STAGE + META);
     uint8_t* meta0 = ring + STAGES * STAGE;
+    uint8_t* tables = meta0 + 2 * MASK_BYTES;
     const uint32_t ring_a = smem_u32(ring);
 
     auto cursor_at = [&](int u) {
@@ -124,45 +137,61 @@ __global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const K
         }
         k.g = 0;
         ++k.bh;
-        k.slot = (k.slot + 1 == NMETA) ? 0 : k.slot + 1;
+        k.slot ^= 1;
         k.row = (size_t)k.bh * p.nmb * p.D;
         return true;
     };
-    // Per (batch, KV head): for every query head of the group the plane-read masks (bit d set = row d of that plane
-    // is read: mid iff (u8)(kqmax - kq[d]) < 8, low iff < 4; K_cache.cu:211,249-250) and q as fp16x2 words with
-    // both halves equal; and the union of the masks, which is what the producer fetches.
-    auto load_meta = [&](long long bh, int slot) {
-        uint32_t* um = reinterpret_cast<uint32_t*>(meta0 + (size_t)slot * META);
-        uint32_t u_mm[8], u_lm[8];
+    // Alignment code of channel d for query head bhq: mid plane read iff (u8)(kqmax - kq[d]) < 8, low plane iff < 4
+    // (K_cache.cu:211,249-250)
+    auto diff_of = [&](long long bhq, int d, uint32_t top) {
+        return p.reference ? 0u : (top - (uint32_t)__ldg(p.kq + (size_t)bhq * p.D + d)) & 0xFFu;
+    };
+    // The union of the group's plane-read masks (bit d set = row d of that plane is read), which is what the producer fetches;
+    // with one head its table too
+    auto load_masks = [&](long long bh, int slot) {
+        uint32_t* um = reinterpret_cast<uint32_t*>(meta0 + slot * MASK_BYTES);
+        uint32_t top[G];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) u_mm[r] = u_lm[r] = 0;
+        for (int g = 0; g < G; ++g) top[g] = __ldg(p.kqmax + bh * G + g);
+        uint32_t least[8], qh[8];                 // (all loads before the first vote)
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int d = r * 32 + lane;
+            least[r] = 0xFFu;
+            qh[r] = 0;
+            if (d < p.D) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) least[r] = min(least[r], diff_of(bh * G + g, d, top[g]));
+                if (G == 1) qh[r] = __ldg(reinterpret_cast<const uint16_t*>(p.q) + (size_t)bh * p.D + d);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            if (r * 32 >= p.D) break;
+            const int d = r * 32 + lane;
+            if (G == 1 && d < p.D) reinterpret_cast<uint32_t*>(tables + slot * HMETA)[d] = qh[r] | (qh[r] << 16);
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, least[r] < 8), l = __ballot_sync(0xFFFFFFFFu, least[r] < 4);
+            if (lane == 0) {
+                um[r] = m;
+                um[8 + r] = l;
+            }
+        }
+        __syncwarp();
+    };
+    // The consumer's tables of a group (all its lanes are done with the previous ones)
+    auto load_tables = [&](long long bh) {
+        if (G == 1) return;
+        __syncwarp();
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const long long bhq = bh * G + g;
-            uint32_t* offw = reinterpret_cast<uint32_t*>(meta0 + (size_t)slot * META + 64 + (size_t)g * HMETA);
-            uint32_t* q2 = offw + p.D;
+            uint32_t* hm = reinterpret_cast<uint32_t*>(tables + (size_t)g * HMETA);
             const uint32_t top = __ldg(p.kqmax + bhq);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                if (r * 32 >= p.D) break;
-                const int d = r * 32 + lane;
-                uint32_t diff = 0, qh = 0;
-                if (d < p.D) {
-                    diff = (top - (uint32_t)__ldg(p.kq + (size_t)bhq * p.D + d)) & 0xFFu;
-                    qh = __ldg(reinterpret_cast<const uint16_t*>(p.q) + (size_t)bhq * p.D + d);
-                    q2[d] = qh | (qh << 16);
-                }
-                const bool m = p.reference || diff < 8, l = p.reference || diff < 4;
-                if (G > 1 && d < p.D) offw[d] = (uint32_t)((m ? 1 : 0) + (l ? 1 : 0)) * SCR_CODE;
-                u_mm[r] |= __ballot_sync(0xFFFFFFFFu, m);
-                u_lm[r] |= __ballot_sync(0xFFFFFFFFu, l);
-            }
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                um[r] = u_mm[r];
-                um[8 + r] = u_lm[r];
+            for (int d = lane; d < p.D; d += 32) {
+                const uint32_t diff = diff_of(bhq, d, top);
+                hm[d] = diff < 4 ? 0xFFFFFFFFu : diff < 8 ? 0xFFF0FFF0u : 0xFF00FF00u;
+                hm[p.D + d] = diff < 4 ? 0u : diff < 8 ? 0x00080008u : 0x00800080u;
+                reinterpret_cast<uint16_t*>(hm + 2 * p.D)[d] = __ldg(reinterpret_cast<const uint16_t*>(p.q) + (size_t)bhq * p.D + d);
             }
         }
         __syncwarp();
@@ -174,7 +203,7 @@ __global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const K
     KCursor pk = cursor_at(u_begin);
     int pstage = 0;
     auto issue = [&]() {
-        const uint32_t* masks = reinterpret_cast<const uint32_t*>(meta0 + (size_t)pk.slot * META);   // union masks
+        const uint32_t* masks = reinterpret_cast<const uint32_t*>(meta0 + pk.slot * MASK_BYTES);
         const int sh = ((pk.c * KCH) & 31) + nrow, wi = (pk.c * KCH) >> 5;
         const bool need_m = (masks[wi] >> sh) & 1u;
         const bool need_l = (masks[8 + wi] >> sh) & 1u;
@@ -200,27 +229,22 @@ __global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const K
             }
         }
         pstage = (pstage + 1 == STAGES) ? 0 : pstage + 1;
-        if (advance(pk) && pk.u < u_end) load_meta(pk.bh, pk.slot);
+        if (advance(pk) && pk.u < u_end) load_masks(pk.bh, pk.slot);
     };
 
     // ---- prologue
-    load_meta(pk.bh, 0);
+    load_masks(pk.bh, 0);
     for (int j = 0; j < STAGES - 1; ++j) {
         if (j < total) issue();
         cp_async_commit();
     }
 
     const int tile = lane >> 3, li = lane & 7;
-    // grouped-query scratch: this lane's 8-byte slot of code 0 ("neither plane": low bytes 0x80) never changes
-    const uint32_t scr_a = smem_u32(meta0 + NMETA * META) + lane * 8;
-    if (G > 1) {
-        sts64(scr_a, 0x80808080u, 0x80808080u);
-        sts64(scr_a + SCR_ROW, 0x80808080u, 0x80808080u);
-    }
     uint32_t acc[G][4];
 #pragma unroll
     for (int g = 0; g < G; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0;
     KCursor ck = cursor_at(u_begin);
+    load_tables(ck.bh);
     int cstage = 0;
     for (int i = 0; i < total; ++i) {
         cp_async_wait<STAGES - 2>();
@@ -233,12 +257,12 @@ __global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const K
         const uint2* fp = reinterpret_cast<const uint2*>(stp + tile * F_TILE + li * 8);
         const uint32_t* mp = reinterpret_cast<const uint32_t*>(stp + F_BYTES + tile * N_TILE + li * 4);
         const uint32_t* lp = reinterpret_cast<const uint32_t*>(stp + F_BYTES + N_BYTES + tile * N_TILE + li * 4);
-        const uint8_t* hm0 = meta0 + (size_t)ck.slot * META + 64;
+        const uint8_t* hm0 = tables + (G == 1 ? ck.slot * HMETA : 0);
         const int ch0 = ck.c * KCH;                       // first channel of the stage
         if (G == 1) {
 #pragma unroll
             for (int r4 = 0; r4 < KCH / 4; ++r4) {
-                const uint4 qv = *reinterpret_cast<const uint4*>(hm0 + (size_t)p.D * 4 + (size_t)(ch0 + r4 * 4) * 4);
+                const uint4 qv = *reinterpret_cast<const uint4*>(hm0 + (size_t)(ch0 + r4 * 4) * 4);
 #pragma unroll
                 for (int rr = 0; rr < 4; ++rr) {
                     // the producer has written the substitutes into the rows it did not fetch
@@ -255,60 +279,42 @@ __global__ void __launch_bounds__(G > 1 ? 256 : 512, 1) k_compute_kernel(const K
                 }
             }
         } else {
-            // Row r: (a) this lane's low bytes for the codes "mid only" and "both" go to its slots of scratch buffer
-            // r & 1 (a plane the union did not fetch leaves garbage there that no head's offset points at), and every
-            // head's pair is fetched back through its offset; (b) a row later the pairs are shuffled with the
-            // high bytes into k~ words and multiplied.  Only this lane reads what it wrote, so no warp
-            // synchronisation is involved; the volatile accesses keep their order.
-            const uint32_t hm_a = smem_u32(hm0);
-            uint2 fprev = make_uint2(0u, 0u), lbprev[G];
-            uint4 ofv[G], qv[G], qprev[G];
 #pragma unroll
-            for (int r = 0; r <= KCH; ++r) {
-                uint2 fcur = make_uint2(0u, 0u), lbcur[G];
-#pragma unroll
-                for (int g = 0; g < G; ++g) lbcur[g] = make_uint2(0u, 0u);
-                if (r < KCH) {
-                    if ((r & 3) == 0) {
-#pragma unroll
-                        for (int g = 0; g < G; ++g) {
-                            ofv[g] = lds128(hm_a + g * HMETA + (ch0 + r) * 4);
-                            qv[g] = lds128(hm_a + g * HMETA + p.D * 4 + (ch0 + r) * 4);
-                        }
-                    }
-                    fcur = fp[r * 8];
-                    const uint32_t M = mp[r * 8], L = lp[r * 8];
-                    const uint32_t me = M & 0xF0F0F0F0u, mo = (M << 4) & 0xF0F0F0F0u;
-                    const uint32_t sb = scr_a + (r & 1) * SCR_ROW;
-                    sts64(sb + SCR_CODE, me | 0x08080808u, mo | 0x08080808u);                         // mid only
-                    sts64(sb + 2 * SCR_CODE, me | ((L >> 4) & 0x0F0F0F0Fu), mo | (L & 0x0F0F0F0Fu));   // both planes
-#pragma unroll
-                    for (int g = 0; g < G; ++g) lbcur[g] = lds64(sb + u4w(ofv[g], r & 3));
-                }
-                if (r > 0) {
-                    const int rr = (r - 1) & 3;
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        const uint4& qq = rr == 3 ? qprev[g] : qv[g];   // (row 3 of a quad is consumed after the reload)
-                        const uint32_t q2 = rr == 0 ? qq.x : rr == 1 ? qq.y : rr == 2 ? qq.z : qq.w;
-                        acc[g][0] = hfma2_bits(__byte_perm(lbprev[g].x, fprev.x, 0x6140), q2, acc[g][0]);
-                        acc[g][1] = hfma2_bits(__byte_perm(lbprev[g].y, fprev.x, 0x7150), q2, acc[g][1]);
-                        acc[g][2] = hfma2_bits(__byte_perm(lbprev[g].x, fprev.y, 0x6342), q2, acc[g][2]);
-                        acc[g][3] = hfma2_bits(__byte_perm(lbprev[g].y, fprev.y, 0x7352), q2, acc[g][3]);
-                    }
-                }
-                fprev = fcur;
+            for (int r4 = 0; r4 < KCH / 4; ++r4) {
+                uint4 mk[G], cn[G];
+                uint2 qv[G];
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    lbprev[g] = lbcur[g];
-                    if ((r & 3) == 3) qprev[g] = qv[g];
+                    const uint8_t* hg = hm0 + (size_t)g * HMETA + (size_t)(ch0 + r4 * 4) * 4;
+                    mk[g] = *reinterpret_cast<const uint4*>(hg);
+                    cn[g] = *reinterpret_cast<const uint4*>(hg + (size_t)p.D * 4);
+                    qv[g] = *reinterpret_cast<const uint2*>(hm0 + (size_t)g * HMETA + (size_t)p.D * 8 + (size_t)(ch0 + r4 * 4) * 2);
+                }
+#pragma unroll
+                for (int rr = 0; rr < 4; ++rr) {
+                    const int r = r4 * 4 + rr;
+                    const uint2 f = fp[r * 8];
+                    const uint32_t M = mp[r * 8], L = lp[r * 8];
+                    const uint32_t lbe = (M & 0xF0F0F0F0u) | ((L >> 4) & 0x0F0F0F0Fu);   // low bytes, tokens 0,2,4,6
+                    const uint32_t lbo = ((M << 4) & 0xF0F0F0F0u) | (L & 0x0F0F0F0Fu);   // low bytes, tokens 1,3,5,7
+                    const uint32_t w0 = __byte_perm(lbe, f.x, 0x6140), w1 = __byte_perm(lbo, f.x, 0x7150);
+                    const uint32_t w2 = __byte_perm(lbe, f.y, 0x6342), w3 = __byte_perm(lbo, f.y, 0x7352);
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        const uint32_t m = u4w(mk[g], rr), c = u4w(cn[g], rr), qw = rr < 2 ? qv[g].x : qv[g].y;
+                        const __half2 q2 = kc_dup(qw, rr & 1);
+                        acc[g][0] = kc_fma((w0 & m) | c, q2, acc[g][0]);
+                        acc[g][1] = kc_fma((w1 & m) | c, q2, acc[g][1]);
+                        acc[g][2] = kc_fma((w2 & m) | c, q2, acc[g][2]);
+                        acc[g][3] = kc_fma((w3 & m) | c, q2, acc[g][3]);
+                    }
                 }
             }
         }
         const long long cbh = ck.bh;
         const int cg = ck.g;
         const bool last_chunk = (ck.c == nch - 1);
-        advance(ck);
+        if (advance(ck) && ck.u < u_end) load_tables(ck.bh);
         if (last_chunk) {  // unit finished: scale, reorder to token order, one 16-byte store per lane and head
             const int blk = cg * TILES + tile;
 #pragma unroll
@@ -402,17 +408,19 @@ int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* 
     const int budget = max_dyn_smem();
     // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of
     // its group size, and the shared-memory budget below is computed from what is actually launched
-    // groups: 8-channel stages (smaller rings, more warps per SM: the consumer does G times the arithmetic per byte)
-    const int kch = group > 1 ? (tuning().k_gqa_kch == 16 ? 16 : 8) : tuning().k_kch;
+    // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of its group
+    const int kch = group > 1 ? gqa_kch(group) : tuning().k_kch;
     int stages = tuning().k_stages;
-    if (group > 1) stages = kch == 8 ? 4 : 3;
+    if (group > 1) stages = gqa_stages(group);
     else if (!((kch == 8 && (stages == 3 || stages == 4 || stages == 6)) || (kch == 16 && stages >= 3 && stages <= 5)))
         stages = (kch == 8) ? 4 : 3;
-    const int per_warp = stages * stage_bytes(kch) + nmeta(group) * meta_bytes(D, group) + scratch_bytes(group);
+    const int per_warp = stages * stage_bytes(kch) + meta_bytes(D, group);
     int wmax = budget / per_warp;
-    if (wmax > (group > 1 ? 8 : 16)) wmax = group > 1 ? 8 : 16;   // (the grouped-query kernels are compiled for 256 threads)
+    if (wmax > max_warps(group)) wmax = max_warps(group);
     if (tuning().k_wpc > 0 && tuning().k_wpc < wmax) wmax = tuning().k_wpc;
     AKV_REQUIRE(wmax >= 1, AKV_ERR_CUDA, "k_cache_compute: %d bytes of shared memory are too few", budget);
+    // (fewer units than that: spread over the SMs first, a warp streams the faster the fewer share its SM)
+    if (units < (long long)sms * wmax) wmax = (int)((units + sms - 1) / sms);
     int wpc = wmax;
     double best_eff = -1.0;
     for (int c = wmax; c >= (wmax * 3 + 3) / 4; --c) {
@@ -465,11 +473,11 @@ int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* 
                 return AKV_ERR_SHAPE;
         }
     } else if (group == 2) {
-        rc = (kch == 8) ? go(k_compute_kernel<8, 4, 2>) : go(k_compute_kernel<16, 3, 2>);
+        rc = go(k_compute_kernel<gqa_kch(2), gqa_stages(2), 2>);
     } else if (group == 4) {
-        rc = (kch == 8) ? go(k_compute_kernel<8, 4, 4>) : go(k_compute_kernel<16, 3, 4>);
+        rc = go(k_compute_kernel<gqa_kch(4), gqa_stages(4), 4>);
     } else {
-        rc = (kch == 8) ? go(k_compute_kernel<8, 4, 8>) : go(k_compute_kernel<16, 3, 8>);
+        rc = go(k_compute_kernel<gqa_kch(8), gqa_stages(8), 8>);
     }
     if (rc != AKV_OK) return rc;
     return cuda_status(cudaGetLastError(), "k_cache_compute launch");
