@@ -232,7 +232,12 @@ __device__ __forceinline__ void residual_scores(uint16_t* __restrict__ row, cons
 // see v_probe_kernel), its chain by the first D/2 threads, and, beside it, the residual tokens' part of the output
 // half(sum_r p[qn + r] * restv[r]) (extension/v_cache_file.py:189) by the others, for the P.V kernel to add.
 // The residual values come into shared memory by asynchronous copies started first, so that the sum at the end waits for
-// nothing.  With few rows the chain of loads, three reductions and the probe's gathers counts, with many the instructions
+// nothing.
+// The order of the additions is part of the result - it moves fp16 probabilities by a step, and through the layers of a model
+// its logits - so it depends on a row's length and the number of rows, not on threads and vectors: exponentials in `cols`
+// columns through shared memory, residual tokens in `shares`.  (Adding each thread's own vectors needs no barrier and no
+// shared memory, and moved a decoder's logits by 8e-4.)
+// With few rows the chain of loads, three reductions and the probe's gathers counts, with many the instructions
 // per score: about 14, of which the division takes three - quotient by the reciprocal of the sum, then one residual
 // correction (Markstein 1990: correctly rounded, as the division it replaces).  MINB: CTAs per SM.
 // Measured (cold, one launch): 256 rows of 4160 scores 8.9 us, 512 rows of 1088 with 48 residual tokens 11.0, 32 rows of
@@ -245,14 +250,14 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
                    uint16_t* __restrict__ pval, int32_t* __restrict__ pidx, float* __restrict__ stats,
                    const uint8_t* __restrict__ first8, uint16_t* __restrict__ test_o, int max_seq_len, int H, int G, int D,
                    int R, int qn, int rest, float sqrt_d, const __half* __restrict__ mask, long long mask_stride,
-                   const __half* __restrict__ restv, uint16_t* __restrict__ res) {
-    constexpr int NW = NT / 32, PARTS = 4;
+                   const __half* __restrict__ restv, uint16_t* __restrict__ res, int cols, int shares) {
+    constexpr int NW = NT / 32;
     __shared__ float red[2][NW];
     __shared__ __align__(16) uint32_t key[NW][TOPK];
     __shared__ __align__(16) uint16_t rs[BLK];                   // residual scores, then their probabilities
-    __shared__ float part[PARTS][256];
+    __shared__ float part[4][256];
     __shared__ __align__(16) uint8_t rows[TOPK][256];            // the probe's rows
-    extern __shared__ __align__(16) uint8_t dyn[];               // residual values [rest][D] (res), then exponentials [R] (NT 1024)
+    extern __shared__ __align__(16) uint8_t dyn[];               // residual values [rest][D] (res), then exponentials [R + 16]
     pdl_enter();
     const int bhq = blockIdx.x, Hq = H * G, b = bhq / Hq, h = (bhq - b * Hq) / G;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -310,11 +315,12 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NW; ++k) m = fmaxf(m, red[0][k]);
-    // sum of exponentials (fp32, as F.softmax(scores.float()) does; model/KVCache_AlignedKV.py:121)
+    // sum of exponentials (fp32, as F.softmax(scores.float()) does; model/KVCache_AlignedKV.py:121), added in columns: column
+    // t % cols takes its values in order.  The halves of the vectors lie in two arrays, the second 16 words further modulo the
+    // 32 banks: neither the 16-byte stores nor the columns' loads conflict.
     float sum = 0.f;
-    // Rows beyond 12288 scores also exist as shards of a sequence, whose probabilities agree bit for bit with one device's as
-    // far as the sums do: their order of additions stays that of a 512-thread CTA that owns every 512th score.
     float* ex = reinterpret_cast<float*>(dyn + (with_res ? (size_t)rest * D * 2 : 0));
+    const int second = (R >> 1) + 16;
     float x[VPT][8];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -326,30 +332,25 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
             x[i][2 * j] = in ? expf(f.x - m) : 0.f;
             x[i][2 * j + 1] = in ? expf(f.y - m) : 0.f;
         }
-        if (NT == 1024) {
-            if (in) {
-                reinterpret_cast<float4*>(ex)[2 * v] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
-                reinterpret_cast<float4*>(ex)[2 * v + 1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) sum += x[i][j];
+        if (in) {
+            *reinterpret_cast<float4*>(ex + 4 * v) = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
+            *reinterpret_cast<float4*>(ex + second + 4 * v) = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
         }
     }
-    if (NT == 1024) {
-        __syncthreads();
-        if (tid < 512)
+    __syncthreads();
+    if (tid < cols) {
+        const float* e = ex + ((tid >> 2) & 1) * second + (tid >> 3) * 4 + (tid & 3);
 #pragma unroll 8
-            for (int t = tid; t < len; t += 512) sum += ex[t];
+        for (int t = tid; t < len; t += cols, e += cols >> 1) sum += *e;
     }
-    constexpr int SW = NT == 1024 ? 16 : NW;                     // warps that hold sums
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     if (lane == 0) red[1][warp] = sum;
     __syncthreads();
     sum = 0.f;
 #pragma unroll
-    for (int k = 0; k < SW; ++k) sum += red[1][k];
+    for (int k = 0; k < (NW < 16 ? NW : 16); ++k)
+        if (k < cols >> 5) sum += red[1][k];
     if (tid == 0) {
         stats[(size_t)bhq * 2] = m;
         stats[(size_t)bhq * 2 + 1] = sum;
@@ -447,25 +448,25 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
     if (!with_res) return;                                       // (uniform)
     // residual part (D <= 256): item = (channel pair, share g of the tokens), fp32 sums, the shares added in order
     const int first = NT >= 2 * hd ? hd : 0;                     // (beside the probe's chain where there are threads left)
-    const int parts = min(PARTS, (NT - first) / hd);
-    if (tid >= first && tid < first + parts * hd) {
-        const int i = tid - first, g = i / hd, c = i - g * hd;
-        const __half2* vr = reinterpret_cast<const __half2*>(dyn) + c;
-        float a0 = 0.f, a1 = 0.f;
+    if (tid >= first)
+        for (int i = tid - first; i < shares * hd; i += NT - first) {
+            const int g = i / hd, c = i - g * hd;
+            const __half2* vr = reinterpret_cast<const __half2*>(dyn) + c;
+            float a0 = 0.f, a1 = 0.f;
 #pragma unroll 4
-        for (int r = g; r < rest; r += parts) {
-            const float2 f = __half22float2(vr[r * hd]);
-            const float pv = __half2float(__ushort_as_half(rs[r]));
-            a0 = fmaf(pv, f.x, a0);
-            a1 = fmaf(pv, f.y, a1);
+            for (int r = g; r < rest; r += shares) {
+                const float2 f = __half22float2(vr[r * hd]);
+                const float pv = __half2float(__ushort_as_half(rs[r]));
+                a0 = fmaf(pv, f.x, a0);
+                a1 = fmaf(pv, f.y, a1);
+            }
+            part[g][2 * c] = a0;
+            part[g][2 * c + 1] = a1;
         }
-        part[g][2 * c] = a0;
-        part[g][2 * c + 1] = a1;
-    }
     __syncthreads();
     for (int d = tid; d < D; d += NT) {
         float v = part[0][d];
-        for (int g = 1; g < parts; ++g) v += part[g][d];
+        for (int g = 1; g < shares; ++g) v += part[g][d];
         res[(size_t)bhq * D + d] = __half_as_ushort(__float2half_rn(v));
     }
 }
@@ -1081,26 +1082,31 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
     uint16_t* res_o = fuse_tail ? sc.o_main : nullptr;
     if (probed) {
         // Few rows: many threads per row, for its latency.  Many rows: few, for rows in flight.
-        const size_t vals = res_v ? (size_t)rest * D * 2 : 0;
-        auto go = [&](auto kern, int nt, size_t smem) -> int {
-            if (smem > 32 * 1024) {
-                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const size_t bytes = (res_v ? (size_t)rest * D * 2 : 0) + ((size_t)R + 16) * sizeof(float);
+        // The order of the additions, which is part of the result (softmax_row_kernel): the exponentials in 256 columns, 512
+        // for few rows of 8193 to 17408 scores, the residual tokens in three shares for few rows and groups of up to four, else in
+        // four as tail_kernel does, whatever the threads hold.
+        const bool wide = R > 8192 && R <= 17408 && rows <= 2 * sm_count();
+        const int cols = wide ? 512 : 256, shares = G <= 4 && (wide || (R <= 8192 && rows <= 4 * sm_count())) ? 3 : 4;
+        auto go = [&](auto kern, int nt) -> int {
+            if (bytes > 32 * 1024) {
+                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
                 if (e != cudaSuccess) return cuda_status(e, "decode_step softmax smem attribute");
             }
-            launch_chained(kern, dim3(rows), dim3(nt), smem, st, sc.s, static_cast<const __half*>(q),
+            launch_chained(kern, dim3(rows), dim3(nt), bytes, st, sc.s, static_cast<const __half*>(q),
                            static_cast<const __half*>(restk), sc.pval, sc.pidx, sc.stats,
                            static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn, rest,
-                           sqrtf((float)D), mk, mask_stride, res_v, res_o);
+                           sqrtf((float)D), mk, mask_stride, res_v, res_o, cols, shares);
             return AKV_OK;
         };
         const bool many = rows > 2 * sm_count();
-        if (R <= 256 * 8) rc = go(softmax_row_kernel<256, 1, 4>, 256, vals);
-        else if (many && R <= 256 * 16) rc = go(softmax_row_kernel<256, 2, 4>, 256, vals);
-        else if (many && R <= 256 * 40) rc = go(softmax_row_kernel<256, 5, 3>, 256, vals);
-        else if (R <= 512 * 8) rc = go(softmax_row_kernel<512, 1, 2>, 512, vals);
-        else if (R <= 512 * 16) rc = go(softmax_row_kernel<512, 2, 2>, 512, vals);
-        else if (R <= 512 * 24) rc = go(softmax_row_kernel<512, 3, 2>, 512, vals);
-        else rc = go(softmax_row_kernel<1024, 3, 1>, 1024, vals + (size_t)R * sizeof(float));
+        if (R <= 256 * 8) rc = go(softmax_row_kernel<256, 1, 4>, 256);
+        else if (many && R <= 256 * 16) rc = go(softmax_row_kernel<256, 2, 4>, 256);
+        else if (many && R <= 256 * 40) rc = go(softmax_row_kernel<256, 5, 3>, 256);
+        else if (R <= 512 * 8) rc = go(softmax_row_kernel<512, 1, 2>, 512);
+        else if (R <= 512 * 16) rc = go(softmax_row_kernel<512, 2, 2>, 512);
+        else if (R <= 512 * 24) rc = go(softmax_row_kernel<512, 3, 2>, 512);
+        else rc = go(softmax_row_kernel<1024, 3, 1>, 1024);
         if (rc != AKV_OK) return rc;
     } else if (split) {
         dim3 grid(sm_chunks, B * H * G);
