@@ -39,8 +39,10 @@ __host__ __device__ constexpr int stage_bytes(int kch) { return TILES * f_tile(k
 }  // namespace kc
 
 namespace kc {
-// Per warp: two sets of union masks (16 words) - the producer is at most STAGES - 1 stages ahead of the consumer, less than a
-// unit's stages, so at most one (batch, KV head) ahead - and the consumer's tables.  G == 1: D words q (both halves equal), two
+// Per warp: two sets of union masks (16 words) and the consumer's tables.  Two sets are enough while the producer, STAGES - 1
+// stages ahead, is at most one (batch, KV head) ahead: the launcher takes no ring of more stages than a unit has (with five
+// stages of 16 channels and D = 64 it issued the last stage of the next head, and loaded the set after that over the current
+// one, before the current head's last stage was multiplied).  G == 1: D words q (both halves equal), two
 // sets that come and go with the masks.  G > 1, one set, loaded when the consumer enters a (batch, KV head): per query head
 // D words mask and D words constant (of the head's alignment code on the channel), D fp16 q.
 constexpr int MASK_BYTES = 64;
@@ -406,14 +408,14 @@ int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* 
     // count so that every warp gets (nearly) the same whole number of units.
     const int sms = sm_count();
     const int budget = max_dyn_smem();
-    // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of
-    // its group size, and the shared-memory budget below is computed from what is actually launched
-    // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of its group
+    // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of its group,
+    // and the shared-memory budget below is computed from what is actually launched
     const int kch = group > 1 ? gqa_kch(group) : tuning().k_kch;
     int stages = tuning().k_stages;
     if (group > 1) stages = gqa_stages(group);
     else if (!((kch == 8 && (stages == 3 || stages == 4 || stages == 6)) || (kch == 16 && stages >= 3 && stages <= 5)))
         stages = (kch == 8) ? 4 : 3;
+    if (group == 1 && stages > D / kch) stages = D / kch;      // (D >= 64: four stages of 16 channels)
     const int per_warp = stages * stage_bytes(kch) + meta_bytes(D, group);
     int wmax = budget / per_warp;
     if (wmax > max_warps(group)) wmax = max_warps(group);
