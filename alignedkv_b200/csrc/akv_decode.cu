@@ -10,6 +10,8 @@
 //   probe       akv_v_compute.cu, then the threshold byte per (batch, head) with the reference's [B,H,H,D] broadcast
 //   P.V         akv_v_compute.cu
 //   tail        adds the residual tokens' contribution
+#include <atomic>
+
 #include "akv_exchange.cuh"
 #include "akv_save.cuh"
 
@@ -470,6 +472,29 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
         res[(size_t)bhq * D + d] = __half_as_ushort(__float2half_rn(v));
     }
 }
+
+// Launch of one form.  The shared-memory limit is an attribute of the kernel on a device, seen by the launches of every host
+// thread: it is set once, to what the device has beside the static part, and not to one call's size.
+template <int NT, int VPT, int MINB>
+struct SoftmaxRow {
+    template <class... Args>
+    static int launch(int rows, size_t bytes, cudaStream_t st, Args... args) {
+        static std::atomic<bool> configured[64];
+        const auto kern = softmax_row_kernel<NT, VPT, MINB>;
+        int dev = -1;
+        cudaGetDevice(&dev);
+        if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+            cudaFuncAttributes a;
+            cudaError_t e = cudaFuncGetAttributes(&a, kern);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem() - (int)a.sharedSizeBytes);
+            if (e != cudaSuccess) return cuda_status(e, "decode_step softmax smem attribute");
+            if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+        }
+        launch_chained(kern, dim3(rows), dim3(NT), bytes, st, args...);
+        return AKV_OK;
+    }
+};
 
 // Rows too long for one CTA's registers, and many of them: three passes over the row, the probe in a launch of its own.
 __global__ void __launch_bounds__(256)
@@ -1088,25 +1113,19 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
         // four as tail_kernel does, whatever the threads hold.
         const bool wide = R > 8192 && R <= 17408 && rows <= 2 * sm_count();
         const int cols = wide ? 512 : 256, shares = G <= 4 && (wide || (R <= 8192 && rows <= 4 * sm_count())) ? 3 : 4;
-        auto go = [&](auto kern, int nt) -> int {
-            if (bytes > 32 * 1024) {
-                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-                if (e != cudaSuccess) return cuda_status(e, "decode_step softmax smem attribute");
-            }
-            launch_chained(kern, dim3(rows), dim3(nt), bytes, st, sc.s, static_cast<const __half*>(q),
-                           static_cast<const __half*>(restk), sc.pval, sc.pidx, sc.stats,
-                           static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn, rest,
-                           sqrtf((float)D), mk, mask_stride, res_v, res_o, cols, shares);
-            return AKV_OK;
+        auto go = [&](auto form) -> int {
+            return form.launch(rows, bytes, st, sc.s, static_cast<const __half*>(q), static_cast<const __half*>(restk), sc.pval,
+                               sc.pidx, sc.stats, static_cast<const uint8_t*>(v_first_8), sc.test_o, max_seq_len, H, G, D, R, qn,
+                               rest, sqrtf((float)D), mk, mask_stride, res_v, res_o, cols, shares);
         };
         const bool many = rows > 2 * sm_count();
-        if (R <= 256 * 8) rc = go(softmax_row_kernel<256, 1, 4>, 256);
-        else if (many && R <= 256 * 16) rc = go(softmax_row_kernel<256, 2, 4>, 256);
-        else if (many && R <= 256 * 40) rc = go(softmax_row_kernel<256, 5, 3>, 256);
-        else if (R <= 512 * 8) rc = go(softmax_row_kernel<512, 1, 2>, 512);
-        else if (R <= 512 * 16) rc = go(softmax_row_kernel<512, 2, 2>, 512);
-        else if (R <= 512 * 24) rc = go(softmax_row_kernel<512, 3, 2>, 512);
-        else rc = go(softmax_row_kernel<1024, 3, 1>, 1024);
+        if (R <= 256 * 8) rc = go(SoftmaxRow<256, 1, 4>());
+        else if (many && R <= 256 * 16) rc = go(SoftmaxRow<256, 2, 4>());
+        else if (many && R <= 256 * 40) rc = go(SoftmaxRow<256, 5, 3>());
+        else if (R <= 512 * 8) rc = go(SoftmaxRow<512, 1, 2>());
+        else if (R <= 512 * 16) rc = go(SoftmaxRow<512, 2, 2>());
+        else if (R <= 512 * 24) rc = go(SoftmaxRow<512, 3, 2>());
+        else rc = go(SoftmaxRow<1024, 3, 1>());
         if (rc != AKV_OK) return rc;
     } else if (split) {
         dim3 grid(sm_chunks, B * H * G);

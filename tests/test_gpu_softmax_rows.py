@@ -171,3 +171,39 @@ def test_residual_tokens(akv_lib, B, H, G, qn, rest, masked):
             layer.v_first_8.data_ptr(), layer.v_mid_4.data_ptr(), layer.v_last_4.data_ptr(), p.data_ptr(),
             layer.scratch[at["amin"]:].data_ptr(), o.data_ptr(), None, 0, B, H, G, R, D, R, qn, 0, stream()))
     assert torch.equal(got.view(torch.int16), (o.float() + res.half().float()).half().view(torch.int16))
+
+
+def test_long_rows_on_two_threads(akv_lib):
+    """Caches of different lengths on two host threads, each with its own stream: rows of 17408 and of 12352 scores, whose
+    softmax asks for different amounts of shared memory of one kernel.  Every call succeeds and repeats its result."""
+    import threading
+
+    from alignedkv_b200.decode import DecodeLayer
+    from alignedkv_b200 import _lib
+    _lib.load()
+    failed = []
+
+    def work(qn):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                g = torch.Generator(device="cuda").manual_seed(qn)
+                rnd = lambda *shape: torch.randn(*shape, device="cuda", generator=g).half()  # noqa: E731
+                layer = DecodeLayer(1, qn + 64, 1, 128, "cuda:0")
+                layer.prefill(rnd(1, qn, 1, 128), rnd(1, qn, 1, 128))
+                q = rnd(1, 1, 1, 128)
+                first = layer.decode(q, append=False).clone()
+                out = torch.empty_like(first)
+                for _ in range(3000):
+                    layer.decode(q, append=False, out=out)
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(out, first):
+                    failed.append(f"{qn}: another result")
+        except Exception as e:  # noqa: BLE001
+            failed.append(f"{qn}: {e}")
+
+    threads = [threading.Thread(target=work, args=(qn,)) for qn in (17344, 12288)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
