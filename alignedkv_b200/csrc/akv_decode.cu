@@ -496,7 +496,8 @@ struct SoftmaxRow {
     }
 };
 
-// Rows too long for one CTA's registers, and many of them: three passes over the row, the probe in a launch of its own.
+// Many rows that are too long for one CTA's registers, or hold residual tokens only: three passes over the row, the probe in
+// a launch of its own.
 __global__ void __launch_bounds__(256)
 softmax_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __half* __restrict__ restk,
                uint16_t* __restrict__ pval, int32_t* __restrict__ pidx, float* __restrict__ stats, int H, int G, int D, int R,
@@ -1092,11 +1093,14 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
     }
     // Rows split across CTAs when they are few and long (softmax_chunk_*); one CTA per row, held in registers, when it has at
     // most 24576 scores; else one CTA in three passes.  (The split form's chunk grid is part of the sequence-sharded
-    // protocol: the line between it and the others stays where it is.)
+    // protocol: the line between it and the others stays where it is.)  Many rows of residual tokens only take the three
+    // passes too: 64 scores are a fraction of the registers' form (13.5 KB of shared memory and the probe's apparatus per row);
+    // a step of 768 / 1760 / 4096 rows of 2 tokens 12.8 / 22.0 / 46.0 us against 14.6 / 24.5 / 51.6.  With few rows (32 / 512:
+    // 8.7 / 14.8 against 7.9 / 12.0) it is the other way round: that form's loads go out together.
     const int sm_chunks = (R + SM_CHUNK - 1) / SM_CHUNK;
     const int rows = B * H * G;
     const bool split = R > 17408 && rows < 2 * sm_count();
-    const bool probed = !split && R <= 1024 * 24;
+    const bool probed = !split && R <= 1024 * 24 && (qn > 0 || rows <= 4 * sm_count());
     // The residual tokens' part of the output without a launch of its own: the softmax CTA of a row computes it beside
     // its probe (into o_main, as fp16), and the exact-order chain kernel adds it in its epilogue.
     const bool fuse_tail = !order_free && !packed_out && qn > 0 && rest > 0 && D <= 256 && probed &&
