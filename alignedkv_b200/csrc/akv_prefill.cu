@@ -311,8 +311,8 @@ int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8,
             S, nmb, max_seq_len, tiles);
     } else {
         const size_t smem = (size_t)2 * PF_BLK * 2 * D;
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) {      // (the device's maximum, not this call's size: the attribute is shared by all host threads)
+            cudaError_t e = cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem());
             if (e != cudaSuccess) return cuda_status(e, "prefill smem attribute");
         }
         prefill_kernel<<<grid, 128, smem, st>>>(

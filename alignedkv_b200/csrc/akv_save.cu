@@ -147,8 +147,9 @@ int launch_k_save(uint8_t* first8, uint8_t* mid4, uint8_t* last4, const uint8_t*
         if (fast) {
             size_t smem = (size_t)64 * 2 * D;
             if (smem > 48 * 1024) {
+                // (the device's maximum, not this call's size: the attribute is shared by all host threads)
                 cudaError_t e = cudaFuncSetAttribute(k_save_block64_kernel<64>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem());
                 if (e != cudaSuccess) return cuda_status(e, "k_cache_save smem attribute");
             }
             dim3 grid(n_blocks, H, bsz);
