@@ -62,3 +62,35 @@ def test_exact_pv_group_of_eight_all_planes(akv_lib):
                                                    da.data_ptr(), out.data_ptr(), None, 0, B, H, G, L, D, n + pad, n, 1, stream()))
     got = out.cpu().numpy().view(np.uint16).reshape(B, H * G, D)
     assert np.array_equal(got, want.view(np.uint16).reshape(B, H * G, D))
+
+
+@pytest.mark.parametrize("B,H,G", [(10, 64, 1), (80, 4, 2), (80, 4, 4), (80, 4, 8)])    # 640 units of one head, 320 of several
+def test_thresholds_of_every_round(akv_lib, B, H, G):
+    """A decode step with more units than fit at once: the threshold bytes that the kernel derives for the units of its second
+    round too, against the rule in integers, and the outputs against the operator with those bytes given."""
+    from alignedkv_b200.decode import DecodeLayer
+    Hq, n = H * G, 192
+    rows, R = B * Hq, n + 64
+    g = torch.Generator(device="cuda").manual_seed(B * H)
+    rnd = lambda *shape: torch.randn(*shape, device="cuda", generator=g).half()  # noqa: E731
+    layer = DecodeLayer(B, R, H, D, "cuda:0", n_q_heads=Hq)
+    v = rnd(B, n, H, D) * torch.exp2(torch.randint(-6, 4, (B, 1, H, 1), device="cuda", generator=g).float()).half()
+    layer.prefill(rnd(B, n, H, D), v)
+    got = layer.decode(rnd(B, 1, Hq, D), append=False)
+    at = {x: layer._scratch_offset(x) for x in ("test_o", "amin")}
+    p = layer.scratch[:rows * R * 2].view(torch.half)
+    amin = layer.scratch[at["amin"]:at["amin"] + rows].clone()
+    exps = (layer.scratch[at["test_o"]:at["test_o"] + rows * D * 2].view(torch.int16).view(rows, D).to(torch.int32) >> 10) & 0x1E
+    v_exp = layer.v_exp_max.view(B, H, D).repeat_interleave(G, 1).view(rows, D).to(torch.int32)
+    # row b * Hq + h of the reference's [B, Hq, Hq] broadcast, read flat (extension/v_cache_file.py:142,156-160)
+    i = torch.arange(rows, device="cuda")
+    bb, hp, he = i // (Hq * Hq), i // Hq % Hq, i % Hq
+    want = ((exps[bb * Hq + hp] + 15 - v_exp[bb * Hq + he]) & 0xFF).amin(dim=1).to(torch.uint8)
+    assert torch.equal(amin, want)
+    assert len(torch.unique(want)) > 2                       # (otherwise a wrong row's byte would pass)
+    o = torch.empty_like(got)
+    check(akv_lib, akv_lib.akv_v_cache_compute_gqa(layer.v_first_8.data_ptr(), layer.v_mid_4.data_ptr(), layer.v_last_4.data_ptr(),
+                                                   p.data_ptr(), want.data_ptr(), o.data_ptr(), None, 0, B, H, G, R, D, R, n, 0,
+                                                   stream()))
+    assert torch.equal(got.view(torch.int16), o.view(torch.int16))
+    assert akv_lib.akv_device_error_flag() == 0
