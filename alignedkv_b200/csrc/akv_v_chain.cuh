@@ -6,9 +6,10 @@
 //
 // Design (B200).  The token order leaves one dependent chain per (batch, query head, channel pair), and the V layout is
 // token-major (a token's 128 high bytes are one row) while a chain thread wants "my channel pairs, next tokens".  That
-// transposition is done by the load instruction: ldmatrix.x4.trans over four token rows (one 8x8 matrix of 16-bit
-// words per token: its eight 16-byte chunks, 128 contiguous bytes, so no bank conflict) hands lane T, for each of
-// the four tokens, one register holding the high-byte pairs of channel pairs 16*(T%4) + T/4 and 16*(T%4) + 8 + T/4.
+// transposition is done by the load instruction: ldmatrix.x4.trans over eight token rows (one 8x8 matrix of 16-bit words
+// per two tokens: four 16-byte chunks of each, the warp's half of the channels) hands lane T, for each two tokens, one
+// register holding their high-byte pairs of channel pair 32*half + 8*(T%4) + T/4.  The two tokens' chunks lie 128 bytes
+// apart, in the same banks: a two-way conflict on every one of these loads.
 // A token that reads no nibble plane - the rule - has the constant low byte 0x80, so its two fp16 words are two byte
 // permutes of that register, the same for every query head of the KV head: a chain warp runs the chains of GH heads, per
 // token two permutes and 2 GH FMAs.
@@ -72,10 +73,6 @@ __device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t a) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(a) : "memory");
 }
-// adds `bytes` to the byte count the current phase waits for (no arrival)
-__device__ __forceinline__ void mbar_expect(uint32_t a, uint32_t bytes) {
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n" ::"r"(a), "r"(bytes) : "memory");
-}
 // arrives and adds `bytes` to the byte count the current phase still waits for
 __device__ __forceinline__ void mbar_arrive_expect(uint32_t a, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(a), "r"(bytes) : "memory");
@@ -101,13 +98,6 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t a, uint32_t parity) {
     }
     atomicOr(&g_v_wait_gave_up, 1u);
     return false;
-}
-// Non-blocking: has the phase with this parity completed?
-__device__ __forceinline__ uint32_t mbar_test(uint32_t a, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-    return ok;
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity) {
     uint32_t ok;
@@ -232,10 +222,6 @@ __global__ void __launch_bounds__(UPC * (2 * NH / GH + vch::helpers(UPC, NH)) * 
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
         sts32(pool + CONST_ROW + lane * 4, 0x80808080u);
-        // (a chain warp loads low bytes from the places of a stage without flagged tokens too, or of a slot that has no stage
-        // yet, without using them: they have to lie inside the pools)
-        for (int s = wi; s < nf; s += HW)
-            for (int i = lane; i < NH * TOK / 2; i += 32) sts32(ring + (uint32_t)s * SLOT + OFF_LOW + i * 4, 0u);
     }
     pdl_enter();
     __syncthreads();
