@@ -240,12 +240,12 @@ __device__ __forceinline__ void residual_scores(uint16_t* __restrict__ row, cons
 // columns through shared memory, residual tokens in `shares`.  (Adding each thread's own vectors needs no barrier and no
 // shared memory, and moved a decoder's logits by 8e-4.)
 // With few rows the chain of loads, three reductions and the probe's gathers counts, with many the instructions
-// per score: about 14, of which the division takes three - quotient by the reciprocal of the sum, then one residual
-// correction (Markstein 1990: correctly rounded, as the division it replaces).  MINB: CTAs per SM.
-// Measured (cold, one launch): 256 rows of 4160 scores 8.9 us, 512 rows of 1088 with 48 residual tokens 11.0, 32 rows of
-// 16448 9.7, 2048 rows of 8192 43.4.  The form before it - scores one at a time, 17 to 34 a thread, exponential, division
-// and checks at 105 instructions per score; for the last, probe and residual part in launches of their own - took 11.2,
-// 21.9, 12.6 and 45.9 + 14.1 + 25.5.
+// per score: about 15, of which the division takes three - quotient by the reciprocal of the sum, then one residual
+// correction (Markstein 1990; the same as the division after rounding to fp16, which is all that leaves).  MINB: CTAs per SM.
+// Measured (cold, one launch): 256 rows of 4160 scores 9.1 us, 512 rows of 1088 with 48 residual tokens 11.2, 32 rows of
+// 16448 10.0, 2048 rows of 8192 43.3 (up to 0.3 of it for the columns).  The form before it - scores one at a time, 17 to 34
+// a thread, exponential, division and checks at 105 instructions per score; for the last, probe and residual part in launches
+// of their own - took 11.2, 21.9, 12.6 and 45.9 + 14.1 + 25.5.
 template <int NT, int VPT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
 softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const __half* __restrict__ restk,
@@ -1110,7 +1110,14 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
     const __half* res_v = fuse_tail ? static_cast<const __half*>(restv) : nullptr;
     uint16_t* res_o = fuse_tail ? sc.o_main : nullptr;
     if (probed) {
-        // Few rows: many threads per row, for its latency.  Many rows: few, for rows in flight.
+        // Few rows: many threads per row, for its latency.  Many rows: few, for rows in flight.  A whole decode step in us, by
+        // form (threads x vectors each; the one taken first):
+        //   256 rows    4096 scores: 512 x 1 93.1, 256 x 2 94.6     8192: 512 x 2 155.1, 256 x 5 156.6, 1024 x 3 162.6
+        //   320 rows    4096: 256 x 2 133.6, 512 x 1 136.2          8192: 256 x 5 220.4, 512 x 2 222.9
+        //   512 rows   10240: 256 x 5 362.7, 512 x 3 362.8         12288: 512 x 3 426.4, 1024 x 3 441.1, three passes 447.3
+        //              16448: 1024 x 3 572.6, three passes 582.4   24576: 828.8, 858.3
+        //   2048 rows  10240: 256 x 5 630.3, 512 x 3 643.8, three passes 671.9   12288: 512 x 3 741.0, 1024 x 3 793.6, 776.3
+        //              16448: 1024 x 3 990.6, three passes 980.2 (the one place where the line could lie lower)
         const size_t bytes = (res_v ? (size_t)rest * D * 2 : 0) + ((size_t)R + 16) * sizeof(float);
         // The order of the additions, which is part of the result (softmax_row_kernel): the exponentials in 256 columns, 512
         // for few rows of 8193 to 17408 scores, the residual tokens in three shares for few rows and groups of up to four, else in

@@ -176,14 +176,13 @@ def test_k_compute_gqa(akv_lib, B, H, G, nb, nmb, reference):
     (1, 4, 1, 255, 3, 512, "order_free"),      # multi-head, order-free P.V, first token flushes
     (2, 2, 2, 128, 3, 256, "order_free"),
     (1, 2, 4, 29, 2, 64, "exact"),             # nothing quantized yet
-    (1, 4, 1, 12400, 3, 12480, "exact"),       # few long rows: the softmax is split across CTAs (4 chunks)
-    (1, 2, 2, 12350, 2, 12416, "order_free"),  # a row of 12416 scores: the 512-thread softmax with the probe fused in
+    (1, 4, 1, 12400, 3, 12480, "exact"),       # rows of 12416 scores: the 1024-thread softmax
+    (1, 2, 2, 12350, 2, 12416, "order_free"),  # a row of 12352 scores: the shortest of that form
     (1, 2, 2, 19990, 2, 20032, "order_free"),  # split softmax (rows too long for one CTA), residual tail in the last chunk
                                                # (heads in multiples of four: the reference's kernels, and with them
                                                # the oracle, cover heads in groups of four)
-    (1, 4, 1, 9000, 2, 9088, "exact"),         # rows too long for the register-cached softmax, too short to split:
-                                               # plain softmax + separate probe and threshold launches
-    (10, 8, 8, 100, 2, 128, "exact"),          # many rows (640): the probe is not fused into the softmax CTAs
+    (1, 4, 1, 9000, 2, 9088, "exact"),         # few rows of 9024 scores: the 512-thread softmax
+    (10, 8, 8, 100, 2, 128, "exact"),          # many rows (640): residual tokens in four shares
 ])
 def test_decode_step_ex(akv_lib, B, H, G, prompt, steps, max_len, v_mode):
     """DecodeLayer (akv_decode_step_ex) with a group and either P.V kernel against the oracle pipeline: planes
