@@ -449,22 +449,21 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
     }
     if (!with_res) return;                                       // (uniform)
     // residual part (D <= 256): item = (channel pair, share g of the tokens), fp32 sums, the shares added in order
-    const int first = NT >= 2 * hd ? hd : 0;                     // (beside the probe's chain where there are threads left)
-    if (tid >= first)
-        for (int i = tid - first; i < shares * hd; i += NT - first) {
-            const int g = i / hd, c = i - g * hd;
-            const __half2* vr = reinterpret_cast<const __half2*>(dyn) + c;
-            float a0 = 0.f, a1 = 0.f;
+    // (items are dealt out behind the threads that run the probe's chain, and to those last)
+    for (int i = tid < hd ? tid + NT - hd : tid - hd; i < shares * hd; i += NT) {
+        const int g = i / hd, c = i - g * hd;
+        const __half2* vr = reinterpret_cast<const __half2*>(dyn) + c;
+        float a0 = 0.f, a1 = 0.f;
 #pragma unroll 4
-            for (int r = g; r < rest; r += shares) {
-                const float2 f = __half22float2(vr[r * hd]);
-                const float pv = __half2float(__ushort_as_half(rs[r]));
-                a0 = fmaf(pv, f.x, a0);
-                a1 = fmaf(pv, f.y, a1);
-            }
-            part[g][2 * c] = a0;
-            part[g][2 * c + 1] = a1;
+        for (int r = g; r < rest; r += shares) {
+            const float2 f = __half22float2(vr[r * hd]);
+            const float pv = __half2float(__ushort_as_half(rs[r]));
+            a0 = fmaf(pv, f.x, a0);
+            a1 = fmaf(pv, f.y, a1);
         }
+        part[g][2 * c] = a0;
+        part[g][2 * c + 1] = a1;
+    }
     __syncthreads();
     for (int d = tid; d < D; d += NT) {
         float v = part[0][d];
