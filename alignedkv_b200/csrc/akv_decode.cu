@@ -13,6 +13,7 @@
 #include <atomic>
 
 #include "akv_exchange.cuh"
+#include "akv_row.cuh"
 #include "akv_save.cuh"
 
 namespace akv {
@@ -43,9 +44,7 @@ int launch_v_probe(const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, int
                    cudaStream_t);
 int launch_lse_merge(const float*, uint8_t*, int, int, int, cudaStream_t);
 
-constexpr int TOPK = 32;     // residue classes of the magnitude probe (extension/v_cache_file.py:16)
 constexpr int SM_CHUNK = 4096;   // scores per CTA of the split softmax
-constexpr int BLK = 64;      // tokens per K block (extension/k_cache_file.py:5-6)
 
 // Workspace of one decode step.  H = KV heads, Hq = query heads.
 struct Scratch {
@@ -189,43 +188,6 @@ __device__ __forceinline__ float masked_score(const uint16_t* __restrict__ row, 
     if (mrow) s = __hadd(s, mrow[t]);
     return __half2float(s);
 }
-// Scores of the residual tokens of one (batch, query head) row, by 256 threads: thread = (token tid / 4,
-// quarter tid % 4 of the channels in 16-byte pieces), all loads of a row in flight at once, fp32 dot product rounded to
-// fp16, then divided by sqrt(D) and rounded again, which is what `matmul(q, restk^T) / sqrt(D)` on fp16 tensors
-// produces (k_cache_file.py:156-157).  Returned by the first thread of each token's four, 0 <= tid / 4 < rest < 64.
-__device__ __forceinline__ __half residual_score(const __half* __restrict__ qr, const __half* __restrict__ restk, int b, int h,
-                                                 int H, int D, int rest, float sqrt_d, bool wanted) {
-    const int r = threadIdx.x >> 2, c = threadIdx.x & 3;
-    float acc = 0.f;
-    if (wanted && r < rest) {
-        const __half* kr = restk + (((size_t)b * BLK + r) * H + h) * D;
-#pragma unroll 4
-        for (int d = c * 8; d < D; d += 32) {
-            const uint4 kv = *reinterpret_cast<const uint4*>(kr + d), qv = *reinterpret_cast<const uint4*>(qr + d);
-            const __half2* k2 = reinterpret_cast<const __half2*>(&kv);
-            const __half2* q2 = reinterpret_cast<const __half2*>(&qv);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 kf = __half22float2(k2[i]), qf = __half22float2(q2[i]);
-                acc = fmaf(qf.x, kf.x, acc);
-                acc = fmaf(qf.y, kf.y, acc);
-            }
-        }
-    }
-    acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
-    acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
-    return __float2half_rn(__half2float(__float2half_rn(acc)) / sqrt_d);
-}
-// The same for a CTA of 256 threads, written into the row; only tokens with t_lo <= qn + r < t_hi (a row split across CTAs).
-__device__ __forceinline__ void residual_scores(uint16_t* __restrict__ row, const __half* __restrict__ qr,
-                                                const __half* __restrict__ restk, int b, int h, int H, int D, int qn,
-                                                int rest, float sqrt_d, int t_lo, int t_hi) {
-    const int r = threadIdx.x >> 2;
-    const bool mine = r < rest && qn + r >= t_lo && qn + r < t_hi;
-    const __half v = residual_score(qr, restk, b, h, H, D, rest, sqrt_d, mine);
-    if (mine && (threadIdx.x & 3) == 0) row[qn + r] = __half_as_ushort(v);
-}
-
 // One CTA per row, which stays in registers: thread = vectors tid, tid + NT, ... of 8 consecutive scores, VPT of them.
 // One 16-byte load and store per vector; the residual tokens' scores go straight from their dot products to the vectors
 // that hold them.  A thread's vectors all have the same eight residue classes (token index mod 32: 8 (tid % 4) + 0..7), so
@@ -418,35 +380,8 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
     if (qn == 0) return;                                         // (uniform)
     __syncthreads();
     const int hd = D >> 1;
-    // probe: o_test[d] = sum_j |half((first_8[row_j][d] << 8) + 0x80)| * p_j over the class maxima, rows
-    // row_j = class position * 32 + j, accumulated in fp16 in j order.  The rows are gathered by the whole CTA, 16 bytes a
-    // thread (all 32 rows of 128 bytes in one load), 256 channels at a time.
-    const uint8_t* F = first8 + (size_t)(bhq / G) * max_seq_len * D;
-    const bool vec = (reinterpret_cast<uintptr_t>(F) & 15u) == 0;
-    for (int d0 = 0; d0 < D; d0 += 256) {
-        const int dn = min(256, D - d0);
-        if (d0 > 0) __syncthreads();
-        auto src = [&](int j) { return F + (size_t)min((int)key[1][j] * TOPK + j, max_seq_len - 1) * D + d0; };
-        if (vec) {
-            const int per = dn >> 4;                             // 16-byte pieces of a row (D is a multiple of 64)
-            for (int i = tid; i < TOPK * per; i += NT)
-                *reinterpret_cast<uint4*>(&rows[i / per][16 * (i % per)]) = __ldg(reinterpret_cast<const uint4*>(src(i / per)) + i % per);
-        } else {
-            const int per = dn >> 1;
-            for (int i = tid; i < TOPK * per; i += NT)
-                *reinterpret_cast<uint16_t*>(&rows[i / per][2 * (i % per)]) = __ldg(reinterpret_cast<const uint16_t*>(src(i / per)) + i % per);
-        }
-        __syncthreads();
-        for (int c = tid; 2 * c < dn; c += NT) {
-            uint32_t acc = 0;
-#pragma unroll 8
-            for (int j = 0; j < TOPK; ++j) {
-                const uint32_t f = *reinterpret_cast<const uint16_t*>(&rows[j][2 * c]);
-                acc = hfma2_bits(__byte_perm(f, 0x80u, 0x1404) & 0x7FFF7FFFu, key[0][j] | (key[0][j] << 16), acc);
-            }
-            reinterpret_cast<uint32_t*>(test_o)[(size_t)bhq * hd + (d0 >> 1) + c] = acc;
-        }
-    }
+    probe_row<NT>(first8 + (size_t)(bhq / G) * max_seq_len * D, key, rows, reinterpret_cast<uint32_t*>(test_o) + (size_t)bhq * hd,
+                  max_seq_len, D);
     if (!with_res) return;                                       // (uniform)
     // residual part (D <= 256): item = (channel pair, share g of the tokens), fp32 sums, the shares added in order
     // (items are dealt out behind the threads that run the probe's chain, and to those last)

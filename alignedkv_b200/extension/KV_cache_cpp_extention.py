@@ -128,5 +128,39 @@ class _CudaModule:
         _lib.check("v_cache_compute", rc)
         return o
 
+    # ---- the cache classes' decoding_compute as one call each (no counterpart in the reference's extension)
+    def _call(self, fn: str, dev: torch.device, *args) -> None:
+        f = getattr(self._lib, fn)
+        if torch.cuda.current_device() == dev.index:
+            rc = f(*args, _stream(dev))
+        else:
+            with torch.cuda.device(dev):
+                rc = f(*args, _stream(dev))
+        _lib.check(fn, rc)
+
+    def k_scores(self, k_cache_first_8, k_cache_mid_4, k_cache_last_4, k_exp_max, restk, q, bsz, n_kv_heads, n_blocks,
+                 n_max_blocks, d_head, rest_len, sqrt_dim, reference) -> torch.Tensor:
+        dev = q.device
+        s = torch.empty((bsz, n_kv_heads, 1, (n_blocks + 1) * 64), dtype=torch.half, device=dev)
+        n = self._lib.akv_operator_scratch_bytes(bsz, n_kv_heads, d_head)
+        ws = torch.empty(n, dtype=torch.uint8, device=dev)
+        self._call("akv_k_scores", dev, _u8("k_cache_first_8", k_cache_first_8, dev), _u8("k_cache_mid_4", k_cache_mid_4, dev),
+                   _u8("k_cache_last_4", k_cache_last_4, dev), k_exp_max.data_ptr(), restk.data_ptr(), q.data_ptr(),
+                   s.data_ptr(), ws.data_ptr(), n, bsz, n_kv_heads, n_blocks, n_max_blocks, d_head, rest_len, sqrt_dim,
+                   int(bool(reference)))
+        return s
+
+    def v_output(self, v_cache_first_8, v_cache_mid_4, v_cache_last_4, v_exp_max, restv, s, bsz, n_kv_heads, max_seq_len,
+                 head_dim, n, rest_len, reference) -> torch.Tensor:
+        dev = s.device
+        o = torch.empty((bsz, n_kv_heads, 1, head_dim), dtype=torch.half, device=dev)
+        nb = self._lib.akv_operator_scratch_bytes(bsz, n_kv_heads, head_dim)
+        ws = torch.empty(nb, dtype=torch.uint8, device=dev)
+        self._call("akv_v_output", dev, _u8("v_cache_first_8", v_cache_first_8, dev), _u8("v_cache_mid_4", v_cache_mid_4, dev),
+                   _u8("v_cache_last_4", v_cache_last_4, dev), v_exp_max.data_ptr(), restv.data_ptr(), s.data_ptr(),
+                   o.data_ptr(), ws.data_ptr(), nb, bsz, n_kv_heads, max_seq_len, head_dim, s.shape[-1], n, rest_len,
+                   int(bool(reference)))
+        return o
+
 
 cuda_module = _CudaModule()

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import torch
+from torch.autograd import forward_ad
 
 # One K channel row of a block holds 256 bits of high bytes = 64 tokens (extension/k_cache_file.py:5-6).
 bits_in_a_channel = 256
@@ -16,6 +17,29 @@ def exponent_field(x: torch.Tensor) -> torch.Tensor:
     """5-bit biased exponent of every fp16 element, as uint8 (the reference's
     `(x.view(int16) >> 10).to(uint8) & 0x1F`, e.g. extension/k_cache_file.py:77-78,98-99,136)."""
     return (x.view(torch.int16) >> 10).to(torch.uint8) & 0x1F
+
+
+def one_call(x: torch.Tensor, rest: torch.Tensor | None, exp_max: torch.Tensor, planes, rest_shape, exp_shape) -> bool:
+    """Whether `decoding_compute` may run as one library call (`cuda_module.k_scores` / `v_output`) instead of tensor
+    operations: plain contiguous 16-byte aligned CUDA tensors of the cache's own shapes on one device, nothing that autograd,
+    forward-mode derivatives or a tensor subclass would have to see.  Everything else takes the tensor operations, and fails
+    there where it failed before."""
+    if type(x) is not torch.Tensor or not x.is_cuda or x.dtype != torch.half or not x.is_contiguous() or type(rest) is not torch.Tensor:
+        return False
+    if rest.dtype != torch.half or rest.shape != rest_shape or not rest.is_contiguous() or rest.device != x.device:
+        return False
+    if exp_max.dtype != torch.uint8 or exp_max.shape != exp_shape or not exp_max.is_contiguous() or exp_max.device != x.device:
+        return False
+    if torch.is_grad_enabled() and (x.requires_grad or rest.requires_grad):
+        return False
+    if forward_ad._current_level >= 0:
+        return False
+    at = x.data_ptr() | rest.data_ptr() | exp_max.data_ptr()
+    for p in planes:
+        if p.device != x.device:
+            return False
+        at |= p.data_ptr()
+    return at % 16 == 0
 
 
 class ResidualBuffer:

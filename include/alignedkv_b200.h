@@ -120,6 +120,28 @@ int akv_v_cache_compute(const void* v_first_8, const void* v_mid_4, const void* 
                         int start_pos_add_seqlen, int reference, void* stream);
 
 /*
+ * K_Cache_Class.decoding_compute (extension/k_cache_file.py:132-159) as one call: alignment inputs from q and k_exp_max
+ * [B,1,H,D] u8, scores of the n_blocks quantized blocks and of the rest_len (0..64) tokens in restk [B,64,H,D] fp16, -inf up
+ * to the end.  s: fp16 [B,H,1,(n_blocks+1)*64].  inv_sqrt_dim: factor of the quantized blocks' scores (the operator's
+ * sqrt_dim).  head_dim a multiple of 64, at most 1024.  Scores of quantized tokens equal k_cache_compute's; those of residual
+ * tokens are fp32 dot products like torch's, which may be added in another order.
+ */
+int akv_k_scores(const void* k_first_8, const void* k_mid_4, const void* k_last_4, const void* k_exp_max, const void* restk,
+                 const void* q, void* s, void* scratch, long long scratch_bytes, int bsz, int n_heads, int n_blocks,
+                 int n_max_blocks, int head_dim, int rest_len, float inv_sqrt_dim, int reference, void* stream);
+/*
+ * V_Cache_Class.decoding_compute (extension/v_cache_file.py:119-190) with top_max_k 32 as one call: class maxima of the first
+ * n probabilities (n a positive multiple of 64, at most 2^21; any fp16 values), magnitude probe, threshold bytes, P.V and the
+ * rest_len (0..64) tokens in restv [B,64,H,D] fp16.  s: fp16 rows of s_last_dim (a multiple of 8, at least n + rest_len),
+ * out: fp16 [B,H,1,D].  head_dim a multiple of 64, at most 256.
+ */
+int akv_v_output(const void* v_first_8, const void* v_mid_4, const void* v_last_4, const void* v_exp_max, const void* restv,
+                 const void* s, void* out, void* scratch, long long scratch_bytes, int bsz, int n_heads, int max_seq_len,
+                 int head_dim, int s_last_dim, int n, int rest_len, int reference, void* stream);
+/* Bytes of workspace either needs (16-byte aligned; -1 on bad extents). */
+long long akv_operator_scratch_bytes(int bsz, int n_heads, int head_dim);
+
+/*
  * One decode step of one layer in a single call: what the reference does between receiving (q, k_new, v_new) of a
  * decode token and returning the attention output - K_Cache_Class.save + decoding_compute
  * (extension/k_cache_file.py:97-118,132-159), the fp32 softmax (model/KVCache_AlignedKV.py:119-121; without a mask -

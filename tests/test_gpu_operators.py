@@ -1,0 +1,107 @@
+"""The cache classes' `decoding_compute` as one library call against the tensor operations it stands for."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def make(B, H, D, P, seed, extra=0):
+    from alignedkv_b200.extension.k_cache_file import K_Cache_Class
+    from alignedkv_b200.extension.v_cache_file import V_Cache_Class
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    k = torch.randn(B, P, H, D, device="cuda", generator=g)
+    k[..., [3, 34]] *= 20
+    v = torch.randn(B, P, H, D, device="cuda", generator=g)
+    L = -(-(P + 1) // 64) * 64 + extra
+    kc, vc = K_Cache_Class(B, L, H, D, 0), V_Cache_Class(B, L, H, D, 0)
+    kc.save(k.half(), 0, P)
+    vc.save(v.half(), 0, P)
+    return kc, vc, torch.randn(B, 1, H, D, device="cuda", generator=g).half()
+
+
+def both(monkeypatch, call):
+    """(result of one library call, result of the tensor operations)"""
+    from alignedkv_b200.extension import k_cache_file, v_cache_file
+    seen = []
+    for m in (k_cache_file, v_cache_file):
+        ok = m.one_call
+        monkeypatch.setattr(m, "one_call", lambda *a, ok=ok: seen.append(ok(*a)) or seen[-1])
+    one = call()
+    assert seen == [True], "the call took the tensor operations"
+    for m in (k_cache_file, v_cache_file):
+        monkeypatch.setattr(m, "one_call", lambda *a: False)
+    many = call()
+    monkeypatch.undo()
+    return one, many
+
+
+def same(a, b):
+    return torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("reference", [False, True])
+@pytest.mark.parametrize("B,H,D,P", [(1, 1, 64, 1), (2, 3, 128, 63), (1, 8, 128, 64), (3, 5, 128, 65), (2, 4, 192, 191),
+                                     (1, 2, 256, 130), (2, 32, 128, 2085), (1, 2, 320, 70)])
+def test_scores(monkeypatch, B, H, D, P, reference):
+    kc, _, q = make(B, H, D, P, P)
+    one, many = both(monkeypatch, lambda: kc.decoding_compute(q, P - 1, 1, reference))
+    n = P // 64 * 64
+    assert one.shape == many.shape and same(one[..., :n], many[..., :n]) and same(one[..., P:], many[..., P:])
+    # residual tokens: a dot product rounded to fp16, then a division rounded to fp16, each off by at most one fp16 step when
+    # the fp32 sum is added in another order or divided through the reciprocal
+    a, b = one[..., n:P].float(), many[..., n:P].float()
+    assert bool(((a - b).abs() <= 2 * 2.0 ** -10 * b.abs() + 2.0 ** -14).all())
+
+
+@pytest.mark.parametrize("reference", [False, True])
+@pytest.mark.parametrize("B,H,D,P,kind", [(1, 1, 64, 64, "softmax"), (2, 3, 128, 65, "softmax"), (2, 4, 192, 127, "softmax"),
+                                          (2, 2, 256, 200, "softmax"), (2, 32, 128, 2085, "softmax"), (1, 3, 128, 640, "flat"),
+                                          (2, 3, 128, 300, "negative"), (2, 3, 128, 321, "nan"), (1, 2, 128, 8192, "ties")])
+def test_output(monkeypatch, B, H, D, P, kind, reference):
+    _, vc, _ = make(B, H, D, P, P, extra=64 if P % 128 else 0)
+    g = torch.Generator(device="cuda").manual_seed(P)
+    W = -(-(P + 1) // 64) * 64
+    s = torch.randn(B, H, 1, W, device="cuda", generator=g) * (0.02 if kind == "flat" else 1.0)
+    s[..., P:] = -torch.inf
+    p = torch.softmax(s, -1).half()
+    if kind == "negative":                     # any fp16 value is a legal "probability" of the operator
+        p = torch.randn(B, H, 1, W, device="cuda", generator=g).half().neg().abs().neg()
+        p[..., ::3] = -0.0
+    elif kind == "nan":
+        p[0, 0, 0, 40], p[0, 0, 0, 104], p[1, 2, 0, 7] = torch.nan, torch.nan, torch.inf
+    elif kind == "ties":
+        p = torch.full_like(p, 1 / 4096)
+    one, many = both(monkeypatch, lambda: vc.decoding_compute(p, P - 1, 1, reference))
+    assert one.shape == many.shape
+    if P % 64 == 0:
+        assert bool(((one == many) | (one.isnan() & many.isnan())).all())
+        return
+    # the residual part is rounded to fp16 before it is added: its last bit may differ, then the sum's
+    nan = many.isnan()
+    assert bool((one.isnan() == nan).all())
+    a, b = one[~nan].float(), many[~nan].float()
+    rest = torch.matmul(p[..., P // 64 * 64:P].float(), vc.restv.transpose(1, 2)[:, :, :P % 64].float())[~nan].abs()
+    fin = b.isfinite()
+    assert bool((a == b)[~fin].all())
+    assert bool(((a - b).abs() <= 2.0 ** -10 * (b.abs() + rest) + 2.0 ** -14)[fin].all())
+
+
+def test_routes():
+    """What has to be seen by autograd, is not contiguous or has another top_max_k keeps the tensor operations."""
+    from alignedkv_b200.extension._planes import one_call
+    kc, _, q = make(2, 3, 128, 70, 1)
+    planes = (kc.k_cache_first_8, kc.k_cache_mid_4, kc.k_cache_last_4)
+    shapes = ((2, 64, 3, 128), (2, 1, 3, 128))
+    assert one_call(q, kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    assert not one_call(q.clone().requires_grad_(), kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    with torch.no_grad():
+        assert one_call(q.clone().requires_grad_(), kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    assert not one_call(q.float(), kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    assert not one_call(q.transpose(2, 3).contiguous().transpose(2, 3), kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    assert not one_call(torch.nn.Parameter(q, requires_grad=False), kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    flat = torch.empty(q.numel() + 1, dtype=torch.half, device="cuda")[1:].view(q.shape)
+    assert not one_call(flat, kc.restk, kc.k_cache_exp_column_max, planes, *shapes)
+    qg = q.clone().requires_grad_()
+    s = kc.decoding_compute(qg, 69, 1)
+    s[..., 64:70].float().sum().backward()
+    assert qg.grad is not None and bool((qg.grad != 0).any())
