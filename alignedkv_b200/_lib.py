@@ -49,6 +49,9 @@ SIGNATURES = {
     "akv_operator_scratch_bytes": (ctypes.c_longlong, [_I] * 3),
     "akv_k_scores": (_I, [_P] * 8 + [ctypes.c_longlong] + [_I] * 6 + [_F, _I, _P]),
     "akv_v_output": (_I, [_P] * 8 + [ctypes.c_longlong] + [_I] * 8 + [_P]),
+    "akv_rope_split": (_I, [_P] * 5 + [_I] * 4 + [_F, _P]),
+    "akv_rms_norm": (_I, [_P] * 3 + [_I] * 2 + [_F, _P]),
+    "akv_silu_mul": (_I, [_P] * 2 + [_I] * 2 + [_P]),
     "akv_timing_reset": (_I, []),
     "akv_timing_read": (_I, [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)]),
 }

@@ -16,6 +16,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
+from . import _lib
 from .decode import DecodeLayer
 
 __all__ = ["LlamaConfig", "LlamaDecoder"]
@@ -111,8 +112,6 @@ class LlamaDecoder:
             else:
                 self.kcache[i][:, :S] = k
                 self.vcache[i][:, :S] = v
-        elif self.attention == "alignedkv":
-            o = self.caches[i].decode(q, k, v)                                   # [B,1,H,D]
         else:
             n = self.pos + 1
             self.kcache[i][:, self.pos:n] = k
@@ -127,23 +126,48 @@ class LlamaDecoder:
         gate, up = F.linear(h, p["w_gate_up"]).chunk(2, dim=-1)
         return torch.addmm(x.view(B * S, -1), F.silu(gate).mul_(up).view(B * S, -1), p["w_down"].t()).view(B, S, -1)
 
-    # ------------------------------------------------------------------ decode step with the dense parts as CUDA graphs
-    def _pre(self, i: int, x: torch.Tensor, tables):
-        """Everything of layer i before its attention: norm, q/k/v projection, rotary embedding."""
+    # ------------------------------------------------------------------ one layer of a decode step through the cache
+    def _pre(self, i: int, x: torch.Tensor, pos: torch.Tensor):
+        """Everything of layer i before its attention: norm, q/k/v projection, rotary embedding at position pos[0]."""
         cfg, p = self.cfg, self.layers[i]
         H, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         B = x.shape[0]
-        qkv = F.linear(_rms_norm(x, p["norm1"], cfg.rms_norm_eps), p["wqkv"]).view(B, 1, H + 2 * Hkv, D)
-        qk = _rope(qkv[:, :, :H + Hkv], tables)
-        return qk[:, :, :H].contiguous(), qk[:, :, H:].contiguous(), qkv[:, :, H + Hkv:].contiguous()
+        qkv = F.linear(self._norm(x, p["norm1"]), p["wqkv"]).view(B, 1, H + 2 * Hkv, D)
+        if D % 16 or D > 256:
+            qk = _rope(qkv[:, :, :H + Hkv], _rope_tables(pos, D, cfg.rope_theta))
+            return qk[:, :, :H].contiguous(), qk[:, :, H:].contiguous(), qkv[:, :, H + Hkv:].contiguous()
+        q, k, v = (torch.empty(B, 1, n, D, dtype=torch.half, device=x.device) for n in (H, Hkv, Hkv))
+        self._native("akv_rope_split", qkv.data_ptr(), pos.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), B, H, Hkv, D,
+                     cfg.rope_theta)
+        return q, k, v
 
     def _post(self, i: int, x: torch.Tensor, o: torch.Tensor) -> torch.Tensor:
         """Everything of layer i after its attention: output projection, residual, SwiGLU MLP, residual."""
         cfg, p = self.cfg, self.layers[i]
-        B = x.shape[0]
+        B, Fi = x.shape[0], cfg.intermediate_size
         x = torch.addmm(x.view(B, -1), o.reshape(B, -1), p["wo"].t()).view(B, 1, -1)
-        gate, up = F.linear(_rms_norm(x, p["norm2"], cfg.rms_norm_eps), p["w_gate_up"]).chunk(2, dim=-1)
-        return torch.addmm(x.view(B, -1), F.silu(gate).mul_(up).view(B, -1), p["w_down"].t()).view(B, 1, -1)
+        gate_up = F.linear(self._norm(x, p["norm2"]), p["w_gate_up"])
+        if Fi % 8:
+            gate, up = gate_up.chunk(2, dim=-1)
+            h = F.silu(gate).mul_(up).view(B, -1)
+        else:
+            h = torch.empty(B, Fi, dtype=torch.half, device=x.device)
+            self._native("akv_silu_mul", gate_up.data_ptr(), h.data_ptr(), B, Fi)
+        return torch.addmm(x.view(B, -1), h, p["w_down"].t()).view(B, 1, -1)
+
+    def _norm(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+        """RMSNorm of a decode step's rows [B,1,E]."""
+        E = x.shape[-1]
+        if E % 8 or E > 16384 or w.dtype != torch.half or not w.is_contiguous() or w.data_ptr() % 16:
+            return _rms_norm(x, w, self.cfg.rms_norm_eps)
+        out = torch.empty_like(x)
+        self._native("akv_rms_norm", x.data_ptr(), w.data_ptr(), out.data_ptr(), x.shape[0], E, self.cfg.rms_norm_eps)
+        return out
+
+    def _native(self, fn: str, *args) -> None:
+        with torch.cuda.device(self.device):
+            rc = getattr(_lib.load(), fn)(*args, torch.cuda.current_stream(self.device).cuda_stream)
+        _lib.check(fn, rc)
 
     @torch.no_grad()
     def capture_graphs(self) -> None:
@@ -161,15 +185,14 @@ class LlamaDecoder:
         segs = []          # (graph, outputs) per stretch
 
         def run(j, x_prev):
-            tables = _rope_tables(self._g_pos, D, cfg.rope_theta)
             if j == 0:
                 x = self.embed[self._g_ids].view(B, 1, -1)
             else:
                 x = self._post(j - 1, x_prev, self._g_o)
             if j == n:
-                x = _rms_norm(x, self.final_norm, cfg.rms_norm_eps)
+                x = self._norm(x, self.final_norm)
                 return (F.linear(x, self.lm_head)[:, 0],)
-            return (x,) + self._pre(j, x, tables)
+            return (x,) + self._pre(j, x, self._g_pos)
 
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
@@ -204,13 +227,20 @@ class LlamaDecoder:
 
     def _forward(self, ids: torch.Tensor, prompt: bool) -> torch.Tensor:
         B, S = ids.shape
-        pos = _rope_tables(torch.arange(self.pos, self.pos + S, device=self.device), self.cfg.head_dim,
-                           self.cfg.rope_theta)
+        pos = torch.arange(self.pos, self.pos + S, device=self.device)
         x = self.embed[ids]
-        for i in range(self.cfg.num_hidden_layers):
-            x = self._layer(i, x, pos, prompt)
+        if prompt or self.attention != "alignedkv":
+            tables = _rope_tables(pos, self.cfg.head_dim, self.cfg.rope_theta)
+            for i in range(self.cfg.num_hidden_layers):
+                x = self._layer(i, x, tables, prompt)
+        else:
+            for i in range(self.cfg.num_hidden_layers):
+                x = self._post(i, x, self.caches[i].decode(*self._pre(i, x, pos)))
         self.pos += S
-        x = _rms_norm(x[:, -1:], self.final_norm, self.cfg.rms_norm_eps)
+        if prompt or self.attention != "alignedkv":
+            x = _rms_norm(x[:, -1:], self.final_norm, self.cfg.rms_norm_eps)
+        else:
+            x = self._norm(x, self.final_norm)
         return F.linear(x, self.lm_head)[:, 0]                                   # logits of the last position [B,V]
 
     # ------------------------------------------------------------------ public

@@ -142,6 +142,19 @@ int akv_v_output(const void* v_first_8, const void* v_mid_4, const void* v_last_
 long long akv_operator_scratch_bytes(int bsz, int n_heads, int head_dim);
 
 /*
+ * Element-wise parts of a decoder layer's decode step (model/Llama_AlignedKV.py; see llama.py).
+ * akv_rope_split: qkv fp16 [B, H + 2 Hkv, D] -> q [B,H,D], k, v [B,Hkv,D]; q and k rotated to position pos[0] (int64 in device
+ * memory), rotate_half form, tables and rotation in fp32.  head_dim a multiple of 16, at most 256.
+ * akv_silu_mul: gate_up fp16 [rows, 2 width] -> out [rows, width] = half(silu(gate)) * up.  width a multiple of 8.
+ * akv_rms_norm: out = half(x / sqrt(mean(x^2) + eps) * w) per row of `width` fp16 values (a multiple of 8, at most 16384).
+ * All pointers 16-byte aligned (pos: 8).
+ */
+int akv_rms_norm(const void* x, const void* w, void* out, int rows, int width, float eps, void* stream);
+int akv_rope_split(const void* qkv, const void* pos, void* q, void* k, void* v, int bsz, int n_heads, int n_kv_heads,
+                   int head_dim, float theta, void* stream);
+int akv_silu_mul(const void* gate_up, void* out, int rows, int width, void* stream);
+
+/*
  * One decode step of one layer in a single call: what the reference does between receiving (q, k_new, v_new) of a
  * decode token and returning the attention output - K_Cache_Class.save + decoding_compute
  * (extension/k_cache_file.py:97-118,132-159), the fp32 softmax (model/KVCache_AlignedKV.py:119-121; without a mask -
