@@ -123,6 +123,13 @@ __device__ __forceinline__ uint32_t hmul2_bits(uint32_t a, uint32_t b) {
     return d;
 }
 
+// c.x += p * (low half of v), c.y += p * (high half of v): products of two fp16 values are exact in fp32, one rounding each.  The
+// sm_100 multiply-add that takes fp16 factors and an fp32 addend: no conversions.
+__device__ __forceinline__ void fma_f32_f16x2(float& x, float& y, uint32_t v, uint32_t p) {
+    asm("{\n.reg .f16 l, h;\nmov.b32 {l, h}, %2;\nfma.rn.f32.f16 %0, l, %3, %0;\nfma.rn.f32.f16 %1, h, %3, %1;\n}\n"
+        : "+f"(x), "+f"(y) : "r"(v), "h"((uint16_t)p));
+}
+
 // Threshold byte of P.V for flat row i = b*Hq + h of the reference's [B,Hq,Hq,1] tensor, computed by one warp:
 // min_d ((exp(test_o[bb, hp, d]) & 0x1E) + 15 - v_exp[bb, he, d]) mod 256 with bb = i / (Hq*Hq), hp = (i / Hq) % Hq,
 // he = i % Hq (extension/v_cache_file.py:142,156-160).  The exponent maxima are stored per KV head; query head he

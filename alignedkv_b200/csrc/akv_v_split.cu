@@ -40,13 +40,10 @@ __device__ __forceinline__ uint2 ldg64_stream(const void* p) {
     asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "l"(p));
     return v;
 }
-__device__ __forceinline__ float2 h2f2(uint32_t h2) {
-    return __half22float2(*reinterpret_cast<const __half2*>(&h2));
-}
 
-// acc[0..15] += p * value(channel 16cg + k), values rebuilt from 16 high bytes and the per-channel low bytes
+// acc[0..15] += p (fp16 bits) * value(channel 16cg + k), values rebuilt from 16 high bytes and the per-channel low bytes
 // lo_e (even channels of each pair, 8 bytes) / lo_o (odd channels).
-__device__ __forceinline__ void fma16(float (&acc)[16], float pf, const uint4& hi, uint2 lo_e, uint2 lo_o) {
+__device__ __forceinline__ void fma16(float (&acc)[16], uint32_t p, const uint4& hi, uint2 lo_e, uint2 lo_o) {
     const uint32_t hw[4] = {hi.x, hi.y, hi.z, hi.w};
     const uint32_t le[2] = {lo_e.x, lo_e.y}, lo[2] = {lo_o.x, lo_o.y};
 #pragma unroll
@@ -55,12 +52,8 @@ __device__ __forceinline__ void fma16(float (&acc)[16], float pf, const uint4& h
         const uint32_t lew = le[j >> 1] >> ((j & 1) * 16), low = lo[j >> 1] >> ((j & 1) * 16);
         const uint32_t lob = (lew & 0xFFu) | ((low & 0xFFu) << 8) | ((lew & 0xFF00u) << 8) | ((low & 0xFF00u) << 16);
         // lob bytes: [lo(4j), lo(4j+1), lo(4j+2), lo(4j+3)]
-        const float2 a = h2f2(__byte_perm(hw[j], lob, 0x1504));   // [lo0, hi0, lo1, hi1]
-        const float2 b = h2f2(__byte_perm(hw[j], lob, 0x3726));   // [lo2, hi2, lo3, hi3]
-        acc[4 * j + 0] = fmaf(pf, a.x, acc[4 * j + 0]);
-        acc[4 * j + 1] = fmaf(pf, a.y, acc[4 * j + 1]);
-        acc[4 * j + 2] = fmaf(pf, b.x, acc[4 * j + 2]);
-        acc[4 * j + 3] = fmaf(pf, b.y, acc[4 * j + 3]);
+        fma_f32_f16x2(acc[4 * j], acc[4 * j + 1], __byte_perm(hw[j], lob, 0x1504), p);       // [lo0, hi0, lo1, hi1]
+        fma_f32_f16x2(acc[4 * j + 2], acc[4 * j + 3], __byte_perm(hw[j], lob, 0x3726), p);   // [lo2, hi2, lo3, hi3]
     }
 }
 
@@ -118,7 +111,7 @@ __global__ void __launch_bounds__(128) v_split_kernel(const VSplitParams p) {
                 const uint2 c80 = make_uint2(0x80808080u, 0x80808080u);
 #pragma unroll
                 for (int g = 0; g < G; ++g)
-                    fma16(acc[g], __half2float(__ushort_as_half((unsigned short)sb[g])), hi[i], c80, c80);
+                    fma16(acc[g], sb[g], hi[i], c80, c80);
             } else {
                 const uint2 mrow = ldg64_stream(M + (size_t)(t0 + i) * HD);
                 const uint2 lrow = (ucode == 0) ? ldg64_stream(L + (size_t)(t0 + i) * HD) : make_uint2(0, 0);
@@ -133,7 +126,7 @@ __global__ void __launch_bounds__(128) v_split_kernel(const VSplitParams p) {
                     lo_e.y = (mb.y & 0xF0F0F0F0u) | ((lb.y >> 4) & 0x0F0F0F0Fu);
                     lo_o.x = ((mb.x << 4) & 0xF0F0F0F0u) | (lb.x & 0x0F0F0F0Fu);
                     lo_o.y = ((mb.y << 4) & 0xF0F0F0F0u) | (lb.y & 0x0F0F0F0Fu);
-                    fma16(acc[g], __half2float(__ushort_as_half((unsigned short)sb[g])), hi[i], lo_e, lo_o);
+                    fma16(acc[g], sb[g], hi[i], lo_e, lo_o);
                 }
             }
         }
