@@ -19,6 +19,7 @@ void count_launch(int n = 1);   // every kernel launch of this library is counte
 struct Tuning {
     int k_kch = 16;     // channels per stage of the q.K^T kernel (8 or 16)
     int k_stages = 3;   // ring depth per warp of the q.K^T kernel (3..6, see launch_k_compute)
+    int k_tiles = 0;    // 64-token blocks per unit of the q.K^T kernel: 0 = by the number of blocks, 1, 4
     int timing = 0;     // 1: akv_decode_step records CUDA events around its two streaming kernels
     int k_wpc = 0;      // cap on warps per CTA of the q.K^T kernel (0 = as many as shared memory allows)
     int pdl = 1;        // 1: the kernels of a decode step are chained with programmatic dependent launch
@@ -43,12 +44,24 @@ static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t
 
 // ---------------------------------------------------------------- programmatic dependent launch
 // The kernels of one decode step form a chain in one stream.  Launched with the programmatic-serialization
-// attribute, a kernel's CTAs may become resident while its predecessor is still running; every such kernel calls
-// pdl_enter() first: it lets ITS successor be scheduled early and then blocks until the predecessor grid has
-// completed and its memory is visible.  Without the attribute both instructions are no-ops.
+// attribute, a kernel's CTAs may become resident while its predecessor is still running; every such kernel waits (pdl_wait)
+// until the predecessor grid has completed and its memory is visible, and lets ITS successor be scheduled early (pdl_trigger).
+// Without the attribute both instructions are no-ops.
+//   pdl_enter   trigger, then wait: for kernels whose successor touches nothing before its own wait.
+//   pdl_turn    wait, then trigger: once the successor runs, everything in front of this kernel is complete and visible.  A
+//               successor that is told so by its launcher may read, before its wait, what this kernel does not write - the
+//               planes, above all: their first stages are then on their way while this kernel still runs.  Such reads go past
+//               L1 (asynchronous copies, ld.relaxed).
+// Whatever a kernel reads early, every kernel waits before it completes: completion stays transitive along the stream.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    pdl_trigger();
+    pdl_wait();
+}
+__device__ __forceinline__ void pdl_turn() {
+    pdl_wait();
+    pdl_trigger();
 }
 template <class Kernel, class... Args>
 static inline cudaError_t launch_chained(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
@@ -128,6 +141,18 @@ __device__ __forceinline__ uint32_t hmul2_bits(uint32_t a, uint32_t b) {
 __device__ __forceinline__ void fma_f32_f16x2(float& x, float& y, uint32_t v, uint32_t p) {
     asm("{\n.reg .f16 l, h;\nmov.b32 {l, h}, %2;\nfma.rn.f32.f16 %0, l, %3, %0;\nfma.rn.f32.f16 %1, h, %3, %1;\n}\n"
         : "+f"(x), "+f"(y) : "r"(v), "h"((uint16_t)p));
+}
+
+// Global loads past L1, of what another kernel may be storing
+__device__ __forceinline__ uint32_t ld_relaxed8(const uint8_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_relaxed16(const uint16_t* p) {
+    uint16_t v;
+    asm volatile("ld.relaxed.gpu.global.u16 %0, [%1];\n" : "=h"(v) : "l"(p) : "memory");
+    return v;
 }
 
 // Threshold byte of P.V for flat row i = b*Hq + h of the reference's [B,Hq,Hq,1] tensor, computed by one warp:

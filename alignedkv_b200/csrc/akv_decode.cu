@@ -23,6 +23,9 @@ int launch_k_save(uint8_t*, uint8_t*, uint8_t*, const uint8_t*, int, int, int, i
                   cudaStream_t);
 int launch_k_compute(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*,
                      const uint8_t*, uint8_t*, int, int, int, int, int, int, int, float, int, cudaStream_t);
+int launch_k_compute_align(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*,
+                           uint8_t*, int, int, int, int, int, int, int, float, int, const uint8_t*, const uint16_t*, cudaStream_t);
+bool k_compute_aligns(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, int, int);
 int launch_v_compute(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*,
                      int, int, int, int, int, int, int, int, cudaStream_t);
 bool v_compute_takes_probe(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, int, int, int,
@@ -114,7 +117,7 @@ append_flush_kernel(uint32_t* __restrict__ restk, uint32_t* __restrict__ restv, 
                     int B, int H, int G, int D, int rest_len, int append, int nmb, int max_seq_len, int qn) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t red[4];
-    pdl_enter();
+    pdl_turn();
     const int BH = B * H, hd = D >> 1;
     if ((int)blockIdx.x < BH) {
         const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
@@ -222,7 +225,7 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
     __shared__ float part[4][256];
     __shared__ __align__(16) uint8_t rows[TOPK][256];            // the probe's rows
     extern __shared__ __align__(16) uint8_t dyn[];               // residual values [rest][D] (res), then exponentials [R + 16]
-    pdl_enter();
+    pdl_turn();
     const int bhq = blockIdx.x, Hq = H * G, b = bhq / Hq, h = (bhq - b * Hq) / G;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint16_t* row = s + (size_t)bhq * R;
@@ -1018,10 +1021,16 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
     cudaEvent_t* ev = timing_slot();
     if (nb > 0) {
         if (ev) cudaEventRecord(ev[0], st);
-        rc = launch_k_compute(static_cast<const uint8_t*>(k_first_8), static_cast<const uint8_t*>(k_mid_4),
-                              static_cast<const uint8_t*>(k_last_4), sc.kq, sc.kqmax, static_cast<const uint8_t*>(q),
-                              reinterpret_cast<uint8_t*>(sc.s), B, H, G, nb, nmb, D, BLK, 1.0f / sqrtf((float)D),
-                              reference, st);
+        // a step that flushes no block: q.K^T makes its alignment inputs itself and runs beside the append kernel
+        const bool aligns = !flush &&
+            k_compute_aligns(static_cast<const uint8_t*>(k_first_8), static_cast<const uint8_t*>(k_mid_4),
+                             static_cast<const uint8_t*>(k_last_4), sc.kq, static_cast<const uint8_t*>(q),
+                             reinterpret_cast<const uint8_t*>(sc.s), G, D);
+        rc = launch_k_compute_align(static_cast<const uint8_t*>(k_first_8), static_cast<const uint8_t*>(k_mid_4),
+                                    static_cast<const uint8_t*>(k_last_4), sc.kq, sc.kqmax, static_cast<const uint8_t*>(q),
+                                    reinterpret_cast<uint8_t*>(sc.s), B, H, G, nb, nmb, D, BLK, 1.0f / sqrtf((float)D),
+                                    reference, aligns ? static_cast<const uint8_t*>(k_exp_max) : nullptr,
+                                    aligns && append ? static_cast<const uint16_t*>(k_new) : nullptr, st);
         if (ev) cudaEventRecord(ev[1], st);
         if (rc != AKV_OK) return rc;
     }

@@ -26,19 +26,22 @@
 // batch 8 x 8 x 8192 but 228 against 223 at batch 64, where the copies are what is left (a stage's issue stalls for 450 to
 // 770 cycles on the load unit; neither bulk copies nor TMA boxes, built and bit-exact, moved these pieces faster).
 // With G == 1 the producer writes the constants into the skipped rows' slots instead.
+// In a decode step that flushes no block the kernel makes its alignment inputs itself and runs beside the append kernel in front of
+// it (KParams::k_exp): batch 8 x 32 heads x 4096 tokens 80.5 -> 78.7 us per step, 16 x 32 x 1000 56.6 -> 53.0, one sequence of
+// 16384 tokens 54.4 -> 53.3.  Bulk copies of the pieces (high bytes and mid plane, 1 KB and 512 bytes) were built again for this
+// form and are slower: 80.3, 54.0, and 8 KV heads x 4, batch 64 x 8192 tokens 532 against 512.
+#include <atomic>
+
 #include "akv_common.cuh"
 
 namespace akv {
 
 namespace kc {
-constexpr int TILES = 4;                         // 64-token blocks per warp unit
 constexpr int MAX_D = 256;
-__host__ __device__ constexpr int f_tile(int kch) { return kch * 64 + 64; }   // +64: tiles land on distinct banks
-__host__ __device__ constexpr int n_tile(int kch) { return kch * 32 + 32; }
-__host__ __device__ constexpr int stage_bytes(int kch) { return TILES * f_tile(kch) + 2 * TILES * n_tile(kch); }
-}  // namespace kc
-
-namespace kc {
+// A unit = TILES consecutive 64-token blocks, a stage = KCH channels of them.  (Padding: the tiles of a stage lie on distinct banks.)
+__host__ __device__ constexpr int f_tile(int kch, int tiles) { return kch * 64 + (tiles > 1 ? 64 : 0); }
+__host__ __device__ constexpr int n_tile(int kch, int tiles) { return kch * 32 + (tiles > 1 ? 32 : 0); }
+__host__ __device__ constexpr int stage_bytes(int kch, int tiles) { return tiles * (f_tile(kch, tiles) + 2 * n_tile(kch, tiles)); }
 // Per warp: two sets of union masks (16 words) and the consumer's tables.  Two sets are enough while the producer, STAGES - 1
 // stages ahead, is at most one (batch, KV head) ahead: the launcher takes no ring of more stages than a unit has (with five
 // stages of 16 channels and D = 64 it issued the last stage of the next head, and loaded the set after that over the current
@@ -68,6 +71,10 @@ struct KParams {
     int units, upw;       // total units, units per warp (contiguous run)
     uint32_t scale2;      // half(sqrt_dim) in both halves
     int reference;
+    // k_exp != nullptr: kq and kqmax are made here from q, the exponent maxima and the new token (k_new, null: none), which the
+    // kernel in front of this one may still be storing, and the planes are read before that kernel has completed (pdl_turn)
+    const uint8_t* k_exp;
+    const uint16_t* k_new;
 };
 
 __device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t v) {
@@ -83,6 +90,23 @@ __device__ __forceinline__ uint32_t kc_fma(uint32_t k, __half2 q, uint32_t acc) 
     const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&k), q, *reinterpret_cast<const __half2*>(&acc));
     return *reinterpret_cast<const uint32_t*>(&r);
 }
+// A row of a stage as fp16x2 words, all planes: tokens (0, 2), (1, 3), (4, 6), (5, 7) of the lane's eight - with one tile its two.
+template <int TILES>
+__device__ __forceinline__ void kc_row(uint32_t (&w)[TILES], const uint8_t* f, const uint8_t* m, const uint8_t* l) {
+    if (TILES == 4) {
+        const uint2 fw = *reinterpret_cast<const uint2*>(f);
+        const uint32_t M = *reinterpret_cast<const uint32_t*>(m), L = *reinterpret_cast<const uint32_t*>(l);
+        const uint32_t lbe = (M & 0xF0F0F0F0u) | ((L >> 4) & 0x0F0F0F0Fu);   // low bytes, tokens 0,2,4,6
+        const uint32_t lbo = ((M << 4) & 0xF0F0F0F0u) | (L & 0x0F0F0F0Fu);   // low bytes, tokens 1,3,5,7
+        w[0] = __byte_perm(lbe, fw.x, 0x6140);
+        w[1 % TILES] = __byte_perm(lbo, fw.x, 0x7150);
+        w[2 % TILES] = __byte_perm(lbe, fw.y, 0x6342);
+        w[3 % TILES] = __byte_perm(lbo, fw.y, 0x7352);
+    } else {
+        const uint32_t fw = *reinterpret_cast<const uint16_t*>(f), M = *m * 0x1001u, L = *l * 0x1001u;
+        w[0] = __byte_perm((M & 0xF0F0u) | ((L >> 4) & 0x0F0Fu), fw, 0x5140);
+    }
+}
 
 // Position of a stream of stages (unit, channel chunk) inside one warp's run of units.
 struct KCursor {
@@ -91,22 +115,133 @@ struct KCursor {
     size_t row;               // plane row index of (tile 0 of the unit, first channel of the chunk)
 };
 
-template <int KCH, int STAGES, int G>
-__global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(const KParams p) {
+// Query bits and alignment differences of heads g0 .. g0 + HC - 1 of a group on channels r * 32 + lane: mid plane read iff
+// (u8)(kqmax - kq[d]) < 8, low plane iff < 4 (K_cache.cu:211,249-250).  kq and kqmax as they are given, or made here from the
+// query, the exponent maxima and the new token (k_cache_file.py:98-99,136-138).
+template <int G, int HC>
+__device__ __forceinline__ void kc_load_heads(const KParams& p, long long bh, int g0, int lane, uint32_t (&qh)[HC][8],
+                                              uint32_t (&diff)[HC][8]) {
+    uint32_t ek[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int d = r * 32 + lane;
+        const bool in = d < p.D;
+        ek[r] = 0;
+        if (p.k_exp && in) {
+            // (old or new maximum: the token's exponent is taken in again)
+            ek[r] = ld_relaxed8(p.k_exp + bh * p.D + d);
+            if (p.k_new) ek[r] = max(ek[r], (ld_relaxed16(p.k_new + bh * p.D + d) >> 10) & 0x1Fu);
+        }
+#pragma unroll
+        for (int g = 0; g < HC; ++g) {
+            const long long at = (bh * G + g0 + g) * p.D + d;
+            qh[g][r] = in ? ld_relaxed16(reinterpret_cast<const uint16_t*>(p.q) + at) : 0u;
+            diff[g][r] = !p.k_exp && in ? __ldg(p.kq + at) : 0u;
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < HC; ++g) {
+        uint32_t top = 0;
+        if (p.k_exp) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (r * 32 + lane < p.D) {
+                    diff[g][r] = (((qh[g][r] >> 10) & 0x1Fu) + ek[r]) & 0xFFu;
+                    top = max(top, diff[g][r]);
+                }
+            top = __reduce_max_sync(0xFFFFFFFFu, top);
+        } else {
+            top = __ldg(p.kqmax + bh * G + g0 + g);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) diff[g][r] = p.reference ? 0u : (top - diff[g][r]) & 0xFFu;
+    }
+}
+// The union of the group's plane-read masks (bit d set = row d of that plane is read), which is what the producer fetches; with
+// one head its table too.
+template <int G>
+__device__ __forceinline__ void kc_load_masks(const KParams& p, long long bh, uint32_t* um, uint32_t* table, int lane) {
+    constexpr int HC = G > 4 ? 4 : G;             // (registers)
+    uint32_t least[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) least[r] = 0xFFu;
+#pragma unroll 1
+    for (int g0 = 0; g0 < G; g0 += HC) {
+        uint32_t qh[HC][8], diff[HC][8];
+        kc_load_heads<G, HC>(p, bh, g0, lane, qh, diff);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int d = r * 32 + lane;
+            if (d >= p.D) break;
+#pragma unroll
+            for (int g = 0; g < HC; ++g) least[r] = min(least[r], diff[g][r]);
+            if (G == 1) table[d] = qh[0][r] | (qh[0][r] << 16);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (r * 32 >= p.D) break;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, least[r] < 8), l = __ballot_sync(0xFFFFFFFFu, least[r] < 4);
+        if (lane == 0) {
+            um[r] = m;
+            um[8 + r] = l;
+        }
+    }
+    __syncwarp();
+}
+// (Groups: out of the loop's instruction stream and registers.  One head is faster inline, 78.8 against 80.0 us per step at
+// batch 8 x 32 x 4096; four the other way round, 515 against 510 at batch 64 x 8 x 8192.)
+template <int G>
+__device__ __noinline__ void kc_load_masks_far(const KParams& p, long long bh, uint32_t* um, uint32_t* table, int lane) {
+    kc_load_masks<G>(p, bh, um, table, lane);
+}
+// The consumer's tables of a group (all its lanes are done with the previous ones).
+template <int G>
+__device__ __noinline__ void kc_load_tables(const KParams& p, long long bh, uint8_t* tables, int lane) {
+    constexpr int HC = G > 4 ? 4 : G;
+    __syncwarp();
+#pragma unroll 1
+    for (int g0 = 0; g0 < G; g0 += HC) {
+        uint32_t qh[HC][8], diff[HC][8];
+        kc_load_heads<G, HC>(p, bh, g0, lane, qh, diff);
+#pragma unroll
+        for (int g = 0; g < HC; ++g) {
+            uint32_t* hm = reinterpret_cast<uint32_t*>(tables + (size_t)(g0 + g) * kc::head_meta(p.D, G));
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int d = r * 32 + lane;
+                if (d >= p.D) break;
+                const uint32_t x = diff[g][r];
+                hm[d] = x < 4 ? 0xFFFFFFFFu : x < 8 ? 0xFFF0FFF0u : 0xFF00FF00u;
+                hm[p.D + d] = x < 4 ? 0u : x < 8 ? 0x00080008u : 0x00800080u;
+                reinterpret_cast<uint16_t*>(hm + 2 * p.D)[d] = (uint16_t)qh[g][r];
+            }
+        }
+    }
+    __syncwarp();
+}
+
+template <int KCH, int STAGES, int G, int TILES>
+__global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(const __grid_constant__ KParams p) {
     using namespace kc;
-    constexpr int F_TILE = f_tile(KCH), N_TILE = n_tile(KCH);
+    constexpr int F_TILE = f_tile(KCH, TILES), N_TILE = n_tile(KCH, TILES);
     constexpr int F_BYTES = TILES * F_TILE, N_BYTES = TILES * N_TILE, STAGE = F_BYTES + 2 * N_BYTES;
     constexpr int F_IT = KCH / 8;                 // 16-byte copies per lane and tile for the high-byte plane
     constexpr int ROW_LANES = 2 * KCH;            // lanes that cover the nibble rows of one tile
     constexpr int TILES_PER_IT = 32 / ROW_LANES;  // 1 (KCH 16) or 2 (KCH 8)
-    static_assert(KCH == 8 || KCH == 16, "channels per stage");
+    constexpr int N_IT = (TILES + TILES_PER_IT - 1) / TILES_PER_IT;
+    static_assert((KCH == 8 || KCH == 16) && (TILES == 1 || TILES == 4), "channels per stage, tiles per unit");
     extern __shared__ __align__(128) uint8_t smem[];
-    pdl_enter();
+    pdl_trigger();
+    if (!p.k_exp) pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wpc = blockDim.x >> 5;
     const int w = blockIdx.x * wpc + warp;
     const int u_begin = w * p.upw;
-    if (u_begin >= p.units) return;
+    if (u_begin >= p.units) {
+        if (p.k_exp) pdl_wait();
+        return;
+    }
     const int u_end = (u_begin + p.upw < p.units) ? u_begin + p.upw : p.units;
     const int nch = p.D / KCH;
     const int total = (u_end - u_begin) * nch;
@@ -134,7 +269,7 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         k.c = 0;
         ++k.u;
         if (++k.g < p.ngroups) {
-            k.row += (size_t)(TILES - 1) * p.D;          // next 4 tiles of the same (batch, KV head)
+            k.row += (size_t)(TILES - 1) * p.D;          // next tiles of the same (batch, KV head)
             return false;
         }
         k.g = 0;
@@ -143,60 +278,14 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         k.row = (size_t)k.bh * p.nmb * p.D;
         return true;
     };
-    // Alignment code of channel d for query head bhq: mid plane read iff (u8)(kqmax - kq[d]) < 8, low plane iff < 4
-    // (K_cache.cu:211,249-250)
-    auto diff_of = [&](long long bhq, int d, uint32_t top) {
-        return p.reference ? 0u : (top - (uint32_t)__ldg(p.kq + (size_t)bhq * p.D + d)) & 0xFFu;
-    };
-    // The union of the group's plane-read masks (bit d set = row d of that plane is read), which is what the producer fetches;
-    // with one head its table too
     auto load_masks = [&](long long bh, int slot) {
         uint32_t* um = reinterpret_cast<uint32_t*>(meta0 + slot * MASK_BYTES);
-        uint32_t top[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) top[g] = __ldg(p.kqmax + bh * G + g);
-        uint32_t least[8], qh[8];                 // (all loads before the first vote)
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int d = r * 32 + lane;
-            least[r] = 0xFFu;
-            qh[r] = 0;
-            if (d < p.D) {
-#pragma unroll
-                for (int g = 0; g < G; ++g) least[r] = min(least[r], diff_of(bh * G + g, d, top[g]));
-                if (G == 1) qh[r] = __ldg(reinterpret_cast<const uint16_t*>(p.q) + (size_t)bh * p.D + d);
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            if (r * 32 >= p.D) break;
-            const int d = r * 32 + lane;
-            if (G == 1 && d < p.D) reinterpret_cast<uint32_t*>(tables + slot * HMETA)[d] = qh[r] | (qh[r] << 16);
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, least[r] < 8), l = __ballot_sync(0xFFFFFFFFu, least[r] < 4);
-            if (lane == 0) {
-                um[r] = m;
-                um[8 + r] = l;
-            }
-        }
-        __syncwarp();
+        uint32_t* table = reinterpret_cast<uint32_t*>(tables + slot * HMETA);
+        if (G == 1) kc_load_masks<G>(p, bh, um, table, lane);
+        else kc_load_masks_far<G>(p, bh, um, table, lane);
     };
-    // The consumer's tables of a group (all its lanes are done with the previous ones)
     auto load_tables = [&](long long bh) {
-        if (G == 1) return;
-        __syncwarp();
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const long long bhq = bh * G + g;
-            uint32_t* hm = reinterpret_cast<uint32_t*>(tables + (size_t)g * HMETA);
-            const uint32_t top = __ldg(p.kqmax + bhq);
-            for (int d = lane; d < p.D; d += 32) {
-                const uint32_t diff = diff_of(bhq, d, top);
-                hm[d] = diff < 4 ? 0xFFFFFFFFu : diff < 8 ? 0xFFF0FFF0u : 0xFF00FF00u;
-                hm[p.D + d] = diff < 4 ? 0u : diff < 8 ? 0x00080008u : 0x00800080u;
-                reinterpret_cast<uint16_t*>(hm + 2 * p.D)[d] = __ldg(reinterpret_cast<const uint16_t*>(p.q) + (size_t)bhq * p.D + d);
-            }
-        }
-        __syncwarp();
+        if (G > 1) kc_load_tables<G>(p, bh, tables, lane);
     };
 
     const int nrow = (lane % ROW_LANES) >> 1, nhalf = (lane & 1) << 4, ntsub = lane / ROW_LANES;
@@ -220,9 +309,9 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         const size_t pn = (pk.row + nrow) * 32 + nhalf;
         const uint32_t nd = st + F_BYTES + nrow * 32 + nhalf;
 #pragma unroll
-        for (int it = 0; it < TILES / TILES_PER_IT; ++it) {   // nibble planes: only the rows some head reads
+        for (int it = 0; it < N_IT; ++it) {              // nibble planes: only the rows some head reads
             const int t = it * TILES_PER_IT + ntsub;
-            if (t < ptiles) {
+            if (t < ptiles && t < TILES) {
                 const uint32_t dm = nd + t * N_TILE, dl = dm + N_BYTES;
                 if (need_m) cp_async16(dm, p.mid4 + pn + t * tile_n);
                 else if (G == 1) st_shared_v4(dm, 0x88888888u);              // plane not read: low byte becomes 0x80
@@ -240,11 +329,12 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         if (j < total) issue();
         cp_async_commit();
     }
-
-    const int tile = lane >> 3, li = lane & 7;
-    uint32_t acc[G][4];
+    const int tile = lane / (32 / TILES), li = lane % (32 / TILES);
+    uint32_t acc[G][TILES];
 #pragma unroll
-    for (int g = 0; g < G; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0;
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int j = 0; j < TILES; ++j) acc[g][j] = 0;
     KCursor ck = cursor_at(u_begin);
     load_tables(ck.bh);
     int cstage = 0;
@@ -256,9 +346,9 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
 
         const uint8_t* stp = ring + (size_t)cstage * STAGE;
         cstage = (cstage + 1 == STAGES) ? 0 : cstage + 1;
-        const uint2* fp = reinterpret_cast<const uint2*>(stp + tile * F_TILE + li * 8);
-        const uint32_t* mp = reinterpret_cast<const uint32_t*>(stp + F_BYTES + tile * N_TILE + li * 4);
-        const uint32_t* lp = reinterpret_cast<const uint32_t*>(stp + F_BYTES + N_BYTES + tile * N_TILE + li * 4);
+        const uint8_t* fp = stp + tile * F_TILE + li * 2 * TILES;
+        const uint8_t* mp = stp + F_BYTES + tile * N_TILE + li * TILES;
+        const uint8_t* lp = mp + N_BYTES;
         const uint8_t* hm0 = tables + (G == 1 ? ck.slot * HMETA : 0);
         const int ch0 = ck.c * KCH;                       // first channel of the stage
         if (G == 1) {
@@ -269,15 +359,11 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
                 for (int rr = 0; rr < 4; ++rr) {
                     // the producer has written the substitutes into the rows it did not fetch
                     const int r = r4 * 4 + rr;
-                    const uint2 f = fp[r * 8];
-                    const uint32_t M = mp[r * 8], L = lp[r * 8];
-                    const uint32_t lbe = (M & 0xF0F0F0F0u) | ((L >> 4) & 0x0F0F0F0Fu);   // low bytes, tokens 0,2,4,6
-                    const uint32_t lbo = ((M << 4) & 0xF0F0F0F0u) | (L & 0x0F0F0F0Fu);   // low bytes, tokens 1,3,5,7
-                    const uint32_t q2 = rr == 0 ? qv.x : rr == 1 ? qv.y : rr == 2 ? qv.z : qv.w;
-                    acc[0][0] = hfma2_bits(__byte_perm(lbe, f.x, 0x6140), q2, acc[0][0]);
-                    acc[0][1] = hfma2_bits(__byte_perm(lbo, f.x, 0x7150), q2, acc[0][1]);
-                    acc[0][2] = hfma2_bits(__byte_perm(lbe, f.y, 0x6342), q2, acc[0][2]);
-                    acc[0][3] = hfma2_bits(__byte_perm(lbo, f.y, 0x7352), q2, acc[0][3]);
+                    uint32_t wd[TILES];
+                    kc_row<TILES>(wd, fp + r * 64, mp + r * 32, lp + r * 32);
+                    const uint32_t q2 = u4w(qv, rr);
+#pragma unroll
+                    for (int j = 0; j < TILES; ++j) acc[0][j] = hfma2_bits(wd[j], q2, acc[0][j]);
                 }
             }
         } else {
@@ -295,20 +381,14 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
 #pragma unroll
                 for (int rr = 0; rr < 4; ++rr) {
                     const int r = r4 * 4 + rr;
-                    const uint2 f = fp[r * 8];
-                    const uint32_t M = mp[r * 8], L = lp[r * 8];
-                    const uint32_t lbe = (M & 0xF0F0F0F0u) | ((L >> 4) & 0x0F0F0F0Fu);   // low bytes, tokens 0,2,4,6
-                    const uint32_t lbo = ((M << 4) & 0xF0F0F0F0u) | (L & 0x0F0F0F0Fu);   // low bytes, tokens 1,3,5,7
-                    const uint32_t w0 = __byte_perm(lbe, f.x, 0x6140), w1 = __byte_perm(lbo, f.x, 0x7150);
-                    const uint32_t w2 = __byte_perm(lbe, f.y, 0x6342), w3 = __byte_perm(lbo, f.y, 0x7352);
+                    uint32_t wd[TILES];
+                    kc_row<TILES>(wd, fp + r * 64, mp + r * 32, lp + r * 32);
 #pragma unroll
                     for (int g = 0; g < G; ++g) {
                         const uint32_t m = u4w(mk[g], rr), c = u4w(cn[g], rr), qw = rr < 2 ? qv[g].x : qv[g].y;
                         const __half2 q2 = kc_dup(qw, rr & 1);
-                        acc[g][0] = kc_fma((w0 & m) | c, q2, acc[g][0]);
-                        acc[g][1] = kc_fma((w1 & m) | c, q2, acc[g][1]);
-                        acc[g][2] = kc_fma((w2 & m) | c, q2, acc[g][2]);
-                        acc[g][3] = kc_fma((w3 & m) | c, q2, acc[g][3]);
+#pragma unroll
+                        for (int j = 0; j < TILES; ++j) acc[g][j] = kc_fma((wd[j] & m) | c, q2, acc[g][j]);
                     }
                 }
             }
@@ -317,26 +397,29 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         const int cg = ck.g;
         const bool last_chunk = (ck.c == nch - 1);
         if (advance(ck) && ck.u < u_end) load_tables(ck.bh);
-        if (last_chunk) {  // unit finished: scale, reorder to token order, one 16-byte store per lane and head
+        if (last_chunk) {  // unit finished: scale, reorder to token order, one store per lane and head
             const int blk = cg * TILES + tile;
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 if (blk < p.nb) {
-                    const uint32_t a0 = hmul2_bits(acc[g][0], p.scale2), a1 = hmul2_bits(acc[g][1], p.scale2);
-                    const uint32_t a2 = hmul2_bits(acc[g][2], p.scale2), a3 = hmul2_bits(acc[g][3], p.scale2);
-                    uint4 o;
-                    o.x = __byte_perm(a0, a1, 0x5410);
-                    o.y = __byte_perm(a0, a1, 0x7632);
-                    o.z = __byte_perm(a2, a3, 0x5410);
-                    o.w = __byte_perm(a2, a3, 0x7632);
-                    const size_t row = (size_t)(cbh * G + g) * (size_t)(p.nb + 1) * 64 + (size_t)blk * 64 + li * 8;
-                    *reinterpret_cast<uint4*>(p.s + row * 2) = o;
+                    uint32_t a[TILES];
+#pragma unroll
+                    for (int j = 0; j < TILES; ++j) a[j] = hmul2_bits(acc[g][j], p.scale2);
+                    const size_t row = (size_t)(cbh * G + g) * (size_t)(p.nb + 1) * 64 + (size_t)blk * 64 + li * 2 * TILES;
+                    uint8_t* dst = p.s + row * 2;
+                    if (TILES == 4)
+                        *reinterpret_cast<uint4*>(dst) = make_uint4(__byte_perm(a[0], a[1 % TILES], 0x5410), __byte_perm(a[0], a[1 % TILES], 0x7632),
+                                                                    __byte_perm(a[2 % TILES], a[3 % TILES], 0x5410),
+                                                                    __byte_perm(a[2 % TILES], a[3 % TILES], 0x7632));
+                    else *reinterpret_cast<uint32_t*>(dst) = a[0];
                 }
-                acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0;
+#pragma unroll
+                for (int j = 0; j < TILES; ++j) acc[g][j] = 0;
             }
         }
     }
     cp_async_wait<0>();
+    if (p.k_exp) pdl_wait();
 }
 
 // Any block length / head size: one thread per token, planes read straight from global memory.
@@ -372,57 +455,35 @@ k_compute_generic_kernel(const uint8_t* __restrict__ first8, const uint8_t* __re
     }
 }
 
-// q.K^T over nb quantized blocks.  H = KV heads, group = query heads per KV head; kq, kqmax, q and the score rows are
-// per (batch, query head) with query head = KV head * group + g.
-int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* kq,
-                     const uint8_t* kqmax, const uint8_t* q, uint8_t* s, int bsz, int H, int group, int nb, int nmb,
-                     int D, int d_block, float sqrt_dim, int reference, cudaStream_t st) {
+// Whether launch_k_compute takes the streaming kernel, which can make the alignment inputs itself.
+static bool k_fast(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* kq, const uint8_t* q,
+                   const uint8_t* s, int group, int D, int d_block) {
+    return d_block == 64 && D % 16 == 0 && D >= 64 && D <= kc::MAX_D && aligned16(first8) && aligned16(mid4) &&
+           aligned16(last4) && aligned16(kq) && aligned16(q) && aligned16(s) &&
+           (group == 1 || group == 2 || group == 4 || group == 8);
+}
+bool k_compute_aligns(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* kq, const uint8_t* q,
+                      const uint8_t* s, int group, int D) {
+    return k_fast(first8, mid4, last4, kq, q, s, group, D, 64);
+}
+
+// Launch of one form: warps per CTA and units per warp, one CTA per SM.
+template <int KCH, int STAGES, int G, int TILES>
+static int k_launch(KParams p, cudaStream_t st) {
     using namespace kc;
-    const __half scale = __float2half_rn(sqrt_dim);
-    const bool fast = d_block == 64 && D % 16 == 0 && D >= 64 && D <= MAX_D && aligned16(first8) &&
-                      aligned16(mid4) && aligned16(last4) && aligned16(kq) && aligned16(q) && aligned16(s) &&
-                      (group == 1 || group == 2 || group == 4 || group == 8);
-    if (!fast) {
-        long long total = (long long)bsz * H * group * nb * d_block;
-        long long want = (total + 127) / 128;
-        int grid = (int)(want < (long long)sm_count() * 16 ? want : (long long)sm_count() * 16);
-        count_launch();
-        k_compute_generic_kernel<<<grid, 128, 0, st>>>(first8, mid4, last4, kq, kqmax,
-                                                       reinterpret_cast<const __half*>(q),
-                                                       reinterpret_cast<__half*>(s), nb, nmb, D, d_block, group,
-                                                       scale, reference, total);
-        return cuda_status(cudaGetLastError(), "k_cache_compute launch");
-    }
-    KParams p;
-    p.first8 = first8; p.mid4 = mid4; p.last4 = last4; p.kq = kq; p.kqmax = kqmax; p.q = q; p.s = s;
-    p.BH = bsz * H; p.nb = nb; p.nmb = nmb; p.D = D;
-    p.ngroups = (nb + TILES - 1) / TILES;
+    p.ngroups = (p.nb + TILES - 1) / TILES;
     const long long units = (long long)p.BH * p.ngroups;
     AKV_REQUIRE(units < (1ll << 30), AKV_ERR_OVERFLOW, "k_cache_compute: too many blocks");
     p.units = (int)units;
-    const unsigned short sb = __half_as_ushort(scale);
-    p.scale2 = (uint32_t)sb | ((uint32_t)sb << 16);
-    p.reference = reference;
-
-    // One CTA per SM.  Pick the channel-chunk size, ring depth and warps per CTA (tunable), trimming the warp
-    // count so that every warp gets (nearly) the same whole number of units.
-    const int sms = sm_count();
-    const int budget = max_dyn_smem();
-    // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of its group,
-    // and the shared-memory budget below is computed from what is actually launched
-    const int kch = group > 1 ? gqa_kch(group) : tuning().k_kch;
-    int stages = tuning().k_stages;
-    if (group > 1) stages = gqa_stages(group);
-    else if (!((kch == 8 && (stages == 3 || stages == 4 || stages == 6)) || (kch == 16 && stages >= 3 && stages <= 5)))
-        stages = (kch == 8) ? 4 : 3;
-    if (group == 1 && stages > D / kch) stages = D / kch;      // (D >= 64: four stages of 16 channels)
-    const int per_warp = stages * stage_bytes(kch) + meta_bytes(D, group);
+    const int sms = sm_count(), budget = max_dyn_smem();
+    const int per_warp = STAGES * stage_bytes(KCH, TILES) + meta_bytes(p.D, G);
     int wmax = budget / per_warp;
-    if (wmax > max_warps(group)) wmax = max_warps(group);
+    if (wmax > max_warps(G)) wmax = max_warps(G);
     if (tuning().k_wpc > 0 && tuning().k_wpc < wmax) wmax = tuning().k_wpc;
     AKV_REQUIRE(wmax >= 1, AKV_ERR_CUDA, "k_cache_compute: %d bytes of shared memory are too few", budget);
     // (fewer units than that: spread over the SMs first, a warp streams the faster the fewer share its SM)
     if (units < (long long)sms * wmax) wmax = (int)((units + sms - 1) / sms);
+    // Trim the warp count so that every warp gets (nearly) the same whole number of units.
     int wpc = wmax;
     double best_eff = -1.0;
     for (int c = wmax; c >= (wmax * 3 + 3) / 4; --c) {
@@ -436,53 +497,90 @@ int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* 
         p.upw = (int)((units + Wt - 1) / Wt);
     }
     const long long warps_needed = (units + p.upw - 1) / p.upw;
-    int grid = (int)((warps_needed + wpc - 1) / wpc);
-    size_t smem = (size_t)wpc * per_warp;
-    auto go = [&](auto kern) -> int {
-        // the opt-in shared-memory size is a per-device attribute of the kernel: set it once per (kernel, device) - to
-        // the device's maximum, so that every launch shape fits - not on every launch
-        static const void* done_kernel[32];
-        static int done_device[32];
-        static int done_count = 0;                 // (guarded by nothing: a racing thread at worst sets it twice)
-        int dev = 0;
-        cudaGetDevice(&dev);
-        const void* kp = reinterpret_cast<const void*>(kern);
-        bool done = false;
-        for (int i = 0; i < done_count && i < 32; ++i) done = done || (done_kernel[i] == kp && done_device[i] == dev);
-        if (!done) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
-            if (e != cudaSuccess) return cuda_status(e, "k_cache_compute smem attribute");
-            if (done_count < 32) {
-                done_kernel[done_count] = kp;
-                done_device[done_count] = dev;
-                ++done_count;
-            }
-        }
-        launch_chained(kern, dim3(grid), dim3(wpc * 32), smem, st, p);
-        return AKV_OK;
-    };
-    int rc;
+    const int grid = (int)((warps_needed + wpc - 1) / wpc);
+    // the opt-in shared-memory size is a per-device attribute of the kernel: set once per device - to the device's maximum, so
+    // that every launch shape fits - not on every launch (a racing thread at worst sets it twice)
+    static std::atomic<bool> configured[64];
+    const auto kern = k_compute_kernel<KCH, STAGES, G, TILES>;
+    int dev = -1;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
+        if (e != cudaSuccess) return cuda_status(e, "k_cache_compute smem attribute");
+        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+    }
+    launch_chained(kern, dim3(grid), dim3(wpc * 32), (size_t)wpc * per_warp, st, p);
+    return cuda_status(cudaGetLastError(), "k_cache_compute launch");
+}
+
+// q.K^T over nb quantized blocks.  H = KV heads, group = query heads per KV head; kq, kqmax, q and the score rows are
+// per (batch, query head) with query head = KV head * group + g.  k_exp != nullptr (only when k_compute_aligns() holds and the
+// kernel launched before is a pdl_turn one that writes no planes): the kernel makes kq and kqmax for itself from q, k_exp and the
+// token k_new (or null), and runs beside that kernel.
+int launch_k_compute_align(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* kq,
+                           const uint8_t* kqmax, const uint8_t* q, uint8_t* s, int bsz, int H, int group, int nb, int nmb,
+                           int D, int d_block, float sqrt_dim, int reference, const uint8_t* k_exp, const uint16_t* k_new,
+                           cudaStream_t st) {
+    using namespace kc;
+    const __half scale = __float2half_rn(sqrt_dim);
+    if (!k_fast(first8, mid4, last4, kq, q, s, group, D, d_block)) {
+        AKV_REQUIRE(!k_exp, AKV_ERR_SHAPE, "k_cache_compute: the aligning form needs the streaming kernel");
+        long long total = (long long)bsz * H * group * nb * d_block;
+        long long want = (total + 127) / 128;
+        int grid = (int)(want < (long long)sm_count() * 16 ? want : (long long)sm_count() * 16);
+        count_launch();
+        k_compute_generic_kernel<<<grid, 128, 0, st>>>(first8, mid4, last4, kq, kqmax,
+                                                       reinterpret_cast<const __half*>(q),
+                                                       reinterpret_cast<__half*>(s), nb, nmb, D, d_block, group,
+                                                       scale, reference, total);
+        return cuda_status(cudaGetLastError(), "k_cache_compute launch");
+    }
+    KParams p;
+    p.first8 = first8; p.mid4 = mid4; p.last4 = last4; p.kq = kq; p.kqmax = kqmax; p.q = q; p.s = s;
+    p.BH = bsz * H; p.nb = nb; p.nmb = nmb; p.D = D;
+    p.ngroups = p.units = p.upw = 0;
+    const unsigned short sb = __half_as_ushort(scale);
+    p.scale2 = (uint32_t)sb | ((uint32_t)sb << 16);
+    p.reference = reference;
+    p.k_exp = k_exp;
+    p.k_new = k_new;
+
+    // Units of one tile for groups of four and eight heads while there are at most four tiles per SM: many short chains of
+    // stages instead of few long ones, their whole depth of channels in flight.  A decode step in us, four tiles against one:
+    // 8 KV heads x 4, batch 1, 700 tokens (80 tiles) 31.8 / 27.0, 4096 tokens (512) 47.6 / 42.8; 4 x 8, 8000 tokens (500)
+    // 78.1 / 69.9; 2000 tiles 67.2 / 75.6.  One head: 384 tiles 25.1 / 24.9, 800 26.7 / 25.9, 1472 26.8 / 29.2.
+    const bool single = tuning().k_tiles ? tuning().k_tiles == 1 : (long long)p.BH * nb <= 4ll * sm_count();
+    if (single && D >= 128 && group == 4) return k_launch<16, 8, 4, 1>(p, st);
+    if (single && D >= 128 && group == 8) return k_launch<16, 8, 8, 1>(p, st);
+    // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of its group
     if (group == 1) {
+        const int kch = tuning().k_kch;
+        int stages = tuning().k_stages;
+        if (!((kch == 8 && (stages == 3 || stages == 4 || stages == 6)) || (kch == 16 && stages >= 3 && stages <= 5)))
+            stages = (kch == 8) ? 4 : 3;
+        if (stages > D / kch) stages = D / kch;      // (D >= 64: four stages of 16 channels)
         switch (kch * 10 + stages) {
-            case 83: rc = go(k_compute_kernel<8, 3, 1>); break;
-            case 84: rc = go(k_compute_kernel<8, 4, 1>); break;
-            case 86: rc = go(k_compute_kernel<8, 6, 1>); break;
-            case 164: rc = go(k_compute_kernel<16, 4, 1>); break;
-            case 165: rc = go(k_compute_kernel<16, 5, 1>); break;
-            case 163: rc = go(k_compute_kernel<16, 3, 1>); break;
+            case 83: return k_launch<8, 3, 1, 4>(p, st);
+            case 84: return k_launch<8, 4, 1, 4>(p, st);
+            case 86: return k_launch<8, 6, 1, 4>(p, st);
+            case 164: return k_launch<16, 4, 1, 4>(p, st);
+            case 165: return k_launch<16, 5, 1, 4>(p, st);
+            case 163: return k_launch<16, 3, 1, 4>(p, st);
             default:
                 set_error("k_cache_compute: no kernel for %d channels x %d stages", kch, stages);
                 return AKV_ERR_SHAPE;
         }
-    } else if (group == 2) {
-        rc = go(k_compute_kernel<gqa_kch(2), gqa_stages(2), 2>);
-    } else if (group == 4) {
-        rc = go(k_compute_kernel<gqa_kch(4), gqa_stages(4), 4>);
-    } else {
-        rc = go(k_compute_kernel<gqa_kch(8), gqa_stages(8), 8>);
     }
-    if (rc != AKV_OK) return rc;
-    return cuda_status(cudaGetLastError(), "k_cache_compute launch");
+    if (group == 2) return k_launch<gqa_kch(2), gqa_stages(2), 2, 4>(p, st);
+    if (group == 4) return k_launch<gqa_kch(4), gqa_stages(4), 4, 4>(p, st);
+    return k_launch<gqa_kch(8), gqa_stages(8), 8, 4>(p, st);
+}
+
+int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* kq,
+                     const uint8_t* kqmax, const uint8_t* q, uint8_t* s, int bsz, int H, int group, int nb, int nmb,
+                     int D, int d_block, float sqrt_dim, int reference, cudaStream_t st) {
+    return launch_k_compute_align(first8, mid4, last4, kq, kqmax, q, s, bsz, H, group, nb, nmb, D, d_block, sqrt_dim,
+                                  reference, nullptr, nullptr, st);
 }
 
 }  // namespace akv

@@ -54,7 +54,7 @@ int akv_device_error_clear(void);
 
 /*
  * Launch-shape knobs for benchmarking ("k_kch" 8|16, "k_stages" 3..6 (at most head_dim / k_kch are used),
- * "k_wpc" 0..16, "timing" 0|1, "pdl" 0|1: chain the kernels of a decode step with programmatic dependent launch; exact P.V:
+ * "k_wpc" 0..16, "k_tiles" 0 by size | 1 | 4: 64-token blocks per unit with groups of 4 and 8, "timing" 0|1, "pdl" 0|1: chain the kernels of a decode step with programmatic dependent launch; exact P.V:
  * "v_impl" 0 chain kernel | 1 producer-transposed kernel, "v_nf" ring depth cap, "v_gqa_form" 0 by size | 1 a ring per
  * query head | 2 one ring per KV head; "k_gqa_kch", "v_nside", "v_upc", "v_npt", "v_ndw", "v_cps" are accepted in their ranges and have
  * no effect any more; order-free P.V: "v_split_impl" 0 staged through shared memory | 1 direct loads).

@@ -1,0 +1,73 @@
+"""q.K^T in units of one 64-token block and of four, bit for bit against the oracle, and a decode step whose q.K^T makes its
+alignment inputs itself (beside the append kernel) against the same step with launches that overlap nothing."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import exponent_field, k_planes_np, make_kvq
+from test_gpu_ext import check, dev, stream, u8
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tiles", [1, 4])
+@pytest.mark.parametrize("B,H,G,D,nb", [(1, 1, 4, 128, 1), (2, 3, 4, 128, 5), (1, 8, 4, 256, 9), (1, 2, 8, 128, 3), (2, 4, 8, 128, 33),
+                                        (1, 3, 8, 256, 2), (9, 8, 4, 128, 8), (1, 2, 4, 144, 7), (1, 2, 2, 128, 6)])
+@pytest.mark.parametrize("reference", [False, True])
+def test_forms(akv_lib, B, H, G, D, nb, tiles, reference):
+    from oracle import akv_oracle as orc
+    lib, Hq, L, nmb = akv_lib, H * G, nb * 64, nb + 1
+    k, _, _ = make_kvq(81, B, L, H, D)
+    _, _, q = make_kvq(82, B, 1, Hq, D)
+    q = (q * 2.0 ** np.random.default_rng(83).integers(-7, 3, size=q.shape)).astype(np.float16)
+    planes = k_planes_np(B, H, nmb, D)
+    orc.k_cache_save(*planes, u8(k), B, H, nb, nmb, D, 64, 0, L)
+    kexp = exponent_field(np.abs(k).max(axis=1, keepdims=True))
+    kq = (exponent_field(q) + np.repeat(kexp, G, axis=2)).astype(np.uint8)
+    kqmax = kq.max(axis=3, keepdims=True)
+    rep = [np.ascontiguousarray(np.repeat(x, G, axis=1)) for x in planes]
+    want, _ = orc.k_cache_compute(*rep, kq, kqmax, u8(q), B, Hq, nb, nmb, D, 64, L, 1 / math.sqrt(D), reference)
+    dp, dkq, dkm, dq = [dev(x) for x in planes], dev(kq), dev(kqmax), dev(u8(q))
+    s = torch.zeros((B, Hq, 1, (nb + 1) * 64), dtype=torch.half, device="cuda")
+    assert lib.akv_set_tuning(b"k_tiles", tiles) == 0
+    try:
+        check(lib, lib.akv_k_cache_compute_gqa(dp[0].data_ptr(), dp[1].data_ptr(), dp[2].data_ptr(), dkq.data_ptr(),
+                                               dkm.data_ptr(), dq.data_ptr(), s.data_ptr(), B, H, G, nb, nmb, D, 64, L,
+                                               1 / math.sqrt(D), int(reference), stream()))
+        torch.cuda.synchronize()
+    finally:
+        lib.akv_set_tuning(b"k_tiles", 0)
+    got = s.cpu().numpy().view(np.uint16).reshape(B, Hq, -1)[..., :L]
+    assert np.array_equal(got, want.view(np.uint16).reshape(B, Hq, -1)[..., :L])
+
+
+@pytest.mark.parametrize("B,H,G,D,P,mode", [(1, 2, 1, 128, 64, "exact"), (3, 4, 1, 64, 100, "exact"), (2, 8, 4, 128, 700, "exact"),
+                                            (1, 4, 8, 128, 190, "exact"), (2, 3, 2, 256, 130, "exact"),
+                                            (1, 8, 1, 128, 1500, "order_free"), (2, 4, 4, 128, 600, "order_free"),
+                                            (40, 8, 1, 128, 300, "exact")])
+@pytest.mark.parametrize("append", [True, False])
+def test_overlapped_steps(akv_lib, B, H, G, D, P, mode, append):
+    """Steps that follow one another without a pause, one of them flushing a block, with and without overlapped launches."""
+    from alignedkv_b200.decode import DecodeLayer
+    g = torch.Generator(device="cuda").manual_seed(P)
+    T = 66 - P % 64 if append and P % 64 else 4
+    r = lambda n, h: torch.randn(n, B, 1, h, D, device="cuda", generator=g)  # noqa: E731
+    k = torch.randn(B, P, H, D, device="cuda", generator=g)
+    k[..., [3, 34]] *= 20
+    k, v, q, k1, v1 = k.half(), torch.randn(B, P, H, D, device="cuda", generator=g).half(), r(T, H * G).half(), r(T, H) * 3, r(T, H).half()
+    k1 = (k1 * torch.linspace(0.2, 9.0, T, device="cuda").view(T, 1, 1, 1, 1)).half()      # the maxima grow under way
+    outs = []
+    for pdl in (0, 1):
+        assert akv_lib.akv_set_tuning(b"pdl", pdl) == 0
+        try:
+            layer = DecodeLayer(B, -(-(P + T) // 64) * 64, H, D, "cuda:0", n_q_heads=H * G, v_mode=mode)
+            layer.prefill(k, v)
+            o = [layer.decode(q[t], k1[t], v1[t]) if append else layer.decode(q[t], append=False) for t in range(T)]
+            torch.cuda.synchronize()
+        finally:
+            akv_lib.akv_set_tuning(b"pdl", 1)
+        outs.append(torch.stack(o + [layer.k_exp_max.float().mean().half().expand_as(o[0])]))
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+    assert akv_lib.akv_device_error_flag() == 0
