@@ -33,13 +33,13 @@ bool v_compute_takes_probe(const uint8_t*, const uint8_t*, const uint8_t*, const
 int launch_v_compute_probe(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, const uint8_t*,
                            const uint8_t*, uint8_t*, int, int, int, int, int, int, int, int, cudaStream_t);
 int launch_v_compute_res(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, const uint8_t*,
-                         const uint8_t*, const uint8_t*, uint8_t*, int, int, int, int, int, int, int, int, cudaStream_t);
+                         const uint8_t*, const uint8_t*, uint8_t*, int, int, int, int, int, int, int, int, int, cudaStream_t);
 bool v_compute_adds_residual(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, int, int, int,
                              int, int, int, int);
 int launch_v_split(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, float*,
                    float*, int, int, int, int, int, int, int, int, cudaStream_t);
 int launch_v_split_probe(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, const uint8_t*,
-                         const uint8_t*, uint8_t*, float*, float*, int*, int, int, int, int, int, int, int, int,
+                         const uint8_t*, uint8_t*, float*, float*, int*, int, int, int, int, int, int, int, int, int,
                          cudaStream_t);
 bool v_split_takes_probe(int, int, int);
 long long v_split_scratch_bytes(int, int, int, int);
@@ -1121,13 +1121,14 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
             if ((rc = cuda_status(cudaGetLastError(), "decode_step threshold launch")) != AKV_OK) return rc;
         }
         if (ev) cudaEventRecord(ev[2], st);
+        // (the kernel in front, of the row softmax or the probe, is a pdl_turn one: P.V requests its first stages beside it)
         if (order_free)
             // the chunk partials stay in the workspace: the tail kernel adds them up (one launch less)
             rc = launch_v_split_probe(static_cast<const uint8_t*>(v_first_8), static_cast<const uint8_t*>(v_mid_4),
                                       static_cast<const uint8_t*>(v_last_4), reinterpret_cast<const uint8_t*>(sc.s),
                                       sc.amin, v_takes_probe ? (const uint8_t*)sc.test_o : nullptr,
                                       static_cast<const uint8_t*>(v_exp_max), nullptr, nullptr, sc.partial, &v_chunks, B,
-                                      H, G, max_seq_len, D, R, qn, reference, st);
+                                      H, G, max_seq_len, D, R, qn, reference, v_takes_probe, st);
         else
             rc = launch_v_compute_res(static_cast<const uint8_t*>(v_first_8), static_cast<const uint8_t*>(v_mid_4),
                                       static_cast<const uint8_t*>(v_last_4), reinterpret_cast<const uint8_t*>(sc.s),
@@ -1135,7 +1136,7 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
                                       static_cast<const uint8_t*>(v_exp_max),
                                       fuse_tail ? reinterpret_cast<const uint8_t*>(sc.o_main) : nullptr,
                                       reinterpret_cast<uint8_t*>(need_tail ? (void*)sc.o_main : out), B, H, G,
-                                      max_seq_len, D, R, qn, reference, st);
+                                      max_seq_len, D, R, qn, reference, v_takes_probe, st);
         if (ev) cudaEventRecord(ev[3], st);
         if (rc != AKV_OK) return rc;
     } else if (order_free) {

@@ -14,7 +14,7 @@ bool v_compute_takes_probe(const uint8_t*, const uint8_t*, const uint8_t*, const
 bool v_compute_adds_residual(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, int, int, int,
                              int, int, int, int);
 int launch_v_compute_res(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, const uint8_t*,
-                         const uint8_t*, const uint8_t*, uint8_t*, int, int, int, int, int, int, int, int, cudaStream_t);
+                         const uint8_t*, const uint8_t*, uint8_t*, int, int, int, int, int, int, int, int, int, cudaStream_t);
 
 namespace {
 
@@ -71,7 +71,7 @@ operator_probe_kernel(const uint16_t* __restrict__ s, const uint8_t* __restrict_
     __shared__ __align__(16) uint32_t key[NW][TOPK];
     __shared__ __align__(16) uint8_t rows[TOPK][256];
     __shared__ float part[4][256];
-    pdl_enter();
+    pdl_turn();
     const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint16_t* row = s + (size_t)bh * s_row;
@@ -231,7 +231,7 @@ int akv_v_output(const void* v_first_8, const void* v_mid_4, const void* v_last_
         if ((rc = cuda_status(cudaGetLastError(), "v_output threshold launch")) != AKV_OK) return rc;
     }
     rc = launch_v_compute_res(f8, m4, l4, sp, amin, takes_probe ? test_o : nullptr, ve, adds ? res : nullptr, o, B, H, 1,
-                              max_seq_len, D, s_last_dim, n, reference, st);
+                              max_seq_len, D, s_last_dim, n, reference, takes_probe, st);
     if (rc != AKV_OK || rest_len == 0 || adds) return rc;
     launch_chained(operator_add_kernel, dim3((rows * D + 255) / 256), dim3(256), 0, st, reinterpret_cast<uint16_t*>(o),
                    reinterpret_cast<const uint16_t*>(res), rows * D);

@@ -62,6 +62,9 @@ struct VParams {
     // chain kernel: res != nullptr adds the residual tokens' part of the output, [B, Hq, D] fp16 computed by the
     // softmax kernel: out = half(o + res) (extension/v_cache_file.py:189), which saves the tail launch
     const uint16_t* res;
+    // chain kernel: the kernel launched before is a pdl_turn one that writes no planes: their first stages are requested before
+    // it has completed
+    int early;
 };
 
 // ---- device error flag and shared-memory barriers (mbarrier) with bounded waits
@@ -223,7 +226,8 @@ __global__ void __launch_bounds__(UPC * (2 * NH / GH + vch::helpers(UPC, NH)) * 
         }
         sts32(pool + CONST_ROW + lane * 4, 0x80808080u);
     }
-    pdl_enter();
+    pdl_trigger();
+    if (!p.early) pdl_wait();
     __syncthreads();
     // units are dealt out a grid apart, so that every SM gets its share
     const int first_unit = uc * gridDim.x + blockIdx.x, stride = UPC * gridDim.x;
@@ -258,6 +262,7 @@ __global__ void __launch_bounds__(UPC * (2 * NH / GH + vch::helpers(UPC, NH)) * 
         // the first ring's high bytes depend on nothing but the planes: under way before the thresholds are known
         const int early = min(nf, nst);
         if (nunits > 0 && wi + HW * lane < early) copy_high(plane_row(first_unit), wi + HW * lane, wi + HW * lane);
+        if (p.early) pdl_wait();
         // the unit's thresholds; probabilities of this lane's two tokens of its next stage
         uint32_t A[NH], nxt[NH];
         auto load_s = [&](int unit, int i) {       // (rows are padded to a multiple of 8 values)
@@ -487,6 +492,7 @@ __global__ void __launch_bounds__(UPC * (2 * NH / GH + vch::helpers(UPC, NH)) * 
             acc[g] = v_fma(k, v_dup(u4w(r.s[g], u >> 1), u & 1), acc[g]);
         }
     };
+    if (p.early) pdl_wait();
     bool alive = true;
     int slot = 0;
     uint32_t parity = 0;

@@ -536,11 +536,13 @@ bool v_compute_takes_probe(const uint8_t* first8, const uint8_t* mid4, const uin
 // v_compute_takes_probe() holds): the threshold bytes are computed in the kernel from the probe result and the
 // exponent maxima v_exp and written to amin_out; otherwise they are read from amin.
 // res != nullptr (only when v_compute_adds_residual() holds): the kernel adds res [B, Hq, D] (fp16) to its result.
+// early: the kernel launched before is a pdl_turn one that writes no planes.
 int launch_v_compute_res(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* s,
                          uint8_t* amin, const uint8_t* test_o, const uint8_t* v_exp, const uint8_t* res, uint8_t* o,
-                         int bsz, int H, int group, int max_seq_len, int D, int s_last_dim, int n, int reference,
+                         int bsz, int H, int group, int max_seq_len, int D, int s_last_dim, int n, int reference, int early,
                          cudaStream_t st) {
     VParams p;
+    p.early = early;
     p.res = reinterpret_cast<const uint16_t*>(res);
     p.first8 = first8; p.mid4 = mid4; p.last4 = last4;
     p.s = reinterpret_cast<const uint16_t*>(s);
@@ -575,7 +577,7 @@ int launch_v_compute_probe(const uint8_t* first8, const uint8_t* mid4, const uin
                            uint8_t* amin, const uint8_t* test_o, const uint8_t* v_exp, uint8_t* o, int bsz, int H,
                            int group, int max_seq_len, int D, int s_last_dim, int n, int reference, cudaStream_t st) {
     return launch_v_compute_res(first8, mid4, last4, s, amin, test_o, v_exp, nullptr, o, bsz, H, group, max_seq_len, D,
-                                s_last_dim, n, reference, st);
+                                s_last_dim, n, reference, 0, st);
 }
 
 // true when launch_v_compute_res runs the chain kernel, which can add the residual tokens' part to its result
@@ -599,7 +601,7 @@ template <int KMAX>
 __global__ void __launch_bounds__(128)
 v_probe_kernel(const uint8_t* __restrict__ first8, const uint16_t* __restrict__ s_val,
                const int32_t* __restrict__ s_idx, uint16_t* __restrict__ out, int max_seq_len, int D, int K, int G) {
-    pdl_enter();
+    pdl_turn();
     const long long bh = blockIdx.x;                                    // (batch, query head)
     const uint8_t* F = first8 + (size_t)(bh / G) * max_seq_len * D;     // planes of its KV head
     for (int c = threadIdx.x; c < (D >> 1); c += blockDim.x) {
@@ -642,8 +644,9 @@ int launch_v_probe(const uint8_t* first8, const uint8_t* s_val, const uint8_t* s
 // Split pass of the order-free P.V in its streaming form (akv_v_stream.cuh), for akv_v_split.cu.
 int launch_v_split_stream(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* s,
                           uint8_t* amin, const uint8_t* test_o, const uint8_t* v_exp, int H, float* partial, int BH,
-                          int max_seq_len, int s_last_dim, int n, int chunk_tokens, int chunks, cudaStream_t st) {
+                          int max_seq_len, int s_last_dim, int n, int chunk_tokens, int chunks, int early, cudaStream_t st) {
     VStreamParams p;
+    p.early = early;
     p.first8 = first8; p.mid4 = mid4; p.last4 = last4;
     p.s = reinterpret_cast<const uint16_t*>(s);
     p.amin = amin; p.partial = partial;

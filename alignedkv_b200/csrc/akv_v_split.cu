@@ -197,7 +197,7 @@ static void stream_plan(int BH, int n, int* chunk_tokens, int* chunks) {
     *chunks = n > 0 ? (n + ct - 1) / ct : 1;
 }
 int launch_v_split_stream(const uint8_t*, const uint8_t*, const uint8_t*, const uint8_t*, uint8_t*, const uint8_t*,
-                          const uint8_t*, int, float*, int, int, int, int, int, int, cudaStream_t);
+                          const uint8_t*, int, float*, int, int, int, int, int, int, int, cudaStream_t);
 
 // true when launch_v_split_probe runs the streaming form, which can compute the threshold bytes itself
 bool v_split_takes_probe(int group, int reference, int n) {
@@ -215,10 +215,11 @@ long long v_split_scratch_bytes(int bsz, int H, int group, int n) {
 // probe result and the exponent maxima v_exp and written to amin; otherwise they are read from amin.
 // o16 == o32 == nullptr: the chunk partials are left in `scratch` for the caller to add up, in chunk order
 // (*chunks_out of them per (batch, query head), D floats each).
+// early: the kernel launched before is a pdl_turn one that writes no planes (streaming form).
 int launch_v_split_probe(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* s,
                          uint8_t* amin, const uint8_t* test_o, const uint8_t* v_exp, uint8_t* o16, float* o32,
                          float* scratch, int* chunks_out, int bsz, int H, int group, int max_seq_len, int D,
-                         int s_last_dim, int n, int reference, cudaStream_t st) {
+                         int s_last_dim, int n, int reference, int early, cudaStream_t st) {
     AKV_REQUIRE(D == 128, AKV_ERR_SHAPE, "v_cache_compute (order-free): head_dim %d is not supported (128 only)", D);
     AKV_REQUIRE(group == 1 || group == 2 || group == 4 || group == 8, AKV_ERR_SHAPE,
                 "v_cache_compute (order-free): group size %d is not supported (1, 2, 4, 8)", group);
@@ -239,7 +240,7 @@ int launch_v_split_probe(const uint8_t* first8, const uint8_t* mid4, const uint8
         stream_plan(bsz * H, n, &p.chunk_tokens, &p.chunks);
         if (chunks_out) *chunks_out = p.chunks;
         rc = launch_v_split_stream(first8, mid4, last4, s, amin, test_o, v_exp, H, scratch, bsz * H, max_seq_len,
-                                   s_last_dim, n, p.chunk_tokens, p.chunks, st);
+                                   s_last_dim, n, p.chunk_tokens, p.chunks, early, st);
         if (rc != AKV_OK || !combine) return rc;
         count_launch();   // the combine
         v_combine_kernel<<<bsz * H * group, 128, 0, st>>>(scratch, reinterpret_cast<__half*>(o16), o32, p.chunks, D);
@@ -263,7 +264,7 @@ int launch_v_split(const uint8_t* first8, const uint8_t* mid4, const uint8_t* la
                    const uint8_t* amin, uint8_t* o16, float* o32, float* scratch, int bsz, int H, int group,
                    int max_seq_len, int D, int s_last_dim, int n, int reference, cudaStream_t st) {
     return launch_v_split_probe(first8, mid4, last4, s, const_cast<uint8_t*>(amin), nullptr, nullptr, o16, o32, scratch,
-                                nullptr, bsz, H, group, max_seq_len, D, s_last_dim, n, reference, st);
+                                nullptr, bsz, H, group, max_seq_len, D, s_last_dim, n, reference, 0, st);
 }
 
 // ------------------------------------------------------------------ log-sum-exp merge of per-rank partial results

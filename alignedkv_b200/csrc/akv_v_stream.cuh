@@ -39,6 +39,7 @@ struct VStreamParams {
     int H;
     float* partial;         // [B*H, chunks, D]
     int max_seq_len, s_last_dim, n, chunk_tokens, chunks, nf;
+    int early;              // the kernel launched before is a pdl_turn one that writes no planes: they are read before it has completed
 };
 
 namespace vst {
@@ -91,12 +92,14 @@ __global__ void __launch_bounds__(160) v_stream_kernel(const VStreamParams p) {
 #pragma unroll
     for (int k = 0; k < 16; ++k) acc[k] = 0.f;
 
-    pdl_enter();
+    pdl_trigger();
+    if (!p.early) pdl_wait();
     {   // the launch must have given the ring its room (uniform over the CTA: all threads leave together)
         uint32_t dyn;
         asm volatile("mov.u32 %0, %%dynamic_smem_size;\n" : "=r"(dyn));
         if (nf < CONSUMERS || nf % CONSUMERS != 0 || dyn < (uint32_t)smem_bytes(nf) || (ring & 127u) != 0 || c1 <= c0) {
             if (threadIdx.x == 0) atomicOr(&g_v_wait_gave_up, 2u);
+            if (p.early) pdl_wait();
             return;
         }
     }
@@ -129,8 +132,10 @@ __global__ void __launch_bounds__(160) v_stream_kernel(const VStreamParams p) {
             if (++slot == nf) { slot = 0; if (i >= nf) parity ^= 1u; }
         }
         if (!alive) v_sleep_ms();
+        if (p.early) pdl_wait();
     } else {
         // ------------------------------------------------------------------ consumer warps
+        if (p.early) pdl_wait();
         const uint8_t* M = p.mid4 + (size_t)bh * p.max_seq_len * HD + cg * 8;
         const uint8_t* L = p.last4 + (size_t)bh * p.max_seq_len * HD + cg * 8;
         const uint16_t* s_row = p.s + (size_t)bh * p.s_last_dim;
