@@ -410,6 +410,111 @@ softmax_row_kernel(uint16_t* __restrict__ s, const __half* __restrict__ q, const
     }
 }
 
+// A whole step of a cache without a quantized block: at most 63 tokens, all of them in the residual buffers.  One CTA per row;
+// the new token is taken from k_new / v_new, and stored, with the exponent maxima, by the first head of its group.  Sums in the
+// order of the kernels it stands for (append, softmax, tail): bit-identical.  Latency only: 64 dot products, one exponential per
+// token, 64 rows of values.  32 rows of 29 tokens, 3 tokens and a rewind: 60 us against 73 with three launches per token, the
+// host's share included.
+__global__ void __launch_bounds__(256)
+small_step_kernel(uint32_t* __restrict__ restk, uint32_t* __restrict__ restv, uint16_t* __restrict__ k_exp,
+                  uint16_t* __restrict__ v_exp, const __half* __restrict__ q, const __half* __restrict__ k_new,
+                  const __half* __restrict__ v_new, __half* __restrict__ out, float* __restrict__ packed,
+                  const __half* __restrict__ mask, long long mask_stride, int H, int G, int D, int rest_len, int append,
+                  int round_packed, float sqrt_d, uint16_t* __restrict__ p) {
+    __shared__ __half sc[BLK];
+    __shared__ float part[4][256];
+    pdl_enter();
+    const int bhq = blockIdx.x, bh = bhq / G, b = bh / H, h = bh - b * H;
+    const int tid = threadIdx.x, lane = tid & 31, hd = D >> 1;
+    const int len = rest_len + append;
+    const size_t vs = (size_t)H * D, row0 = ((size_t)b * BLK * H + h) * D;      // token stride, first token's row
+    {
+        const int r = tid >> 2;
+        const __half* kr = r < rest_len ? reinterpret_cast<const __half*>(restk) + row0 + (size_t)r * vs
+                         : r < len ? k_new + (size_t)bh * D : nullptr;
+        __half v = residual_score_of(q + (size_t)bhq * D, kr, D, sqrt_d);
+        if (r >= len) v = __ushort_as_half((unsigned short)0xFC00u);
+        else if (mask) v = __hadd(v, mask[(size_t)b * mask_stride + r]);
+        if ((tid & 3) == 0) sc[r] = v;
+    }
+    if (append && bhq % G == 0) {
+        auto exps = [](uint32_t w) { return ((w >> 10) & 0x1Fu) | (((w >> 26) & 0x1Fu) << 8); };
+        for (int c = tid; c < hd; c += 256) {
+            const size_t at = (size_t)bh * hd + c, dst = (row0 + (size_t)rest_len * vs) / 2 + c;
+            const uint32_t kw = reinterpret_cast<const uint32_t*>(k_new)[at], vw = reinterpret_cast<const uint32_t*>(v_new)[at];
+            restk[dst] = kw;
+            restv[dst] = vw;
+            k_exp[at] = (uint16_t)(__vmaxu4(k_exp[at], exps(kw)) & 0xFFFFu);
+            v_exp[at] = (uint16_t)(__vmaxu4(v_exp[at], exps(vw)) & 0xFFFFu);
+        }
+    }
+    __syncthreads();
+    // softmax of tokens lane and lane + 32, by every warp
+    const float f0 = __half2float(sc[lane]), f1 = __half2float(sc[lane + 32]);
+    float m = fmaxf(f0, f1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+    const float x0 = lane < len ? expf(f0 - m) : 0.f, x1 = lane + 32 < len ? expf(f1 - m) : 0.f;
+    float s0 = x0, s1 = x1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s0 += __shfl_xor_sync(0xFFFFFFFFu, s0, o);
+        s1 += __shfl_xor_sync(0xFFFFFFFFu, s1, o);
+    }
+    const float sum = s0 + s1, inv = 1.f / sum;
+    auto prob = [&](float x) {                                   // (as in softmax_row_kernel)
+        const float y = x * inv;
+        return __half2float(__float2half_rn(fmaf(fmaf(-y, sum, x), inv, y)));
+    };
+    const float p0 = prob(x0), p1 = prob(x1);
+    if (tid < 32) {                                              // (the row of probabilities, as a longer cache's step leaves it)
+        p[(size_t)bhq * BLK + lane] = lane < len ? __half_as_ushort(__float2half_rn(p0)) : (uint16_t)0;
+        p[(size_t)bhq * BLK + lane + 32] = lane + 32 < len ? __half_as_ushort(__float2half_rn(p1)) : (uint16_t)0;
+    }
+    // item = (channel pair, quarter g of the tokens: r = g, g + 4, ...), the quarters added in order
+    for (int i0 = 0; i0 < 4 * hd; i0 += 256) {                   // (whole warps: D is a multiple of 64)
+        const int i = i0 + tid;
+        const bool on = i < 4 * hd;
+        const int g = i / hd, c = i - g * hd;
+        float a0 = 0.f, a1 = 0.f;
+        uint32_t w[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int r = g + 4 * j;
+            w[j] = 0;
+            if (on && r < len)
+                w[j] = r < rest_len ? restv[(row0 + (size_t)r * vs) / 2 + c]
+                                    : reinterpret_cast<const uint32_t*>(v_new)[(size_t)bh * hd + c];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            // (g is the same in a warp, and so is r; no weight beyond the last token, also where the sum is not a number)
+            const int r = (g + 4 * j) & 63;
+            const float pv = __shfl_sync(0xFFFFFFFFu, r < 32 ? p0 : p1, r & 31);
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+            if (r < len) {
+                a0 = fmaf(pv, f.x, a0);
+                a1 = fmaf(pv, f.y, a1);
+            }
+        }
+        if (on) {
+            part[g][2 * c] = a0;
+            part[g][2 * c + 1] = a1;
+        }
+    }
+    __syncthreads();
+    for (int d = tid; d < D; d += 256) {
+        const float acc = ((part[0][d] + part[1][d]) + part[2][d]) + part[3][d];
+        const float v = round_packed ? 0.f + __half2float(__float2half_rn(acc)) : 0.f + acc;
+        if (out) out[(size_t)bhq * D + d] = __float2half_rn(v);
+        if (packed) packed[(size_t)bhq * (D + 2) + 2 + d] = v;
+    }
+    if (packed && tid == 0) {
+        packed[(size_t)bhq * (D + 2)] = m;
+        packed[(size_t)bhq * (D + 2) + 1] = sum;
+    }
+}
+
 // Launch of one form.  The shared-memory limit is an attribute of the kernel on a device, seen by the launches of every host
 // thread: it is set once, to what the device has beside the static part, and not to one call's size.
 template <int NT, int VPT, int MINB>
@@ -987,6 +1092,14 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
 
     int rest = rest_len + (append ? 1 : 0), qn = rest_start;
     const bool flush = rest == BLK;
+    if (qn == 0 && !flush && rest > 0 && D <= 256 && xp.R == 0) {
+        launch_chained(small_step_kernel, dim3(B * H * G), dim3(256), 0, st, static_cast<uint32_t*>(restk),
+                       static_cast<uint32_t*>(restv), static_cast<uint16_t*>(k_exp_max), static_cast<uint16_t*>(v_exp_max),
+                       static_cast<const __half*>(q), static_cast<const __half*>(k_new), static_cast<const __half*>(v_new),
+                       static_cast<__half*>(out), static_cast<float*>(packed_out), mk, mask_stride, H, G, D, rest_len,
+                       append ? 1 : 0, order_free ? 0 : 1, sqrtf((float)D), sc.s);
+        return cuda_status(cudaGetLastError(), "decode_step launch");
+    }
     // append and (when the residual buffer fills up) the flush of the block to the planes
     // (k_cache_file.py:102-118, v_cache_file.py:103-116): one launch when the block tile fits in default shared memory
     const bool fused_flush = flush && D <= 256 && aligned16(k_first_8) && aligned16(k_mid_4) && aligned16(k_last_4) &&

@@ -8,16 +8,14 @@ namespace akv {
 constexpr int TOPK = 32;     // residue classes of the magnitude probe (extension/v_cache_file.py:16)
 constexpr int BLK = 64;      // tokens per K block (extension/k_cache_file.py:5-6)
 
-// Scores of the residual tokens of one (batch, query head) row, by 256 threads: thread = (token tid / 4,
-// quarter tid % 4 of the channels in 16-byte pieces), all loads of a row in flight at once, fp32 dot product rounded to
-// fp16, then divided by sqrt(D) and rounded again, which is what `matmul(q, restk^T) / sqrt(D)` on fp16 tensors
-// produces (k_cache_file.py:156-157).  Returned by the first thread of each token's four, 0 <= tid / 4 < rest < 64.
-__device__ __forceinline__ __half residual_score(const __half* __restrict__ qr, const __half* __restrict__ restk, int b, int h,
-                                                 int H, int D, int rest, float sqrt_d, bool wanted) {
-    const int r = threadIdx.x >> 2, c = threadIdx.x & 3;
+// Score of one residual token of a (batch, query head) row by four threads: thread % 4 = quarter of the channels in 16-byte
+// pieces, all loads of a row in flight at once, fp32 dot product rounded to fp16, then divided by sqrt(D) and rounded again,
+// which is what `matmul(q, restk^T) / sqrt(D)` on fp16 tensors produces (k_cache_file.py:156-157).  kr: the token's key, or null.
+// All four threads return it.
+__device__ __forceinline__ __half residual_score_of(const __half* __restrict__ qr, const __half* __restrict__ kr, int D, float sqrt_d) {
+    const int c = threadIdx.x & 3;
     float acc = 0.f;
-    if (wanted && r < rest) {
-        const __half* kr = restk + (((size_t)b * BLK + r) * H + h) * D;
+    if (kr) {
 #pragma unroll 4
         for (int d = c * 8; d < D; d += 32) {
             const uint4 kv = *reinterpret_cast<const uint4*>(kr + d), qv = *reinterpret_cast<const uint4*>(qr + d);
@@ -34,6 +32,12 @@ __device__ __forceinline__ __half residual_score(const __half* __restrict__ qr, 
     acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
     acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
     return __float2half_rn(__half2float(__float2half_rn(acc)) / sqrt_d);
+}
+// ... of residual token tid / 4 of a row, by 256 threads, 0 <= tid / 4 < rest <= 64
+__device__ __forceinline__ __half residual_score(const __half* __restrict__ qr, const __half* __restrict__ restk, int b, int h,
+                                                 int H, int D, int rest, float sqrt_d, bool wanted) {
+    const int r = threadIdx.x >> 2;
+    return residual_score_of(qr, wanted && r < rest ? restk + (((size_t)b * BLK + r) * H + h) * D : nullptr, D, sqrt_d);
 }
 // The same for a CTA of 256 threads, written into the row; only tokens with t_lo <= qn + r < t_hi (a row split across CTAs).
 __device__ __forceinline__ void residual_scores(uint16_t* __restrict__ row, const __half* __restrict__ qr,
