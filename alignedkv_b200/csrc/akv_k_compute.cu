@@ -31,6 +31,7 @@
 // 16384 tokens 54.4 -> 53.3.  Bulk copies of the pieces (high bytes and mid plane, 1 KB and 512 bytes) were built again for this
 // form and are slower: 80.3, 54.0, and 8 KV heads x 4, batch 64 x 8192 tokens 532 against 512.
 #include <atomic>
+#include <type_traits>
 
 #include "akv_common.cuh"
 
@@ -221,7 +222,10 @@ __device__ __noinline__ void kc_load_tables(const KParams& p, long long bh, uint
     __syncwarp();
 }
 
-template <int KCH, int STAGES, int G, int TILES>
+// DC: the head size when it is known, 0 for any: the copies' addresses are then immediate offsets from two pointers, and a unit whose
+// tiles all exist checks none of them.  A row of four heads took 68 instructions where the arithmetic needs 46: 8 KV heads x 4, batch
+// 64 x 8192 tokens 505 -> 479 us per step, 8 x 32 x 4096 78.1 -> 77.9.
+template <int KCH, int STAGES, int G, int TILES, int DC>
 __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(const __grid_constant__ KParams p) {
     using namespace kc;
     constexpr int F_TILE = f_tile(KCH, TILES), N_TILE = n_tile(KCH, TILES);
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_trigger();
     if (!p.k_exp) pdl_wait();
+    const int D = DC ? DC : p.D;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wpc = blockDim.x >> 5;
     const int w = blockIdx.x * wpc + warp;
@@ -243,10 +248,10 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         return;
     }
     const int u_end = (u_begin + p.upw < p.units) ? u_begin + p.upw : p.units;
-    const int nch = p.D / KCH;
+    const int nch = D / KCH;
     const int total = (u_end - u_begin) * nch;
-    const size_t tile_f = (size_t)p.D * 64, tile_n = (size_t)p.D * 32;
-    const int META = meta_bytes(p.D, G), HMETA = head_meta(p.D, G);
+    const size_t tile_f = (size_t)D * 64, tile_n = (size_t)D * 32;
+    const int META = meta_bytes(D, G), HMETA = head_meta(D, G);
 
     uint8_t* ring = smem + (size_t)warp * (STAGES * STAGE + META);
     uint8_t* meta0 = ring + STAGES * STAGE;
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         k.g = u - k.bh * p.ngroups;
         k.c = 0;
         k.slot = 0;
-        k.row = ((size_t)k.bh * p.nmb + (size_t)k.g * TILES) * p.D;
+        k.row = ((size_t)k.bh * p.nmb + (size_t)k.g * TILES) * D;
         return k;
     };
     auto advance = [&](KCursor& k) {   // next stage; returns true when a new (batch, KV head) starts
@@ -269,13 +274,13 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         k.c = 0;
         ++k.u;
         if (++k.g < p.ngroups) {
-            k.row += (size_t)(TILES - 1) * p.D;          // next tiles of the same (batch, KV head)
+            k.row += (size_t)(TILES - 1) * D;          // next tiles of the same (batch, KV head)
             return false;
         }
         k.g = 0;
         ++k.bh;
         k.slot ^= 1;
-        k.row = (size_t)k.bh * p.nmb * p.D;
+        k.row = (size_t)k.bh * p.nmb * D;
         return true;
     };
     auto load_masks = [&](long long bh, int slot) {
@@ -301,24 +306,30 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
         const uint32_t st = ring_a + (uint32_t)pstage * STAGE;
         const int ptiles = p.nb - pk.g * TILES;
         const uint8_t* pf = p.first8 + pk.row * 64 + lane * 16;
-#pragma unroll
-        for (int it = 0; it < TILES * F_IT; ++it) {      // high-byte plane: KCH*64 contiguous bytes per tile
-            const int t = it / F_IT, v = it % F_IT;
-            if (t < ptiles) cp_async16(st + t * F_TILE + v * 512 + lane * 16, pf + t * tile_f + v * 512);
-        }
         const size_t pn = (pk.row + nrow) * 32 + nhalf;
-        const uint32_t nd = st + F_BYTES + nrow * 32 + nhalf;
+        const uint8_t *pm = p.mid4 + pn, *pl = p.last4 + pn;
+        const uint32_t fd = st + lane * 16, nd = st + F_BYTES + nrow * 32 + nhalf;
+        auto copies = [&](auto whole) {                      // whole: all tiles of the unit exist
+            constexpr bool WHOLE = decltype(whole)::value;
 #pragma unroll
-        for (int it = 0; it < N_IT; ++it) {              // nibble planes: only the rows some head reads
-            const int t = it * TILES_PER_IT + ntsub;
-            if (t < ptiles && t < TILES) {
-                const uint32_t dm = nd + t * N_TILE, dl = dm + N_BYTES;
-                if (need_m) cp_async16(dm, p.mid4 + pn + t * tile_n);
-                else if (G == 1) st_shared_v4(dm, 0x88888888u);              // plane not read: low byte becomes 0x80
-                if (need_l) cp_async16(dl, p.last4 + pn + t * tile_n);
-                else if (G == 1) st_shared_v4(dl, need_m ? 0x88888888u : 0u);  // low plane not read: low nibble becomes 8
+            for (int it = 0; it < TILES * F_IT; ++it) {      // high-byte plane: KCH*64 contiguous bytes per tile
+                const int t = it / F_IT, v = it % F_IT;
+                if (WHOLE || t < ptiles) cp_async16(fd + t * F_TILE + v * 512, pf + t * tile_f + v * 512);
             }
-        }
+#pragma unroll
+            for (int it = 0; it < N_IT; ++it) {              // nibble planes: only the rows some head reads
+                const int t = it * TILES_PER_IT + ntsub;
+                if ((WHOLE && TILES_PER_IT == 1) || (t < ptiles && t < TILES)) {
+                    const uint32_t dm = nd + t * N_TILE, dl = dm + N_BYTES;
+                    if (need_m) cp_async16(dm, pm + t * tile_n);
+                    else if (G == 1) st_shared_v4(dm, 0x88888888u);              // plane not read: low byte becomes 0x80
+                    if (need_l) cp_async16(dl, pl + t * tile_n);
+                    else if (G == 1) st_shared_v4(dl, need_m ? 0x88888888u : 0u);  // low plane not read: low nibble becomes 8
+                }
+            }
+        };
+        if (ptiles >= TILES) copies(std::true_type{});
+        else copies(std::false_type{});
         pstage = (pstage + 1 == STAGES) ? 0 : pstage + 1;
         if (advance(pk) && pk.u < u_end) load_masks(pk.bh, pk.slot);
     };
@@ -375,8 +386,8 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
                 for (int g = 0; g < G; ++g) {
                     const uint8_t* hg = hm0 + (size_t)g * HMETA + (size_t)(ch0 + r4 * 4) * 4;
                     mk[g] = *reinterpret_cast<const uint4*>(hg);
-                    cn[g] = *reinterpret_cast<const uint4*>(hg + (size_t)p.D * 4);
-                    qv[g] = *reinterpret_cast<const uint2*>(hm0 + (size_t)g * HMETA + (size_t)p.D * 8 + (size_t)(ch0 + r4 * 4) * 2);
+                    cn[g] = *reinterpret_cast<const uint4*>(hg + (size_t)D * 4);
+                    qv[g] = *reinterpret_cast<const uint2*>(hm0 + (size_t)g * HMETA + (size_t)D * 8 + (size_t)(ch0 + r4 * 4) * 2);
                 }
 #pragma unroll
                 for (int rr = 0; rr < 4; ++rr) {
@@ -468,7 +479,7 @@ bool k_compute_aligns(const uint8_t* first8, const uint8_t* mid4, const uint8_t*
 }
 
 // Launch of one form: warps per CTA and units per warp, one CTA per SM.
-template <int KCH, int STAGES, int G, int TILES>
+template <int KCH, int STAGES, int G, int TILES, int DC = 0>
 static int k_launch(KParams p, cudaStream_t st) {
     using namespace kc;
     p.ngroups = (p.nb + TILES - 1) / TILES;
@@ -501,7 +512,7 @@ static int k_launch(KParams p, cudaStream_t st) {
     // the opt-in shared-memory size is a per-device attribute of the kernel: set once per device - to the device's maximum, so
     // that every launch shape fits - not on every launch (a racing thread at worst sets it twice)
     static std::atomic<bool> configured[64];
-    const auto kern = k_compute_kernel<KCH, STAGES, G, TILES>;
+    const auto kern = k_compute_kernel<KCH, STAGES, G, TILES, DC>;
     int dev = -1;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
@@ -550,8 +561,9 @@ int launch_k_compute_align(const uint8_t* first8, const uint8_t* mid4, const uin
     // 8 KV heads x 4, batch 1, 700 tokens (80 tiles) 31.8 / 27.0, 4096 tokens (512) 47.6 / 42.8; 4 x 8, 8000 tokens (500)
     // 78.1 / 69.9; 2000 tiles 67.2 / 75.6.  One head: 384 tiles 25.1 / 24.9, 800 26.7 / 25.9, 1472 26.8 / 29.2.
     const bool single = tuning().k_tiles ? tuning().k_tiles == 1 : (long long)p.BH * nb <= 4ll * sm_count();
-    if (single && D >= 128 && group == 4) return k_launch<16, 8, 4, 1>(p, st);
-    if (single && D >= 128 && group == 8) return k_launch<16, 8, 8, 1>(p, st);
+    const bool d128 = D == 128;
+    if (single && D >= 128 && group == 4) return d128 ? k_launch<16, 8, 4, 1, 128>(p, st) : k_launch<16, 8, 4, 1>(p, st);
+    if (single && D >= 128 && group == 8) return d128 ? k_launch<16, 8, 8, 1, 128>(p, st) : k_launch<16, 8, 8, 1>(p, st);
     // (channels per stage, ring depth): the instantiated combinations; anything else falls back to the default of its group
     if (group == 1) {
         const int kch = tuning().k_kch;
@@ -565,15 +577,18 @@ int launch_k_compute_align(const uint8_t* first8, const uint8_t* mid4, const uin
             case 86: return k_launch<8, 6, 1, 4>(p, st);
             case 164: return k_launch<16, 4, 1, 4>(p, st);
             case 165: return k_launch<16, 5, 1, 4>(p, st);
-            case 163: return k_launch<16, 3, 1, 4>(p, st);
+            case 163: return d128 ? k_launch<16, 3, 1, 4, 128>(p, st) : k_launch<16, 3, 1, 4>(p, st);
             default:
                 set_error("k_cache_compute: no kernel for %d channels x %d stages", kch, stages);
                 return AKV_ERR_SHAPE;
         }
     }
-    if (group == 2) return k_launch<gqa_kch(2), gqa_stages(2), 2, 4>(p, st);
-    if (group == 4) return k_launch<gqa_kch(4), gqa_stages(4), 4, 4>(p, st);
-    return k_launch<gqa_kch(8), gqa_stages(8), 8, 4>(p, st);
+    if (group == 2) return d128 ? k_launch<gqa_kch(2), gqa_stages(2), 2, 4, 128>(p, st)
+                                : k_launch<gqa_kch(2), gqa_stages(2), 2, 4>(p, st);
+    if (group == 4) return d128 ? k_launch<gqa_kch(4), gqa_stages(4), 4, 4, 128>(p, st)
+                                : k_launch<gqa_kch(4), gqa_stages(4), 4, 4>(p, st);
+    return d128 ? k_launch<gqa_kch(8), gqa_stages(8), 8, 4, 128>(p, st)
+                : k_launch<gqa_kch(8), gqa_stages(8), 8, 4>(p, st);
 }
 
 int launch_k_compute(const uint8_t* first8, const uint8_t* mid4, const uint8_t* last4, const uint8_t* kq,
