@@ -7,8 +7,27 @@ from __future__ import annotations
 import ctypes
 import os
 
+import torch
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libalignedkv_b200.so")
+
+
+class Layer(ctypes.Structure):
+    """`akv_layer`: what stays the same from one decode step of a layer to the next."""
+    _fields_ = [(n, ctypes.c_void_p) for n in (
+        "k_first_8", "k_mid_4", "k_last_4", "v_first_8", "v_mid_4", "v_last_4", "k_exp_max", "v_exp_max", "restk", "restv",
+        "scratch")] + [("scratch_bytes", ctypes.c_longlong)] + [
+        (n, ctypes.c_int) for n in ("bsz", "n_kv_heads", "group", "head_dim", "max_seq_len")]
+
+
+def _raw_stream(device_index: int) -> int:
+    return torch.cuda.current_stream(device_index).cuda_stream
+
+
+#: Handle of torch's current stream on a device (without a Stream object where torch offers that).
+raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _raw_stream)
+
 
 # every symbol include/alignedkv_b200.h declares, with its ctypes signature
 _P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
@@ -33,6 +52,7 @@ SIGNATURES = {
     "akv_decode_step_ex": (_I, [_P] * 16 + [ctypes.c_longlong] + [_I] * 8 + [_P]),
     "akv_decode_scratch_bytes_ex": (ctypes.c_longlong, [_I] * 6),
     "akv_decode_step_masked": (_I, [_P] * 16 + [ctypes.c_longlong, _P, ctypes.c_longlong] + [_I] * 8 + [_P]),
+    "akv_decode_step_layer": (_I, [_P] * 7 + [ctypes.c_longlong] + [_I] * 3 + [_P]),
     "akv_shard_step": (_I, [_P] * 16 + [ctypes.c_longlong] + [_I] * 13 + [_P]),
     "akv_lse_merge": (_I, [_P] * 2 + [_I] * 3 + [_P]),
     "akv_exchange_bytes": (ctypes.c_longlong, [_I] * 3),

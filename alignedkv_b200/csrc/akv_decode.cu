@@ -1102,6 +1102,16 @@ int akv_decode_step_masked(void* k_first_8, void* k_mid_4, void* k_last_4, void*
                             group, head_dim, max_seq_len, rest_len, rest_start, flags, stream, XchgParams{});
 }
 
+int akv_decode_step_layer(const akv_layer* l, const void* q, const void* k_new, const void* v_new, void* out, void* packed_out,
+                          const void* mask, long long mask_stride, int rest_len, int rest_start, int flags, void* stream) {
+    set_error("");
+    AKV_REQUIRE(l, AKV_ERR_NULL, "decode_step: null pointer");
+    return decode_step_impl(l->k_first_8, l->k_mid_4, l->k_last_4, l->v_first_8, l->v_mid_4, l->v_last_4, l->k_exp_max,
+                            l->v_exp_max, l->restk, l->restv, q, k_new, v_new, out, packed_out, mask, mask_stride, l->scratch,
+                            l->scratch_bytes, l->bsz, l->n_kv_heads, l->group, l->head_dim, l->max_seq_len, rest_len, rest_start,
+                            flags, stream, XchgParams{});
+}
+
 int akv_decode_step_exchange(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8, void* v_mid_4,
                              void* v_last_4, void* k_exp_max, void* v_exp_max, void* restk, void* restv, const void* q,
                              const void* k_new, const void* v_new, void* merged_out, void* packed_out, void* scratch,

@@ -7,6 +7,7 @@ kernels behind `akv_decode_step`, so a step is a single library call.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 
@@ -18,6 +19,8 @@ from .extension.KV_cache_cpp_extention import cuda_module
 
 __all__ = ["DecodeLayer"]
 
+
+_nothing = contextlib.nullcontext()
 
 AKV_STEP_REFERENCE, AKV_STEP_ORDER_FREE, AKV_STEP_NO_APPEND, AKV_STEP_TRACK_MAXIMA = 1, 2, 4, 8
 
@@ -61,7 +64,9 @@ class DecodeLayer:
             raise ValueError("bad extents")
         self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         self._sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
-        self._static_ptrs = None
+        self._desc = None                    # `_lib.Layer`, made by the first step
+        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+        self._q_shape, self._kv_shape = (bsz, 1, self.Hq, head_dim), (bsz, 1, n_heads, head_dim)
         self.launches = 0
 
     @property
@@ -93,13 +98,13 @@ class DecodeLayer:
         if S > 0 and D % 32 == 0 and D <= 256:
             nbytes = self.lib.akv_prefill_scratch_bytes(B, H, D, S)
             ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-            with torch.cuda.device(self.device):
+            with _nothing if torch.cuda.current_device() == self._index else torch.cuda.device(self._index):
                 rc = self.lib.akv_prefill(
                     self.k_first_8.data_ptr(), self.k_mid_4.data_ptr(), self.k_last_4.data_ptr(),
                     self.v_first_8.data_ptr(), self.v_mid_4.data_ptr(), self.v_last_4.data_ptr(),
                     self.k_exp_max.data_ptr(), self.v_exp_max.data_ptr(), self.restk.data_ptr(), self.restv.data_ptr(),
                     k.data_ptr(), v.data_ptr(), ws.data_ptr(), nbytes, B, H, D, self.L, S,
-                    torch.cuda.current_stream(self.device).cuda_stream)
+                    _lib.raw_stream(self._index))
             _lib.check("prefill", rc)
         elif S > 0:
             # head sizes the fused kernel does not cover: the operator-by-operator route
@@ -114,6 +119,11 @@ class DecodeLayer:
         self.rest_len = S % column_block
         self.rest_start = full
         self.cache_len = S
+
+    @staticmethod
+    def _check_token(name: str, t: torch.Tensor | None, shape: tuple) -> None:
+        if t is None or t.shape != shape or t.dtype != torch.half or not t.is_cuda or not t.is_contiguous():
+            raise RuntimeError(f"{name}: expected a contiguous CUDA fp16 tensor of shape {shape}")
 
     # ------------------------------------------------------------------ one decode token
     def decode(self, q: torch.Tensor, k: torch.Tensor | None = None, v: torch.Tensor | None = None, *,
@@ -136,53 +146,51 @@ class DecodeLayer:
         if exchange is not None and (packed or mask is not None):
             raise RuntimeError("exchange: not together with packed or mask")
         packed = packed or exchange is not None
-        B, H, Hq, D = self.B, self.H, self.Hq, self.D
         mask_ptr, mask_stride = None, 0
         if mask is not None:
             need = self.cache_len + (1 if append else 0)
             if mask.dtype != torch.half or not mask.is_cuda or mask.dim() != 4 or mask.shape[1] != 1 or \
-                    mask.shape[2] != 1 or mask.shape[0] not in (1, B) or mask.shape[3] < need or mask.stride(3) != 1:
-                raise RuntimeError(f"mask: expected a CUDA fp16 tensor of shape [{B} or 1, 1, 1, >= {need}] with a "
+                    mask.shape[2] != 1 or mask.shape[0] not in (1, self.B) or mask.shape[3] < need or mask.stride(3) != 1:
+                raise RuntimeError(f"mask: expected a CUDA fp16 tensor of shape [{self.B} or 1, 1, 1, >= {need}] with a "
                                    "unit stride along the positions")
-            mask_ptr, mask_stride = mask.data_ptr(), (mask.stride(0) if mask.shape[0] == B else 0)
-        checks = [("q", q, Hq)] + ([("k", k, H), ("v", v, H)] if append else [])
-        for name, t, heads in checks:
-            if t is None or t.shape != (B, 1, heads, D) or t.dtype != torch.half or not t.is_cuda or \
-                    not t.is_contiguous():
-                raise RuntimeError(f"{name}: expected a contiguous CUDA fp16 tensor of shape {(B, 1, heads, D)}")
-        if append and self.cache_len + 1 > self.L:
-            raise RuntimeError(f"cache is full ({self.L} tokens)")
-        if out is not None and (packed or out.shape != (B, 1, Hq, D) or out.dtype != torch.half or not out.is_cuda or
+            mask_ptr, mask_stride = mask.data_ptr(), (mask.stride(0) if mask.shape[0] == self.B else 0)
+        self._check_token("q", q, self._q_shape)
+        if append:
+            self._check_token("k", k, self._kv_shape)
+            self._check_token("v", v, self._kv_shape)
+            if self.cache_len + 1 > self.L:
+                raise RuntimeError(f"cache is full ({self.L} tokens)")
+        if out is not None and (packed or out.shape != self._q_shape or out.dtype != torch.half or not out.is_cuda or
                                 not out.is_contiguous()):
-            raise RuntimeError(f"out: expected a contiguous CUDA fp16 tensor of shape {(B, 1, Hq, D)}")
-        if out is None and not packed:
-            out = torch.empty((B, 1, Hq, D), dtype=torch.half, device=self.device)
-        rec = torch.empty((B * Hq, D + 2), dtype=torch.float32, device=self.device) if packed else None
-        # (the planes, exponent maxima, residual buffers and the workspace never move: their addresses are taken once;
-        # the device is only switched when it is not the current one - both keep the host's share of a step small,
-        # which is what bounds a rank whose CPU is slow)
-        ptrs = self._static_ptrs
-        if ptrs is None:
-            ptrs = self._static_ptrs = tuple(t.data_ptr() for t in (
-                self.k_first_8, self.k_mid_4, self.k_last_4, self.v_first_8, self.v_mid_4, self.v_last_4,
-                self.k_exp_max, self.v_exp_max, self.restk, self.restv)) + (self.scratch.data_ptr(), self.scratch.numel())
-        args = ptrs[:10] + (
-            q.data_ptr(), k.data_ptr() if append else None, v.data_ptr() if append else None,
-            out.data_ptr() if out is not None else None, rec.data_ptr() if rec is not None else None,
-            mask_ptr, mask_stride, ptrs[10], ptrs[11], B, H, self.G, D, self.L, self.rest_len, self.rest_start,
-            self._flags(append), torch.cuda.current_stream(self.device).cuda_stream)
-        fn = self.lib.akv_decode_step_masked
-        if exchange is not None:
-            out = torch.empty((B, 1, Hq, D), dtype=torch.half, device=self.device)
-            fn = self.lib.akv_decode_step_exchange
-            args = args[:13] + (out.data_ptr(),) + args[14:15] + args[17:27] + (
-                exchange.bufs, exchange.rank, exchange.world, exchange.next_epoch(), exchange.timeout_ms, args[27])
-        if torch.cuda.current_device() == self.device.index:
-            rc = fn(*args)
-        else:
-            with torch.cuda.device(self.device):
-                rc = fn(*args)
-        _lib.check("decode_step", rc)
+            raise RuntimeError(f"out: expected a contiguous CUDA fp16 tensor of shape {self._q_shape}")
+        if out is None and (not packed or exchange is not None):
+            out = torch.empty(self._q_shape, dtype=torch.half, device=self.device)
+        rec = torch.empty((self.B * self.Hq, self.D + 2), dtype=torch.float32, device=self.device) if packed else None
+        # (the planes, exponent maxima, residual buffers and the workspace never move: their addresses are taken once, and a step
+        # gets one pointer to them; the device is only switched when it is not the current one - the host's share bounds a step
+        # of few short sequences)
+        if self._desc is None:
+            self._desc = _lib.Layer(*(t.data_ptr() for t in (
+                self.k_first_8, self.k_mid_4, self.k_last_4, self.v_first_8, self.v_mid_4, self.v_last_4, self.k_exp_max,
+                self.v_exp_max, self.restk, self.restv, self.scratch)), self.scratch.numel(), self.B, self.H, self.G, self.D,
+                self.L)
+        with _nothing if torch.cuda.current_device() == self._index else torch.cuda.device(self._index):
+            stream = _lib.raw_stream(self._index)
+            k_ptr, v_ptr = (k.data_ptr(), v.data_ptr()) if append else (None, None)
+            if exchange is None:
+                rc = self.lib.akv_decode_step_layer(
+                    ctypes.byref(self._desc), q.data_ptr(), k_ptr, v_ptr, None if packed else out.data_ptr(),
+                    rec.data_ptr() if packed else None, mask_ptr, mask_stride, self.rest_len, self.rest_start,
+                    self._flags(append), stream)
+            else:
+                d = self._desc
+                rc = self.lib.akv_decode_step_exchange(
+                    d.k_first_8, d.k_mid_4, d.k_last_4, d.v_first_8, d.v_mid_4, d.v_last_4, d.k_exp_max, d.v_exp_max, d.restk,
+                    d.restv, q.data_ptr(), k_ptr, v_ptr, out.data_ptr(), rec.data_ptr(), d.scratch, d.scratch_bytes, self.B,
+                    self.H, self.G, self.D, self.L, self.rest_len, self.rest_start, self._flags(append), exchange.bufs,
+                    exchange.rank, exchange.world, exchange.next_epoch(), exchange.timeout_ms, stream)
+        if rc != 0:
+            _lib.check("decode_step", rc)
         self.last_q = q                                   # (for bytes_accounting)
         flush = append and self.rest_len + 1 == column_block
         qn = self.rest_start + (column_block if flush else 0)
@@ -208,11 +216,11 @@ class DecodeLayer:
         appended = self.cache_len - snap["cache_len"]
         if appended < 0 or (snap["rest_len"] and snap["rest_len"] + appended > column_block):
             raise RuntimeError("restore: the residual tokens of the snapshot have been overwritten since")
-        with torch.cuda.device(self.device):
+        with _nothing if torch.cuda.current_device() == self._index else torch.cuda.device(self._index):
             rc = self.lib.akv_rollback(self.k_mid_4.data_ptr(), self.k_last_4.data_ptr(), self.k_exp_max.data_ptr(),
                                        self.v_exp_max.data_ptr(), snap["k_exp"].data_ptr(), snap["v_exp"].data_ptr(),
                                        self.B, self.H, self.D, self.L, first_blk, max(0, last_blk - first_blk),
-                                       torch.cuda.current_stream(self.device).cuda_stream)
+                                       _lib.raw_stream(self._index))
         _lib.check("rollback", rc)
         self.rest_len, self.rest_start, self.cache_len = snap["rest_len"], snap["rest_start"], snap["cache_len"]
 

@@ -238,6 +238,17 @@ int akv_decode_step_masked(void* k_first_8, void* k_mid_4, void* k_last_4, void*
                            const void* mask, long long mask_stride, void* scratch, long long scratch_bytes,
                            int bsz, int n_kv_heads, int group, int head_dim, int max_seq_len, int rest_len, int rest_start,
                            int flags, void* stream);
+/* The same with what stays from step to step - planes, buffers, workspace, extents - behind one pointer (read during the call,
+ * not kept), for callers whose share of a short step is the passing of arguments. */
+typedef struct akv_layer {
+    void *k_first_8, *k_mid_4, *k_last_4, *v_first_8, *v_mid_4, *v_last_4, *k_exp_max, *v_exp_max, *restk, *restv, *scratch;
+    long long scratch_bytes;
+    int bsz, n_kv_heads, group, head_dim, max_seq_len;
+} akv_layer;
+int akv_decode_step_layer(const akv_layer* layer, const void* q, const void* k_new, const void* v_new, void* out,
+                          void* packed_out, const void* mask, long long mask_stride, int rest_len, int rest_start, int flags,
+                          void* stream);
+
 
 /*
  * Prompt ingestion in one pass: K_Cache_Class.save + V_Cache_Class.save for start_pos == 0
