@@ -123,7 +123,11 @@ constexpr int TOK = 64;            // tokens per stage
 // pools of four would leave too little room for the ring.  (Stages of 128 tokens, prepared by two helpers, were faster in
 // back-to-back launches and slower in a decode step, where every plane byte comes from HBM: 96 against 85 us per step at
 // batch 8 x 32 heads x 4096 tokens.)
-__host__ __device__ constexpr int helpers(int upc, int heads) { return upc > (heads > 1 ? 1 : 2) ? 2 : 4; }
+// Two units of two heads: three, with a ring of six stages (two with eight were what the chains waited for: 24 sequences x 16 KV
+// heads x 2 x 8192 tokens 302 -> 271 us per step, 32 x 16 x 2 x 4096 204 -> 184; units of four heads do not gain, 480 / 480).
+__host__ __device__ constexpr int helpers(int upc, int heads) {
+    return upc > (heads > 1 ? 1 : 2) ? (heads == 2 ? 3 : 2) : 4;
+}
 // A ring slot: high bytes | probabilities [heads][TOK] | places of the low bytes [heads][8][8] (token 8 g + w of the
 // stage at [w][g]: what a lane needs for its rows of the groups lies together), in 2-byte units into the unit's pools |
 // how many tokens of the stage read a nibble plane
