@@ -65,6 +65,7 @@ SIGNATURES = {
                                                                                ctypes.c_uint, _I, _P]),
     "akv_rollback": (_I, [_P] * 6 + [_I] * 6 + [_P]),
     "akv_prefill": (_I, [_P] * 13 + [ctypes.c_longlong] + [_I] * 5 + [_P]),
+    "akv_prefill_ex": (_I, [_P] * 13 + [ctypes.c_longlong] + [_I] * 6 + [_P]),
     "akv_prefill_scratch_bytes": (ctypes.c_longlong, [_I] * 4),
     "akv_operator_scratch_bytes": (ctypes.c_longlong, [_I] * 3),
     "akv_k_scores": (_I, [_P] * 8 + [ctypes.c_longlong] + [_I] * 6 + [_F, _I, _P]),

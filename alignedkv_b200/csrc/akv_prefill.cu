@@ -90,12 +90,15 @@ __device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t byt
 __device__ __forceinline__ uint32_t mid_nibbles(uint32_t x) { return (x & 0x00F000F0u) | ((x >> 12) & 0x000F000Fu); }
 __device__ __forceinline__ uint32_t low_nibbles(uint32_t x) { return ((x << 4) & 0x00F000F0u) | ((x >> 8) & 0x000F000Fu); }
 
-// Bound by HBM: 32 KB in, 32 KB out and 8 KB of nibble planes read per tile (the K nibbles are added onto what the planes
-// hold).  Thread = (channel pair c = tid / 4, 16 tokens q = tid % 4): 16 four-byte shared loads of a tile give 2 x (16 high
-// bytes, 8 mid, 8 low bytes) of the K planes, all transposition by byte permutes; for V = (token, 32 channels).  About 4
-// integer instructions per value where the form before it (thread = channel, one 2-byte load per value, results stored 16
-// bytes at a time straight to the planes) took 10 and half-filled every sector it wrote: batch 8 x 32 heads x
-// 4096 tokens 182.5 us (1.21 GB: 6.6 TB/s) against 356.4.
+// ADD: the K nibbles are added onto what the planes hold, as the reference's writer does; else they are stored, for a caller that
+// knows the planes to be zero there: batch 8 x 32 heads x 4096 tokens 200.7 us with the rewind, 219.5 with ADD.  (Launched with
+// programmatic serialization it took 228, and the maxima so launched 270.)
+// Bound by HBM: 32 KB in, 32 KB out and, with ADD, 8 KB of nibble planes read per tile.  Thread = (channel pair c = tid / 4, 16
+// tokens q = tid % 4): 16 four-byte shared loads of a tile give 2 x (16 high bytes, 8 mid, 8 low bytes) of the K planes, all
+// transposition by byte permutes; for V = (token, 32 channels).  About 4 integer instructions per value where the form before it
+// (thread = channel, one 2-byte load per value, results stored 16 bytes at a time straight to the planes) took 10 and half-filled
+// every sector it wrote: batch 8 x 32 heads x 4096 tokens 182.5 us with ADD (1.21 GB: 6.6 TB/s) against 356.4.
+template <bool ADD>
 __global__ void __launch_bounds__(pf::NT, 4)
 prefill128_kernel(uint8_t* __restrict__ k_first_8, uint8_t* __restrict__ k_mid_4, uint8_t* __restrict__ k_last_4,
                   uint8_t* __restrict__ v_first_8, uint8_t* __restrict__ v_mid_4, uint8_t* __restrict__ v_last_4,
@@ -123,7 +126,7 @@ prefill128_kernel(uint8_t* __restrict__ k_first_8, uint8_t* __restrict__ k_mid_4
     uint8_t* mid = k_mid_4 + (tile + 2 * c) * 32 + q * 8;
     uint8_t* low = k_last_4 + (tile + 2 * c) * 32 + q * 8;
     uint2 om[2], ol[2];                                              // the nibble bytes this thread adds onto
-    if (cnt == PF_BLK) {
+    if (ADD && cnt == PF_BLK) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             om[e] = *reinterpret_cast<const uint2*>(mid + e * 32);
@@ -187,7 +190,7 @@ prefill128_kernel(uint8_t* __restrict__ k_first_8, uint8_t* __restrict__ k_mid_4
         }
     }
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {                                    // bytewise, modulo 256
+    for (int e = 0; ADD && e < 2; ++e) {                             // bytewise, modulo 256
         m[e][0] = __vadd4(m[e][0], om[e].x);
         m[e][1] = __vadd4(m[e][1], om[e].y);
         l[e][0] = __vadd4(l[e][0], ol[e].x);
@@ -279,10 +282,10 @@ long long akv_prefill_scratch_bytes(int bsz, int n_kv_heads, int head_dim, int s
     return 2ll * bsz * n_kv_heads * tiles * head_dim * 2;
 }
 
-int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8, void* v_mid_4, void* v_last_4,
-                void* k_exp_max, void* v_exp_max, void* restk, void* restv, const void* k, const void* v,
-                void* scratch, long long scratch_bytes, int bsz, int n_kv_heads, int head_dim, int max_seq_len,
-                int seqlen, void* stream) {
+int akv_prefill_ex(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8, void* v_mid_4, void* v_last_4,
+                   void* k_exp_max, void* v_exp_max, void* restk, void* restv, const void* k, const void* v,
+                   void* scratch, long long scratch_bytes, int bsz, int n_kv_heads, int head_dim, int max_seq_len,
+                   int seqlen, int flags, void* stream) {
     set_error("");
     const int B = bsz, H = n_kv_heads, D = head_dim, S = seqlen;
     AKV_REQUIRE(k_first_8 && k_mid_4 && k_last_4 && v_first_8 && v_mid_4 && v_last_4 && k_exp_max && v_exp_max &&
@@ -303,7 +306,8 @@ int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8,
     dim3 grid(tiles, H, B);
     count_launch(2);
     if (D == pf::D) {
-        prefill128_kernel<<<grid, pf::NT, 0, st>>>(
+        const auto kern = (flags & AKV_PREFILL_STORE) ? prefill128_kernel<false> : prefill128_kernel<true>;
+        kern<<<grid, pf::NT, 0, st>>>(
             static_cast<uint8_t*>(k_first_8), static_cast<uint8_t*>(k_mid_4), static_cast<uint8_t*>(k_last_4),
             static_cast<uint8_t*>(v_first_8), static_cast<uint8_t*>(v_mid_4), static_cast<uint8_t*>(v_last_4),
             static_cast<uint8_t*>(restk), static_cast<uint8_t*>(restv), static_cast<const uint8_t*>(k),
@@ -326,6 +330,14 @@ int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8,
     exp_reduce_kernel<<<B * H, 256, 0, st>>>(reinterpret_cast<const uint32_t*>(kmax_part), reinterpret_cast<const uint32_t*>(vmax_part),
                                             static_cast<uint8_t*>(k_exp_max), static_cast<uint8_t*>(v_exp_max), D / 2, tiles);
     return cuda_status(cudaGetLastError(), "prefill reduce launch");
+}
+
+int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8, void* v_mid_4, void* v_last_4,
+                void* k_exp_max, void* v_exp_max, void* restk, void* restv, const void* k, const void* v,
+                void* scratch, long long scratch_bytes, int bsz, int n_kv_heads, int head_dim, int max_seq_len,
+                int seqlen, void* stream) {
+    return akv_prefill_ex(k_first_8, k_mid_4, k_last_4, v_first_8, v_mid_4, v_last_4, k_exp_max, v_exp_max, restk, restv, k, v,
+                          scratch, scratch_bytes, bsz, n_kv_heads, head_dim, max_seq_len, seqlen, 0, stream);
 }
 
 }  // extern "C"
