@@ -143,15 +143,16 @@ __device__ __forceinline__ void fma_f32_f16x2(float& x, float& y, uint32_t v, ui
         : "+f"(x), "+f"(y) : "r"(v), "h"((uint16_t)p));
 }
 
-// Global loads past L1, of what another kernel may be storing
+// Global loads past L1, of what another kernel may be storing (any of the values it had will do; no
+// memory clobber, so that the loads of a thread go out together)
 __device__ __forceinline__ uint32_t ld_relaxed8(const uint8_t* p) {
     uint32_t v;
-    asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];\n" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint32_t ld_relaxed16(const uint16_t* p) {
     uint16_t v;
-    asm volatile("ld.relaxed.gpu.global.u16 %0, [%1];\n" : "=h"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u16 %0, [%1];\n" : "=h"(v) : "l"(p));
     return v;
 }
 

@@ -119,59 +119,63 @@ struct KCursor {
 // Query bits and alignment differences of heads g0 .. g0 + HC - 1 of a group on channels r * 32 + lane: mid plane read iff
 // (u8)(kqmax - kq[d]) < 8, low plane iff < 4 (K_cache.cu:211,249-250).  kq and kqmax as they are given, or made here from the
 // query, the exponent maxima and the new token (k_cache_file.py:98-99,136-138).
-template <int G, int HC>
-__device__ __forceinline__ void kc_load_heads(const KParams& p, long long bh, int g0, int lane, uint32_t (&qh)[HC][8],
-                                              uint32_t (&diff)[HC][8]) {
-    uint32_t ek[8];
+// NR: rows of 32 channels, D = 32 NR or less.  All loads go out before the first use: a warp that has two or three units pays this
+// latency twice per (batch, KV head), in the masks and in the tables (19 sequences x 8 KV heads x 4 x 3968 tokens 137 us per step with
+// loads a head at a time, 143 with ordered loads in functions of their own, 129 so; 8 x 4 x 8 x 10432 146.5, 149, 129).
+template <int G, int HC, int NR>
+__device__ __forceinline__ void kc_load_heads(const KParams& p, long long bh, int g0, int lane, uint32_t (&qh)[HC][NR],
+                                              uint32_t (&diff)[HC][NR]) {
+    uint32_t ek[NR], kn[NR], top[HC];
+    const bool own = p.k_exp != nullptr;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < NR; ++r) {
         const int d = r * 32 + lane;
         const bool in = d < p.D;
-        ek[r] = 0;
-        if (p.k_exp && in) {
-            // (old or new maximum: the token's exponent is taken in again)
-            ek[r] = ld_relaxed8(p.k_exp + bh * p.D + d);
-            if (p.k_new) ek[r] = max(ek[r], (ld_relaxed16(p.k_new + bh * p.D + d) >> 10) & 0x1Fu);
-        }
+        ek[r] = own && in ? ld_relaxed8(p.k_exp + bh * p.D + d) : 0u;
+        kn[r] = own && p.k_new && in ? ld_relaxed16(p.k_new + bh * p.D + d) : 0u;
 #pragma unroll
         for (int g = 0; g < HC; ++g) {
             const long long at = (bh * G + g0 + g) * p.D + d;
             qh[g][r] = in ? ld_relaxed16(reinterpret_cast<const uint16_t*>(p.q) + at) : 0u;
-            diff[g][r] = !p.k_exp && in ? __ldg(p.kq + at) : 0u;
+            diff[g][r] = !own && in ? __ldg(p.kq + at) : 0u;
         }
     }
 #pragma unroll
-    for (int g = 0; g < HC; ++g) {
-        uint32_t top = 0;
-        if (p.k_exp) {
+    for (int g = 0; g < HC; ++g) top[g] = own ? 0u : __ldg(p.kqmax + bh * G + g0 + g);
+    if (own) {
+        // (old or new maximum: the token's exponent is taken in again)
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+        for (int r = 0; r < NR; ++r) ek[r] = max(ek[r], (kn[r] >> 10) & 0x1Fu);
+#pragma unroll
+        for (int g = 0; g < HC; ++g) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
                 if (r * 32 + lane < p.D) {
                     diff[g][r] = (((qh[g][r] >> 10) & 0x1Fu) + ek[r]) & 0xFFu;
-                    top = max(top, diff[g][r]);
+                    top[g] = max(top[g], diff[g][r]);
                 }
-            top = __reduce_max_sync(0xFFFFFFFFu, top);
-        } else {
-            top = __ldg(p.kqmax + bh * G + g0 + g);
+            top[g] = __reduce_max_sync(0xFFFFFFFFu, top[g]);
         }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) diff[g][r] = p.reference ? 0u : (top - diff[g][r]) & 0xFFu;
     }
+#pragma unroll
+    for (int g = 0; g < HC; ++g)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) diff[g][r] = p.reference ? 0u : (top[g] - diff[g][r]) & 0xFFu;
 }
 // The union of the group's plane-read masks (bit d set = row d of that plane is read), which is what the producer fetches; with
 // one head its table too.
-template <int G>
+template <int G, int NR>
 __device__ __forceinline__ void kc_load_masks(const KParams& p, long long bh, uint32_t* um, uint32_t* table, int lane) {
     constexpr int HC = G > 4 ? 4 : G;             // (registers)
-    uint32_t least[8];
+    uint32_t least[NR];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) least[r] = 0xFFu;
+    for (int r = 0; r < NR; ++r) least[r] = 0xFFu;
 #pragma unroll 1
     for (int g0 = 0; g0 < G; g0 += HC) {
-        uint32_t qh[HC][8], diff[HC][8];
-        kc_load_heads<G, HC>(p, bh, g0, lane, qh, diff);
+        uint32_t qh[HC][NR], diff[HC][NR];
+        kc_load_heads<G, HC, NR>(p, bh, g0, lane, qh, diff);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < NR; ++r) {
             const int d = r * 32 + lane;
             if (d >= p.D) break;
 #pragma unroll
@@ -180,7 +184,7 @@ __device__ __forceinline__ void kc_load_masks(const KParams& p, long long bh, ui
         }
     }
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < NR; ++r) {
         if (r * 32 >= p.D) break;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, least[r] < 8), l = __ballot_sync(0xFFFFFFFFu, least[r] < 4);
         if (lane == 0) {
@@ -190,26 +194,20 @@ __device__ __forceinline__ void kc_load_masks(const KParams& p, long long bh, ui
     }
     __syncwarp();
 }
-// (Groups: out of the loop's instruction stream and registers.  One head is faster inline, 78.8 against 80.0 us per step at
-// batch 8 x 32 x 4096; four the other way round, 515 against 510 at batch 64 x 8 x 8192.)
-template <int G>
-__device__ __noinline__ void kc_load_masks_far(const KParams& p, long long bh, uint32_t* um, uint32_t* table, int lane) {
-    kc_load_masks<G>(p, bh, um, table, lane);
-}
 // The consumer's tables of a group (all its lanes are done with the previous ones).
-template <int G>
-__device__ __noinline__ void kc_load_tables(const KParams& p, long long bh, uint8_t* tables, int lane) {
+template <int G, int NR>
+__device__ __forceinline__ void kc_load_tables(const KParams& p, long long bh, uint8_t* tables, int lane) {
     constexpr int HC = G > 4 ? 4 : G;
     __syncwarp();
 #pragma unroll 1
     for (int g0 = 0; g0 < G; g0 += HC) {
-        uint32_t qh[HC][8], diff[HC][8];
-        kc_load_heads<G, HC>(p, bh, g0, lane, qh, diff);
+        uint32_t qh[HC][NR], diff[HC][NR];
+        kc_load_heads<G, HC, NR>(p, bh, g0, lane, qh, diff);
 #pragma unroll
         for (int g = 0; g < HC; ++g) {
             uint32_t* hm = reinterpret_cast<uint32_t*>(tables + (size_t)(g0 + g) * kc::head_meta(p.D, G));
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
+            for (int r = 0; r < NR; ++r) {
                 const int d = r * 32 + lane;
                 if (d >= p.D) break;
                 const uint32_t x = diff[g][r];
@@ -239,6 +237,7 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
     pdl_trigger();
     if (!p.k_exp) pdl_wait();
     const int D = DC ? DC : p.D;
+    constexpr int NR = DC ? (DC + 31) / 32 : MAX_D / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wpc = blockDim.x >> 5;
     const int w = blockIdx.x * wpc + warp;
@@ -286,11 +285,10 @@ __global__ void __launch_bounds__(kc::max_warps(G) * 32, 1) k_compute_kernel(con
     auto load_masks = [&](long long bh, int slot) {
         uint32_t* um = reinterpret_cast<uint32_t*>(meta0 + slot * MASK_BYTES);
         uint32_t* table = reinterpret_cast<uint32_t*>(tables + slot * HMETA);
-        if (G == 1) kc_load_masks<G>(p, bh, um, table, lane);
-        else kc_load_masks_far<G>(p, bh, um, table, lane);
+        kc_load_masks<G, NR>(p, bh, um, table, lane);
     };
     auto load_tables = [&](long long bh) {
-        if (G > 1) kc_load_tables<G>(p, bh, tables, lane);
+        if (G > 1) kc_load_tables<G, NR>(p, bh, tables, lane);
     };
 
     const int nrow = (lane % ROW_LANES) >> 1, nhalf = (lane & 1) << 4, ntsub = lane / ROW_LANES;
