@@ -1,11 +1,13 @@
 // The element-wise parts of a decoder's decode step between its matrix products (model/Llama_AlignedKV.py's layer, as
-// llama.py restates it): rotary embedding with the split into queries, keys and values, and SwiGLU's activation.
+// llama.py restates it): rotary embedding with the split into queries, keys and values, SwiGLU's activation, RMSNorm.
 //   rope_split_kernel   qkv [B, H + 2 Hkv, D] -> q [B,H,D], k, v [B,Hkv,D]; q and k rotated (rotate_half form)
 //   silu_mul_kernel     [rows, 2 F] (gate | up) -> silu(gate) * up
 //   rms_norm_kernel     x / sqrt(mean(x^2) + eps) * w per row
 // One launch each where tensor operations take 22, 2 and 1: at batch 16 every one of those is a kernel of 2 us and more that
-// moves a few hundred kilobytes.  Arithmetic and roundings are those of the tensor operations: tables and rotation in fp32,
-// rounded once; silu in fp32, rounded to fp16, then an fp16 product; the norm in fp32, rounded once.
+// moves a few hundred kilobytes.  Rotation and activation are the tensor operations' bit for bit: tables and rotation in fp32,
+// rounded once; silu in fp32, rounded to fp16, then an fp16 product.  The norm is computed in fp32 and rounded once, but adds its
+// squares in an order of its own (about one value in 20000 is one fp16 step off torch's, which two layers turn into logits
+// 8e-4 off): LlamaDecoder takes torch's, one launch as well.
 #include "akv_common.cuh"
 
 namespace akv {

@@ -132,7 +132,7 @@ class LlamaDecoder:
         cfg, p = self.cfg, self.layers[i]
         H, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         B = x.shape[0]
-        qkv = F.linear(self._norm(x, p["norm1"]), p["wqkv"]).view(B, 1, H + 2 * Hkv, D)
+        qkv = F.linear(_rms_norm(x, p["norm1"], cfg.rms_norm_eps), p["wqkv"]).view(B, 1, H + 2 * Hkv, D)
         if D % 16 or D > 256:
             qk = _rope(qkv[:, :, :H + Hkv], _rope_tables(pos, D, cfg.rope_theta))
             return qk[:, :, :H].contiguous(), qk[:, :, H:].contiguous(), qkv[:, :, H + Hkv:].contiguous()
@@ -146,7 +146,7 @@ class LlamaDecoder:
         cfg, p = self.cfg, self.layers[i]
         B, Fi = x.shape[0], cfg.intermediate_size
         x = torch.addmm(x.view(B, -1), o.reshape(B, -1), p["wo"].t()).view(B, 1, -1)
-        gate_up = F.linear(self._norm(x, p["norm2"]), p["w_gate_up"])
+        gate_up = F.linear(_rms_norm(x, p["norm2"], cfg.rms_norm_eps), p["w_gate_up"])
         if Fi % 8:
             gate, up = gate_up.chunk(2, dim=-1)
             h = F.silu(gate).mul_(up).view(B, -1)
@@ -154,15 +154,6 @@ class LlamaDecoder:
             h = torch.empty(B, Fi, dtype=torch.half, device=x.device)
             self._native("akv_silu_mul", gate_up.data_ptr(), h.data_ptr(), B, Fi)
         return torch.addmm(x.view(B, -1), h, p["w_down"].t()).view(B, 1, -1)
-
-    def _norm(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-        """RMSNorm of a decode step's rows [B,1,E]."""
-        E = x.shape[-1]
-        if E % 8 or E > 16384 or w.dtype != torch.half or not w.is_contiguous() or w.data_ptr() % 16:
-            return _rms_norm(x, w, self.cfg.rms_norm_eps)
-        out = torch.empty_like(x)
-        self._native("akv_rms_norm", x.data_ptr(), w.data_ptr(), out.data_ptr(), x.shape[0], E, self.cfg.rms_norm_eps)
-        return out
 
     def _native(self, fn: str, *args) -> None:
         with torch.cuda.device(self.device):
@@ -190,7 +181,7 @@ class LlamaDecoder:
             else:
                 x = self._post(j - 1, x_prev, self._g_o)
             if j == n:
-                x = self._norm(x, self.final_norm)
+                x = _rms_norm(x, self.final_norm, cfg.rms_norm_eps)
                 return (F.linear(x, self.lm_head)[:, 0],)
             return (x,) + self._pre(j, x, self._g_pos)
 
@@ -237,10 +228,7 @@ class LlamaDecoder:
             for i in range(self.cfg.num_hidden_layers):
                 x = self._post(i, x, self.caches[i].decode(*self._pre(i, x, pos)))
         self.pos += S
-        if prompt or self.attention != "alignedkv":
-            x = _rms_norm(x[:, -1:], self.final_norm, self.cfg.rms_norm_eps)
-        else:
-            x = self._norm(x, self.final_norm)
+        x = _rms_norm(x[:, -1:], self.final_norm, self.cfg.rms_norm_eps)
         return F.linear(x, self.lm_head)[:, 0]                                   # logits of the last position [B,V]
 
     # ------------------------------------------------------------------ public

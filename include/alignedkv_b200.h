@@ -146,7 +146,8 @@ long long akv_operator_scratch_bytes(int bsz, int n_heads, int head_dim);
  * akv_rope_split: qkv fp16 [B, H + 2 Hkv, D] -> q [B,H,D], k, v [B,Hkv,D]; q and k rotated to position pos[0] (int64 in device
  * memory), rotate_half form, tables and rotation in fp32.  head_dim a multiple of 16, at most 256.
  * akv_silu_mul: gate_up fp16 [rows, 2 width] -> out [rows, width] = half(silu(gate)) * up.  width a multiple of 8.
- * akv_rms_norm: out = half(x / sqrt(mean(x^2) + eps) * w) per row of `width` fp16 values (a multiple of 8, at most 16384).
+ * akv_rms_norm: out = half(x / sqrt(mean(x^2) + eps) * w) per row of `width` fp16 values (a multiple of 8, at most 16384), the
+ * squares added in fp32 in an order of its own.
  * All pointers 16-byte aligned (pos: 8).
  */
 int akv_rms_norm(const void* x, const void* w, void* out, int rows, int width, float eps, void* stream);

@@ -52,3 +52,46 @@ def test_decoder_graph_replay_matches_eager(akv_lib):
         assert err <= 1e-3, err
         tok = la.argmax(-1)
     assert a.pos == b.pos and akv_lib.akv_device_error_flag() == 0
+
+
+def tensor_step(dec, ids):
+    """`LlamaDecoder.step` with torch's operations between the matrix products and the attention."""
+    from alignedkv_b200.llama import _rms_norm, _rope, _rope_tables
+    F, cfg, B = torch.nn.functional, dec.cfg, dec.B
+    H, Hkv, D, eps = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.rms_norm_eps
+    tables = _rope_tables(torch.tensor([dec.pos], device=dec.device), D, cfg.rope_theta)
+    x = dec.embed[ids.view(B, 1)]
+    for p, cache in zip(dec.layers, dec.caches):
+        qkv = F.linear(_rms_norm(x, p["norm1"], eps), p["wqkv"]).view(B, 1, H + 2 * Hkv, D)
+        qk = _rope(qkv[:, :, :H + Hkv], tables)
+        o = cache.decode(qk[:, :, :H].contiguous(), qk[:, :, H:].contiguous(), qkv[:, :, H + Hkv:].contiguous())
+        x = torch.addmm(x.view(B, -1), o.reshape(B, -1), p["wo"].t()).view(B, 1, -1)
+        gate, up = F.linear(_rms_norm(x, p["norm2"], eps), p["w_gate_up"]).chunk(2, dim=-1)
+        x = torch.addmm(x.view(B, -1), F.silu(gate).mul_(up).view(B, -1), p["w_down"].t()).view(B, 1, -1)
+    dec.pos += 1
+    return F.linear(_rms_norm(x, dec.final_norm, eps), dec.lm_head)[:, 0]
+
+
+@pytest.mark.parametrize("E,Fi,H,Hkv,B", [(256, 512, 4, 4, 1), (512, 1032, 4, 2, 3), (768, 1000, 4, 4, 5), (1024, 2048, 4, 1, 2),
+                                          (4096, 11008, 32, 8, 16)])
+def test_step_is_that_of_tensor_operations(akv_lib, E, Fi, H, Hkv, B):
+    """Bit for bit: the kernels between the matrix products round as the tensor operations do, in the same order of additions."""
+    from alignedkv_b200.llama import LlamaConfig, LlamaDecoder
+    cfg = LlamaConfig(hidden_size=E, intermediate_size=Fi, num_hidden_layers=2, num_attention_heads=H, num_key_value_heads=Hkv,
+                      vocab_size=1000)
+    g = torch.Generator(device="cuda").manual_seed(E)
+    S, new = 100, 4
+    ids = torch.randint(0, cfg.vocab_size, (B, S + new), device="cuda", generator=g)
+    decs = [LlamaDecoder(cfg, B, S + new + 64, "cuda:0", seed=2) for _ in range(3)]
+    norms = [(torch.randn(E, device="cuda", generator=g) * 0.3 + 1).half() for _ in range(5)]
+    for dec in decs:
+        for i, p in enumerate(dec.layers):
+            p["norm1"], p["norm2"] = norms[2 * i], norms[2 * i + 1]
+        dec.final_norm = norms[4]
+        dec.prefill(ids[:, :S])
+    decs[1].capture_graphs()
+    with torch.no_grad():
+        for t in range(new):
+            want = tensor_step(decs[2], ids[:, S + t])
+            for dec in decs[:2]:
+                assert torch.equal(dec.step(ids[:, S + t]).view(torch.int16), want.view(torch.int16))
