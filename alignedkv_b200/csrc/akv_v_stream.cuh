@@ -121,6 +121,8 @@ __global__ void __launch_bounds__(160) v_stream_kernel(const VStreamParams p) {
 #pragma unroll 1
         for (int i = 0; i < nst; ++i) {
             if (i >= nf) {
+                // (no slot comes free before the consumers may start: a bounded wait must not count the kernel in front)
+                if (p.early && i == nf) pdl_wait();
                 alive = mbar_wait(bar_free + slot * 8, parity);
                 if (!alive) break;
             }

@@ -209,3 +209,15 @@ def test_cpu_baseline_leg_runs():
     want = dense_attention_fp32(q, k, v)
     assert got.shape == (1, 1, 4, 64)
     assert np.abs(got.astype(np.float32) - want).max() / np.abs(want).max() < 5e-3
+
+
+def test_bounded_waits_start_behind_the_kernel_in_front():
+    """The order-free P.V kernel's copy warp runs ahead of the kernel in front of it.  The ring's slots come free only once the
+    consumers have passed their own wait for that kernel, so the copy warp waits for it before its first bounded wait: a kernel in
+    front that is held up must not make that wait give up.  (By reading: nothing holds a kernel up for a second on purpose.)"""
+    with open(os.path.join(ROOT, "alignedkv_b200", "csrc", "akv_v_stream.cuh")) as f:
+        src = f.read()
+    copy_warp = src[src.index("if (warp == CONSUMERS) {"):src.index("consumer warps", src.index("if (warp == CONSUMERS) {"))]
+    assert copy_warp.count("mbar_wait(") == 1
+    front = copy_warp[:copy_warp.index("mbar_wait(")]
+    assert re.search(r"if \(i >= nf\) \{[^}]*if \(p\.early && i == nf\) pdl_wait\(\);\s*alive = $", front)
