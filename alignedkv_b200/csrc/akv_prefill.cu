@@ -90,9 +90,10 @@ __device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t byt
 __device__ __forceinline__ uint32_t mid_nibbles(uint32_t x) { return (x & 0x00F000F0u) | ((x >> 12) & 0x000F000Fu); }
 __device__ __forceinline__ uint32_t low_nibbles(uint32_t x) { return ((x << 4) & 0x00F000F0u) | ((x >> 8) & 0x000F000Fu); }
 
-// ADD: the K nibbles are added onto what the planes hold, as the reference's writer does; else they are stored, for a caller that
-// knows the planes to be zero there: batch 8 x 32 heads x 4096 tokens 200.7 us with the rewind, 219.5 with ADD.  (Launched with
-// programmatic serialization it took 228, and the maxima so launched 270.)
+// ADD: the K nibbles are added onto what the planes hold, as the reference's writer does (DecodeLayer.prefill); else they are
+// stored, for a caller of the library that knows the planes to be zero there: batch 8 x 32 heads x 4096 tokens 200.7 us with the
+// rewind, 219.5 with ADD.  A layer cannot know: a tensor's version counter sees no writer that has its address (this library's
+// K block writer, `.data`, DLPack).  (Launched with programmatic serialization it took 228, and the maxima so launched 270.)
 // Bound by HBM: 32 KB in, 32 KB out and, with ADD, 8 KB of nibble planes read per tile.  Thread = (channel pair c = tid / 4, 16
 // tokens q = tid % 4): 16 four-byte shared loads of a tile give 2 x (16 high bytes, 8 mid, 8 low bytes) of the K planes, all
 // transposition by byte permutes; for V = (token, 32 channels).  About 4 integer instructions per value where the form before it

@@ -23,7 +23,6 @@ __all__ = ["DecodeLayer"]
 _nothing = contextlib.nullcontext()
 
 AKV_STEP_REFERENCE, AKV_STEP_ORDER_FREE, AKV_STEP_NO_APPEND, AKV_STEP_TRACK_MAXIMA = 1, 2, 4, 8
-AKV_PREFILL_STORE = 1
 
 
 class DecodeLayer:
@@ -65,8 +64,6 @@ class DecodeLayer:
             raise ValueError("bad extents")
         self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         self._sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
-        m, l = self.k_mid_4, self.k_last_4
-        self._nibbles = None if m.is_inference() else (m.data_ptr(), l.data_ptr(), m._version, l._version)   # (they are zero)
         self._desc = None                    # `_lib.Layer`, made by the first step
         self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self._q_shape, self._kv_shape = (bsz, 1, self.Hq, head_dim), (bsz, 1, n_heads, head_dim)
@@ -86,14 +83,6 @@ class DecodeLayer:
         return (AKV_STEP_REFERENCE if getattr(self, "reference", False) else 0) | \
                (AKV_STEP_ORDER_FREE if self.v_mode == "order_free" else 0) | (0 if append else AKV_STEP_NO_APPEND)
 
-    def _nibbles_known(self) -> bool:
-        """Whether only this layer has written the K nibble planes, which are then zero wherever no block is cached (`restore`
-        clears what it takes back): they have the addresses and version counters they were made with - a tensor operation on
-        them counts the version up.  False where versions are not kept (inference tensors)."""
-        m, l, was = self.k_mid_4, self.k_last_4, self._nibbles
-        return was is not None and m.data_ptr() == was[0] and l.data_ptr() == was[1] and not m.is_inference() and \
-            not l.is_inference() and m._version == was[2] and l._version == was[3]
-
     # ------------------------------------------------------------------ prompt
     def prefill(self, k: torch.Tensor, v: torch.Tensor) -> None:
         """Ingest a prompt [B,S,H,D]: whole 64-token blocks to the planes, the tail to the residual buffers, the
@@ -110,12 +99,11 @@ class DecodeLayer:
             nbytes = self.lib.akv_prefill_scratch_bytes(B, H, D, S)
             ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             with _nothing if torch.cuda.current_device() == self._index else torch.cuda.device(self._index):
-                rc = self.lib.akv_prefill_ex(
+                rc = self.lib.akv_prefill(
                     self.k_first_8.data_ptr(), self.k_mid_4.data_ptr(), self.k_last_4.data_ptr(),
                     self.v_first_8.data_ptr(), self.v_mid_4.data_ptr(), self.v_last_4.data_ptr(),
                     self.k_exp_max.data_ptr(), self.v_exp_max.data_ptr(), self.restk.data_ptr(), self.restv.data_ptr(),
-                    k.data_ptr(), v.data_ptr(), ws.data_ptr(), nbytes, B, H, D, self.L, S,
-                    AKV_PREFILL_STORE if self._nibbles_known() else 0, _lib.raw_stream(self._index))
+                    k.data_ptr(), v.data_ptr(), ws.data_ptr(), nbytes, B, H, D, self.L, S, _lib.raw_stream(self._index))
             _lib.check("prefill", rc)
         elif S > 0:
             # head sizes the fused kernel does not cover: the operator-by-operator route
