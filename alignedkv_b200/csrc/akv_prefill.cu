@@ -294,6 +294,7 @@ int akv_prefill_ex(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first
     AKV_REQUIRE(B > 0 && B <= 65535 && H > 0 && H <= 65535 && D > 0 && D % 32 == 0 && D <= 256 && S > 0 &&
                 S <= max_seq_len, AKV_ERR_SHAPE, "prefill: unsupported extent (bsz %d, heads %d, head_dim %d [multiple "
                 "of 32, at most 256], seqlen %d, max_seq_len %d)", B, H, D, S, max_seq_len);
+    AKV_REQUIRE((flags & ~AKV_PREFILL_STORE) == 0, AKV_ERR_SHAPE, "prefill: unknown flags %d", flags);
     AKV_REQUIRE(scratch_bytes >= akv_prefill_scratch_bytes(B, H, D, S), AKV_ERR_SHAPE,
                 "prefill: scratch of %lld bytes is too small", scratch_bytes);
     AKV_REQUIRE(aligned16(k_first_8) && aligned16(k_mid_4) && aligned16(k_last_4) && aligned16(v_first_8) &&

@@ -265,8 +265,8 @@ int akv_prefill(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8,
                 void* k_exp_max, void* v_exp_max, void* restk, void* restv, const void* k, const void* v,
                 void* scratch, long long scratch_bytes, int bsz, int n_kv_heads, int head_dim, int max_seq_len,
                 int seqlen, void* stream);
-/* The same.  flags: AKV_PREFILL_STORE stores the K nibbles instead of adding them, which is the same where the K nibble planes of
- * the prompt's whole blocks are zero, as akv_prefill expects them, and spares reading them. */
+/* The same.  flags: 0 or AKV_PREFILL_STORE, by which the caller states that the K nibble planes of the prompt's whole blocks are
+ * zero, as akv_prefill expects them: with head_dim 128 the nibbles are then stored instead of added, which spares reading them. */
 #define AKV_PREFILL_STORE 1
 int akv_prefill_ex(void* k_first_8, void* k_mid_4, void* k_last_4, void* v_first_8, void* v_mid_4, void* v_last_4,
                 void* k_exp_max, void* v_exp_max, void* restk, void* restv, const void* k, const void* v,

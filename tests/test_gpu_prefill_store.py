@@ -91,3 +91,11 @@ def test_inference_tensors_add():
         layer.k_mid_4.fill_(3)
         layer.prefill(k, v)
     assert torch.equal(layer.k_mid_4[:, :, :1], clean.k_mid_4[:, :, :1] + 3)
+
+
+def test_unknown_flags_are_refused():
+    from alignedkv_b200.decode import DecodeLayer
+    k, v, _ = inputs(1, 1, 128, 64)
+    layer = DecodeLayer(1, 128, 1, 128, "cuda:0")
+    for flags in (2, 3, -1):
+        assert call_ex(layer, k, v, flags) == -2 and int(layer.k_first_8.count_nonzero()) == 0
