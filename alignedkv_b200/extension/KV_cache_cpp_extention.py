@@ -15,7 +15,7 @@ import torch
 
 from .. import _lib
 
-__all__ = ["cuda_module"]
+__all__ = ["cuda_module", "own_operators"]
 
 
 def _u8(name: str, t: torch.Tensor, dev: torch.device | None = None) -> int:
@@ -161,6 +161,16 @@ class _CudaModule:
                    o.data_ptr(), ws.data_ptr(), nb, bsz, n_kv_heads, max_seq_len, head_dim, s.shape[-1], n, rest_len,
                    int(bool(reference)))
         return o
+
+
+#: The operators as this file defines them.
+_OWN = {name: f for name, f in vars(_CudaModule).items() if not name.startswith("_")}
+
+
+def own_operators(module, *names: str) -> bool:
+    """Whether `module` serves these operators itself: none of them wrapped or replaced, on the object or on its class."""
+    return type(module) is _CudaModule and all(
+        name not in module.__dict__ and vars(_CudaModule).get(name) is _OWN[name] for name in names)
 
 
 cuda_module = _CudaModule()

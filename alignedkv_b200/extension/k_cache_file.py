@@ -13,7 +13,7 @@ import math
 import torch
 
 from ._planes import ResidualBuffer, bits_in_a_channel, cdiv, column_block, exponent_field, one_call
-from .KV_cache_cpp_extention import cuda_module
+from .KV_cache_cpp_extention import cuda_module, own_operators
 
 __all__ = ["K_Cache_Class", "bits_in_a_channel", "column_block", "cdiv"]
 
@@ -108,12 +108,11 @@ class K_Cache_Class(torch.nn.Module):
         assert q.shape == want, f"q.shape: {q.shape} != {want}"
         B, H, D, start, fill = self.bsz, self.n_local_kv_heads, self.head_dim, self._rest.start, self._rest.fill
         planes = (self.k_cache_first_8, self.k_cache_mid_4, self.k_cache_last_4)
-        op = getattr(cuda_module, "k_scores", None)
-        if op is not None and seqlen == 1 and D % 64 == 0 and D <= 1024 and start % column_block == 0 and \
-                0 <= fill <= column_block and start + fill == start_pos + 1 and \
+        if own_operators(cuda_module, "k_cache_compute") and seqlen == 1 and D % 64 == 0 and D <= 1024 and \
+                start % column_block == 0 and 0 <= fill <= column_block and start + fill == start_pos + 1 and \
                 one_call(q, self._rest.data, self.k_cache_exp_column_max, planes, (B, column_block, H, D), (B, 1, H, D)):
-            return op(*planes, self.k_cache_exp_column_max, self._rest.data, q, B, H, start // column_block, self.n_max_blocks,
-                      D, fill, 1.0 / math.sqrt(D), reference)
+            return cuda_module.k_scores(*planes, self.k_cache_exp_column_max, self._rest.data, q, B, H, start // column_block,
+                                        self.n_max_blocks, D, fill, 1.0 / math.sqrt(D), reference)
         # alignment inputs: exponent upper bound of every product q_d * k_{t,d}, and its maximum over channels
         k_column_max_multiply_q = exponent_field(q) + self.k_cache_exp_column_max
         k_column_max_multiply_q_max = torch.max(k_column_max_multiply_q, dim=3, keepdim=True).values

@@ -10,7 +10,7 @@ import torch
 import torch.nn.functional as F
 
 from ._planes import ResidualBuffer, bits_in_a_channel, cdiv, column_block, exponent_field, one_call
-from .KV_cache_cpp_extention import cuda_module
+from .KV_cache_cpp_extention import cuda_module, own_operators
 
 __all__ = ["V_Cache_Class", "bits_in_a_channel", "column_block", "cdiv"]
 
@@ -126,14 +126,14 @@ class V_Cache_Class(torch.nn.Module):
         quantized = self._rest.start
         B, H, D, fill = self.bsz, self.n_local_kv_heads, self.head_dim, self._rest.fill
         planes = (self.v_cache_first_8, self.v_cache_mid_4, self.v_cache_last_4)
-        op = getattr(cuda_module, "v_output", None)
-        if op is not None and type(self).test_compute is V_Cache_Class.test_compute and self.top_max_k == 32 and \
+        if own_operators(cuda_module, "v_cache_test_compute", "v_cache_compute") and \
+                getattr(self.test_compute, "__func__", None) is _test_compute and self.top_max_k == 32 and \
                 seqlen == 1 and D % 64 == 0 and D <= 256 and quantized > 0 and quantized % column_block == 0 and \
                 quantized <= 1 << 21 and 0 <= fill <= column_block and quantized + fill == start_pos + 1 <= s.shape[-1] and \
                 s.shape[-1] % 8 == 0 and \
                 one_call(s, self._rest.data, self.v_cache_exp_column_max, planes, (B, column_block, H, D), (B, 1, H, D)):
-            return op(*planes, self.v_cache_exp_column_max, self._rest.data, s, B, H, self.max_seq_len, D, quantized, fill,
-                      reference)
+            return cuda_module.v_output(*planes, self.v_cache_exp_column_max, self._rest.data, s, B, H, self.max_seq_len, D,
+                                        quantized, fill, reference)
         s_cut = s[:, :, :, :quantized]
         test_o_exp = self.test_compute(s_cut if quantized else s, start_pos, seqlen, self.top_max_k)
         # Smallest probability exponent whose product with this head's largest V can still reach the probe
@@ -150,3 +150,6 @@ class V_Cache_Class(torch.nn.Module):
         o += torch.matmul(s[:, :, :, quantized:start_pos + seqlen],
                           self._rest.data.transpose(1, 2)[:, :, :self._rest.fill, :])
         return o
+
+
+_test_compute = V_Cache_Class.test_compute      # (`decoding_compute`: the probe is this class's own, not one put in its place)

@@ -105,3 +105,53 @@ def test_routes():
     s = kc.decoding_compute(qg, 69, 1)
     s[..., 64:70].float().sum().backward()
     assert qg.grad is not None and bool((qg.grad != 0).any())
+
+
+def counting(f, seen):
+    def wrapped(*a, **kw):
+        seen.append(f.__name__)
+        return f(*a, **kw)
+    return wrapped
+
+
+@pytest.mark.parametrize("where", ["instance", "class", "subclass"])
+def test_replaced_probe_is_called(monkeypatch, where):
+    """A `test_compute` put in the class's place, wherever it was put, is the one that runs."""
+    from alignedkv_b200.extension.v_cache_file import V_Cache_Class
+    _, vc, _ = make(2, 3, 128, 130, 7)
+    p = torch.softmax(torch.randn(2, 3, 1, 192, device="cuda"), -1).half()
+    want = vc.decoding_compute(p, 129, 1)
+    seen, own = [], V_Cache_Class.test_compute
+    replaced = lambda self, *a: seen.append("test_compute") or own(self, *a)  # noqa: E731
+    if where == "instance":
+        vc.test_compute = lambda *a: replaced(vc, *a)
+    elif where == "class":
+        monkeypatch.setattr(V_Cache_Class, "test_compute", replaced)
+    else:
+        vc.__class__ = type("Sub", (V_Cache_Class,), {"test_compute": replaced})
+    got = vc.decoding_compute(p, 129, 1)
+    assert seen == ["test_compute"]
+    assert bool(((got.float() - want.float()).abs() <= 2.0 ** -9 * want.float().abs() + 2.0 ** -14).all())
+
+
+@pytest.mark.parametrize("where", ["object", "class", "module"])
+def test_wrapped_operators_are_called(monkeypatch, where):
+    """Operators of `cuda_module` that a program wraps (to log, count or replace them) are called as before."""
+    from helpers import CudaModuleSpy
+    from alignedkv_b200.extension import k_cache_file, v_cache_file
+    cm = k_cache_file.cuda_module
+    kc, vc, q = make(2, 3, 128, 130, 7)
+    p = torch.softmax(torch.randn(2, 3, 1, 192, device="cuda"), -1).half()
+    names = ["k_cache_compute", "v_cache_test_compute", "v_cache_compute"]
+    seen = []
+    if where == "module":
+        spy = CudaModuleSpy(cm)
+        for m in (k_cache_file, v_cache_file):
+            monkeypatch.setattr(m, "cuda_module", spy)
+    else:
+        at = cm if where == "object" else type(cm)
+        for n in names:
+            monkeypatch.setattr(at, n, counting(getattr(at, n), seen))
+    kc.decoding_compute(q, 129, 1)
+    vc.decoding_compute(p, 129, 1)
+    assert (list(spy.calls) if where == "module" else seen) == names
