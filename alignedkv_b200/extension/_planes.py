@@ -19,11 +19,25 @@ def exponent_field(x: torch.Tensor) -> torch.Tensor:
     return (x.view(torch.int16) >> 10).to(torch.uint8) & 0x1F
 
 
+def observed() -> bool:
+    """Whether something is in force that sees, records or changes single tensor operations, so that they have to run as such:
+    a dispatch or function mode (one that only names the default device aside), a functorch transform, forward-mode
+    derivatives, tracing, autocast.  A private query that this torch does not have counts as a yes."""
+    try:
+        if torch._C._len_torch_dispatch_stack() or forward_ad._current_level >= 0 or torch.jit.is_tracing() or \
+                torch.is_autocast_enabled("cuda") or torch._C._functorch.peek_interpreter_stack() is not None:
+            return True
+        n = torch._C._len_torch_function_stack()
+        return n > 0 and any(type(torch._C._get_function_stack_at(i)).__module__ != "torch.utils._device" for i in range(n))
+    except (AttributeError, TypeError):
+        return True
+
+
 def one_call(x: torch.Tensor, rest: torch.Tensor | None, exp_max: torch.Tensor, planes, rest_shape, exp_shape) -> bool:
     """Whether `decoding_compute` may run as one library call (`cuda_module.k_scores` / `v_output`) instead of tensor
-    operations: plain contiguous 16-byte aligned CUDA tensors of the cache's own shapes on one device, nothing that autograd,
-    forward-mode derivatives or a tensor subclass would have to see.  Everything else takes the tensor operations, and fails
-    there where it failed before."""
+    operations: plain contiguous 16-byte aligned CUDA tensors of the cache's own shapes on one device, nothing that autograd, a
+    tensor subclass or what `observed` asks for would have to see.  Everything else takes the tensor operations, and fails there
+    where it failed before."""
     if type(x) is not torch.Tensor or not x.is_cuda or x.dtype != torch.half or not x.is_contiguous() or type(rest) is not torch.Tensor:
         return False
     if rest.dtype != torch.half or rest.shape != rest_shape or not rest.is_contiguous() or rest.device != x.device:
@@ -32,7 +46,7 @@ def one_call(x: torch.Tensor, rest: torch.Tensor | None, exp_max: torch.Tensor, 
         return False
     if torch.is_grad_enabled() and (x.requires_grad or rest.requires_grad):
         return False
-    if forward_ad._current_level >= 0:
+    if observed():
         return False
     at = x.data_ptr() | rest.data_ptr() | exp_max.data_ptr()
     for p in planes:

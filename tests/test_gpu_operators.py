@@ -155,3 +155,40 @@ def test_wrapped_operators_are_called(monkeypatch, where):
     kc.decoding_compute(q, 129, 1)
     vc.decoding_compute(p, 129, 1)
     assert (list(spy.calls) if where == "module" else seen) == names
+
+
+def test_modes_see_the_operations():
+    """Dispatch and function modes, autocast and functorch transforms keep the tensor operations; a default device does not."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from alignedkv_b200.extension._planes import observed
+    kc, vc, q = make(2, 3, 128, 130, 7)
+    p = torch.softmax(torch.randn(2, 3, 1, 192, device="cuda"), -1).half()
+    seen = []
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", str(func)))
+            return func(*args, **(kwargs or {}))
+
+    for mode in (Dispatch, Function):
+        seen.clear()
+        with mode():
+            kc.decoding_compute(q, 129, 1)
+            vc.decoding_compute(p, 129, 1)
+        assert sum("matmul" in n or "bmm" in n for n in seen) >= 2 and any("max" in n for n in seen), seen
+    # autocast computes the residual tokens' products in its own type
+    with torch.autocast("cuda", torch.bfloat16):
+        s = kc.decoding_compute(q, 129, 1)
+    rest = torch.matmul(q.transpose(1, 2).bfloat16(), kc.restk[:, :2].permute(0, 2, 3, 1).bfloat16()) / 128 ** 0.5
+    assert torch.equal(s[..., 128:130], rest.half())
+    assert not observed()
+    with torch.device("cuda"):
+        assert not observed()
+    torch.func.vmap(lambda x: seen.append(observed()) or x)(q)
+    assert seen[-1] is True
