@@ -18,6 +18,7 @@ import torch.nn.functional as F
 
 from . import _lib
 from .decode import DecodeLayer
+from .extension._planes import observed
 
 __all__ = ["LlamaConfig", "LlamaDecoder"]
 
@@ -57,6 +58,12 @@ def _rope(x, tables):
     D = x.shape[-1]
     swapped = torch.cat([x[..., D // 2:], x[..., :D // 2]], -1)
     return torch.addcmul(x.float() * cos, swapped.float(), sin).to(x.dtype)
+
+
+def _plain(x: torch.Tensor) -> bool:
+    """Whether the library may take x's values as they lie in memory: contiguous fp16 on a 16-byte boundary, and nothing in force
+    that has to see tensor operations or computes them in another type."""
+    return not observed() and type(x) is torch.Tensor and x.dtype == torch.half and x.is_contiguous() and x.data_ptr() % 16 == 0
 
 
 class LlamaDecoder:
@@ -133,7 +140,7 @@ class LlamaDecoder:
         H, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         B = x.shape[0]
         qkv = F.linear(_rms_norm(x, p["norm1"], cfg.rms_norm_eps), p["wqkv"]).view(B, 1, H + 2 * Hkv, D)
-        if D % 16 or D > 256:
+        if D % 16 or D > 256 or not _plain(qkv):
             qk = _rope(qkv[:, :, :H + Hkv], _rope_tables(pos, D, cfg.rope_theta))
             return qk[:, :, :H].contiguous(), qk[:, :, H:].contiguous(), qkv[:, :, H + Hkv:].contiguous()
         q, k, v = (torch.empty(B, 1, n, D, dtype=torch.half, device=x.device) for n in (H, Hkv, Hkv))
@@ -147,7 +154,7 @@ class LlamaDecoder:
         B, Fi = x.shape[0], cfg.intermediate_size
         x = torch.addmm(x.view(B, -1), o.reshape(B, -1), p["wo"].t()).view(B, 1, -1)
         gate_up = F.linear(_rms_norm(x, p["norm2"], cfg.rms_norm_eps), p["w_gate_up"])
-        if Fi % 8:
+        if Fi % 8 or not _plain(gate_up):
             gate, up = gate_up.chunk(2, dim=-1)
             h = F.silu(gate).mul_(up).view(B, -1)
         else:

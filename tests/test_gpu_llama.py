@@ -95,3 +95,18 @@ def test_step_is_that_of_tensor_operations(akv_lib, E, Fi, H, Hkv, B):
             want = tensor_step(decs[2], ids[:, S + t])
             for dec in decs[:2]:
                 assert torch.equal(dec.step(ids[:, S + t]).view(torch.int16), want.view(torch.int16))
+
+
+def test_step_under_autocast(akv_lib):
+    """Autocast's type is what the products come out in: fp16 as without it, bf16 is refused by the cache, not misread."""
+    from alignedkv_b200.llama import LlamaConfig, LlamaDecoder
+    cfg = LlamaConfig(hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=4,
+                      vocab_size=1000)
+    ids = torch.randint(0, cfg.vocab_size, (2, 71), device="cuda", generator=torch.Generator(device="cuda").manual_seed(9))
+    a, b = (LlamaDecoder(cfg, 2, 128, "cuda:0", seed=4) for _ in range(2))
+    for dec in (a, b):
+        dec.prefill(ids[:, :70])
+    with torch.no_grad(), torch.autocast("cuda", torch.float16):
+        assert torch.equal(a.step(ids[:, 70]), tensor_step(b, ids[:, 70]))
+    with torch.autocast("cuda", torch.bfloat16), pytest.raises(RuntimeError, match="fp16"):
+        a.step(ids[:, 70])
