@@ -53,19 +53,19 @@ rope_split_kernel(const uint16_t* __restrict__ qkv, const long long* __restrict_
 
 __global__ void __launch_bounds__(128)
 silu_mul_kernel(const uint16_t* __restrict__ gate_up, uint16_t* __restrict__ out, int F) {
-    const int i = (blockIdx.x * 128 + threadIdx.x) * 8;
-    const size_t row = blockIdx.y;
-    if (i >= F) return;
-    const uint4 g4 = *reinterpret_cast<const uint4*>(gate_up + row * 2 * F + i);
-    const uint4 u4 = *reinterpret_cast<const uint4*>(gate_up + row * 2 * F + F + i);
-    uint4 o4;
+    const size_t row = blockIdx.x;
+    const uint16_t *gate = gate_up + row * 2 * F, *up = gate + F;
+    for (int i = (blockIdx.y * 128 + threadIdx.x) * 8; i < F; i += gridDim.y * 1024) {
+        const uint4 g4 = *reinterpret_cast<const uint4*>(gate + i), u4 = *reinterpret_cast<const uint4*>(up + i);
+        uint4 o4;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float2 g = __half22float2(reinterpret_cast<const __half2*>(&g4)[j]);
-        const __half2 a = __floats2half2_rn(g.x / (1.f + expf(-g.x)), g.y / (1.f + expf(-g.y)));
-        reinterpret_cast<__half2*>(&o4)[j] = __hmul2(a, reinterpret_cast<const __half2*>(&u4)[j]);
+        for (int j = 0; j < 4; ++j) {
+            const float2 g = __half22float2(reinterpret_cast<const __half2*>(&g4)[j]);
+            const __half2 a = __floats2half2_rn(g.x / (1.f + expf(-g.x)), g.y / (1.f + expf(-g.y)));
+            reinterpret_cast<__half2*>(&o4)[j] = __hmul2(a, reinterpret_cast<const __half2*>(&u4)[j]);
+        }
+        *reinterpret_cast<uint4*>(out + row * F + i) = o4;
     }
-    *reinterpret_cast<uint4*>(out + row * F + i) = o4;
 }
 
 // One CTA per row, its values in registers between the sum and the scaling: one pass over memory, one reduction.
@@ -146,11 +146,12 @@ int akv_rope_split(const void* qkv, const void* pos, void* q, void* k, void* v, 
 int akv_silu_mul(const void* gate_up, void* out, int rows, int width, void* stream) {
     set_error("");
     AKV_REQUIRE(gate_up && out, AKV_ERR_NULL, "silu_mul: null pointer");
-    AKV_REQUIRE(rows > 0 && rows <= 65535 && width > 0 && width % 8 == 0 && width <= (1 << 30), AKV_ERR_SHAPE,
+    AKV_REQUIRE(rows > 0 && width > 0 && width % 8 == 0 && width <= (1 << 30), AKV_ERR_SHAPE,
                 "silu_mul: unsupported extent (%d rows of %d [multiple of 8])", rows, width);
     AKV_REQUIRE(aligned16(gate_up) && aligned16(out), AKV_ERR_ALIGN, "silu_mul: pointers must be 16-byte aligned");
     count_launch();
-    silu_mul_kernel<<<dim3((width / 8 + 127) / 128, rows), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const int across = (width / 8 + 127) / 128;
+    silu_mul_kernel<<<dim3(rows, across < 65535 ? across : 65535), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint16_t*>(gate_up), static_cast<uint16_t*>(out), width);
     return cuda_status(cudaGetLastError(), "silu_mul launch");
 }

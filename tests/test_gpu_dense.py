@@ -47,8 +47,33 @@ def test_silu_mul(rows, width):
     call("akv_silu_mul", x.data_ptr(), out.data_ptr(), rows, width)
     gate, up = x.chunk(2, dim=-1)
     want = F.silu(gate) * up
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     fin = want.isfinite()
-    assert torch.equal(fin, out.isfinite()) and close(out[fin], want[fin], 2)
+    assert close(out[fin].float(), (gate.double() * torch.sigmoid(gate.double())).half().double().mul(up.double())[fin].float(), 2)
+
+
+def test_silu_of_every_value():
+    """Every fp16 gate, NaN and infinities among them, against the tensor operations bit for bit and against 64 bits."""
+    gate = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.half)
+    for up in (1.0, 0.3333, -1000.0, 65504.0, torch.inf, torch.nan, 1e-7):
+        x = torch.stack([gate, torch.full_like(gate, up)])
+        out = torch.empty_like(gate)
+        call("akv_silu_mul", x.data_ptr(), out.data_ptr(), 1, gate.numel())
+        want = F.silu(x[0]).mul_(x[1])
+        assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out[~want.isnan()], want[~want.isnan()])
+        if up == 1.0:
+            d = gate.double()
+            fin = d.isfinite()
+            exact = (d / (1 + torch.exp(-d)))[fin]
+            # (one rounding of an fp32 quotient that is off by a few fp32 steps; gates whose exponential overflows give -0)
+            assert bool(((out[fin].double() - exact).abs() <= (2.0 ** -11 + 2.0 ** -20) * exact.abs() + 2.0 ** -25).all())
+
+
+def test_silu_of_many_rows():
+    x = rand(70000, 16, seed=3)
+    out = torch.empty(70000, 8, dtype=torch.half, device="cuda")
+    call("akv_silu_mul", x.data_ptr(), out.data_ptr(), 70000, 8)
+    assert torch.equal(out, F.silu(x[:, :8]) * x[:, 8:])
 
 
 @pytest.mark.parametrize("rows,width", [(1, 8), (2, 520), (16, 4096), (3, 8192), (2, 16384), (64, 4104)])
