@@ -64,6 +64,8 @@ class DecodeLayer:
             raise ValueError("bad extents")
         self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         self._sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
+        m, l = self.k_mid_4, self.k_last_4
+        self._nibbles = None if m.is_inference() else (m.data_ptr(), l.data_ptr(), m._version, l._version)
         self._desc = None                    # `_lib.Layer`, made by the first step
         self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self._q_shape, self._kv_shape = (bsz, 1, self.Hq, head_dim), (bsz, 1, n_heads, head_dim)
@@ -82,6 +84,14 @@ class DecodeLayer:
     def _flags(self, append: bool = True) -> int:
         return (AKV_STEP_REFERENCE if getattr(self, "reference", False) else 0) | \
                (AKV_STEP_ORDER_FREE if self.v_mode == "order_free" else 0) | (0 if append else AKV_STEP_NO_APPEND)
+
+    def _nibbles_known(self) -> bool:
+        """Whether no tensor operation has touched the K nibble planes since they were made: they have the addresses and version
+        counters they had then (False where versions are not kept, inference tensors).  What AKV_PREFILL_STORE asks for is more: a
+        writer that has a tensor's address (`cuda_module.k_cache_save`, `.data`, DLPack) leaves the counter alone, so `prefill` adds."""
+        m, l, was = self.k_mid_4, self.k_last_4, self._nibbles
+        return was is not None and m.data_ptr() == was[0] and l.data_ptr() == was[1] and not m.is_inference() and \
+            not l.is_inference() and m._version == was[2] and l._version == was[3]
 
     # ------------------------------------------------------------------ prompt
     def prefill(self, k: torch.Tensor, v: torch.Tensor) -> None:

@@ -47,6 +47,18 @@ def test_silu_mul(rows, width):
     call("akv_silu_mul", x.data_ptr(), out.data_ptr(), rows, width)
     gate, up = x.chunk(2, dim=-1)
     want = F.silu(gate) * up
+    fin = want.isfinite()
+    assert torch.equal(fin, out.isfinite()) and close(out[fin], want[fin], 2)
+
+
+@pytest.mark.parametrize("rows,width", [(1, 8), (3, 1032), (16, 11008), (7, 14336)])
+def test_silu_mul_is_the_tensor_operations(rows, width):
+    x = rand(rows, 2 * width, seed=width, scale=3.0)
+    x[0, 0], x[0, 1] = -60000.0, 60000.0
+    out = torch.empty(rows, width, dtype=torch.half, device="cuda")
+    call("akv_silu_mul", x.data_ptr(), out.data_ptr(), rows, width)
+    gate, up = x.chunk(2, dim=-1)
+    want = F.silu(gate) * up
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     fin = want.isfinite()
     assert close(out[fin].float(), (gate.double() * torch.sigmoid(gate.double())).half().double().mul(up.double())[fin].float(), 2)

@@ -29,12 +29,15 @@ def inputs(B, H, D, S):
 @pytest.mark.parametrize("B,H,D,S", [(1, 1, 128, 64), (2, 3, 128, 130), (3, 8, 128, 63), (2, 2, 64, 200), (1, 4, 128, 1027)])
 def test_store_and_add(B, H, D, S):
     from alignedkv_b200.decode import DecodeLayer
-    k, v, q = inputs(B, H, D, S)
+    g = torch.Generator(device="cuda").manual_seed(S)
+    k, v, q = (torch.randn(B, n, H, D, device="cuda", generator=g).half() for n in (S, S, 1))
     make = lambda: DecodeLayer(B, -(-(S + 70) // 64) * 64, H, D, "cuda:0")  # noqa: E731
     stored, added, dirty = make(), make(), make()
+    assert stored._nibbles_known()
+    added.k_mid_4.add_(0)                                  # a tensor operation: the layer can no longer know
+    assert not added._nibbles_known()
     dirty.k_mid_4.fill_(1)
-    assert call_ex(stored, k, v, 1) == 0
-    for layer in (added, dirty):
+    for layer in (stored, added, dirty):
         layer.prefill(k, v)
     for a, b in zip(planes(stored), planes(added)):
         assert torch.equal(a, b)
@@ -52,6 +55,18 @@ def test_store_and_add(B, H, D, S):
     empty.prefill(k, v)
     for a, b in zip(planes(empty)[:3], planes(stored)[:3]):
         assert torch.equal(a[:, :, :n], b[:, :, :n])
+
+
+@pytest.mark.parametrize("B,H,D,S", [(1, 1, 128, 64), (2, 3, 128, 130), (3, 8, 128, 63), (2, 2, 64, 200), (1, 4, 128, 1027)])
+def test_store_on_request(B, H, D, S):
+    """AKV_PREFILL_STORE on planes that are zero leaves what adding leaves."""
+    from alignedkv_b200.decode import DecodeLayer
+    k, v, _ = inputs(B, H, D, S)
+    stored, added = (DecodeLayer(B, -(-(S + 70) // 64) * 64, H, D, "cuda:0") for _ in range(2))
+    assert call_ex(stored, k, v, 1) == 0
+    added.prefill(k, v)
+    for a, b in zip(planes(stored), planes(added)):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -82,6 +97,14 @@ def test_adds_onto_what_others_wrote(D, writer):
 
 
 def test_inference_tensors_add():
+    from alignedkv_b200.decode import DecodeLayer
+    with torch.inference_mode():
+        layer = DecodeLayer(1, 128, 1, 128, "cuda:0")
+        assert not layer._nibbles_known()
+        layer.prefill(torch.randn(1, 100, 1, 128, device="cuda").half(), torch.randn(1, 100, 1, 128, device="cuda").half())
+
+
+def test_inference_tensors_add_the_same():
     from alignedkv_b200.decode import DecodeLayer
     k, v, _ = inputs(1, 1, 128, 100)
     clean = DecodeLayer(1, 128, 1, 128, "cuda:0")
