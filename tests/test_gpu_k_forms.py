@@ -71,3 +71,45 @@ def test_overlapped_steps(akv_lib, B, H, G, D, P, mode, append):
         outs.append(torch.stack(o + [layer.k_exp_max.float().mean().half().expand_as(o[0])]))
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
     assert akv_lib.akv_device_error_flag() == 0
+
+
+# rows of more than 17408 scores (few: the split softmax with P.V's first stages requested in front of its end; many: three passes
+# and a probe of their own), a padded batch, a step that flushes among them
+@pytest.mark.parametrize("B,H,G,P,T,mode,packed,masked", [(1, 3, 1, 17500, 4, "order_free", True, False),
+                                                          (1, 3, 1, 17500, 38, "exact", False, False),
+                                                          (2, 2, 4, 17470, 3, "exact", True, False),
+                                                          (75, 1, 4, 24576, 2, "exact", False, False),
+                                                          (75, 4, 1, 24570, 8, "order_free", True, False),
+                                                          (5, 8, 4, 700, 6, "exact", False, True),
+                                                          (3, 4, 1, 16440, 3, "exact", False, True)])
+def test_overlapped_steps_leave_the_same(akv_lib, B, H, G, P, T, mode, packed, masked):
+    """Everything that a run of steps returns and leaves behind, with and without overlapped launches."""
+    from alignedkv_b200.decode import DecodeLayer
+    D = 128
+    g = torch.Generator(device="cuda").manual_seed(P + B)
+    r = lambda *s: torch.randn(*s, D, device="cuda", generator=g).half()  # noqa: E731
+    k, v, q, k1, v1 = r(B, P, H), r(B, P, H), r(T, B, 1, H * G), r(T, B, 1, H), r(T, B, 1, H)
+    k[..., [3, 34]] *= 20
+    k1 *= torch.linspace(0.2, 9.0, T, device="cuda").view(T, 1, 1, 1, 1)
+    v1 *= torch.linspace(1.0, 30.0, T, device="cuda").view(T, 1, 1, 1, 1)                  # the maxima grow under way
+    L = -(-(P + T) // 64) * 64
+    mask = None
+    if masked:
+        mask = torch.zeros(B, 1, 1, L, device="cuda", dtype=torch.half)
+        mask[0, ..., :P // 3] = torch.finfo(torch.half).min
+    seen = []
+    for pdl in (0, 1):
+        assert akv_lib.akv_set_tuning(b"pdl", pdl) == 0
+        try:
+            layer = DecodeLayer(B, L, H, D, "cuda:0", n_q_heads=H * G, v_mode=mode)
+            layer.prefill(k, v)
+            out = [layer.decode(q[t], k1[t], v1[t], packed=packed, mask=mask) for t in range(T)]
+            torch.cuda.synchronize()
+        finally:
+            akv_lib.akv_set_tuning(b"pdl", 1)
+        n = layer.rest_len
+        seen.append(out + [layer.restk[:, :n], layer.restv[:, :n], layer.k_exp_max, layer.v_exp_max, layer.k_first_8, layer.k_mid_4,
+                           layer.k_last_4] + [t[:, :, :layer.rest_start] for t in (layer.v_first_8, layer.v_mid_4, layer.v_last_4)])
+    for a, b in zip(*seen):
+        assert torch.equal(a, b) and bool(a.count_nonzero() or not a.numel())
+    assert akv_lib.akv_device_error_flag() == 0
