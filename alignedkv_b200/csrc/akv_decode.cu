@@ -1223,10 +1223,10 @@ static int decode_step_impl(void* k_first_8, void* k_mid_4, void* k_last_4, void
     }
     // Rows split across CTAs when they are few and long (softmax_chunk_*); one CTA per row, held in registers, when it has at
     // most 24576 scores; else one CTA in three passes.  (The split form's chunk grid is part of the sequence-sharded
-    // protocol: the line between it and the others stays where it is.)  Many rows of residual tokens only take the three
-    // passes too: 64 scores are a fraction of the registers' form (13.5 KB of shared memory and the probe's apparatus per row);
-    // a step of 768 / 1760 / 4096 rows of 2 tokens 12.8 / 22.0 / 46.0 us against 14.6 / 24.5 / 51.6.  With few rows (32 / 512:
-    // 8.7 / 14.8 against 7.9 / 12.0) it is the other way round: that form's loads go out together.
+    // protocol: the line between it and the others stays where it is.)  A step without a quantized block comes here only with
+    // head sizes above 256, with the exchange, or with an empty cache (the others are small_step_kernel's): few rows take the
+    // registers' form, whose loads go out together, many the three passes, since 64 scores are a fraction of that form (13.5 KB of
+    // shared memory and the probe's apparatus per row).
     const int sm_chunks = (R + SM_CHUNK - 1) / SM_CHUNK;
     const int rows = B * H * G;
     const bool split = R > 17408 && rows < 2 * sm_count();

@@ -7,12 +7,12 @@
 //
 // Design (B200): the kernel is a pure HBM stream.  Each WARP owns a private ring of shared-memory stages that
 // it fills with 16-byte asynchronous copies and drains itself - no block-level barrier exists.  A warp works
-// through a contiguous run of units; a unit is 4 consecutive 64-token blocks of one (batch, KV head), and a stage
-// holds KCH channels of those 4 blocks: the high-byte rows plus, only for the channels whose alignment code
-// asks for them, the 32-byte rows of the mid / low nibble planes (rows that are skipped are never requested
-// from memory).  Lane (tile, i) owns tokens 8i..8i+7 of its tile and keeps four fp16x2 accumulators per query head:
-// one 8-byte and two 4-byte shared loads feed four FMAs, and no cross-lane reduction exists, which is what keeps the
-// channel-order fp16 sum exact.
+// through a contiguous run of units; a unit is 4 consecutive 64-token blocks of one (batch, KV head), or one block (few blocks
+// and groups of four or eight, see the launcher), and a stage holds KCH channels of the unit's blocks: the high-byte rows plus,
+// only for the channels whose alignment code asks for them, the 32-byte rows of the mid / low nibble planes (rows that are
+// skipped are never requested from memory).  With four blocks lane (tile, i) owns tokens 8i..8i+7 of its tile and keeps four
+// fp16x2 accumulators per query head: one 8-byte and two 4-byte shared loads feed four FMAs; with one block it owns tokens
+// 2i, 2i+1 and one accumulator.  No cross-lane reduction exists, which is what keeps the channel-order fp16 sum exact.
 // Grouped-query attention (G query heads per KV head): a row is fetched when ANY head of the group needs it, every
 // staged row is read from shared memory once and applied to the G heads in turn, each head substituting the
 // reference's constants where its own code skips the plane - so plane bytes cross HBM once per group and the

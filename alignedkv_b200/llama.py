@@ -173,7 +173,7 @@ class LlamaDecoder:
         (embedding + layer 0 up to its attention; the rest of layer i + layer i+1 up to its attention; the rest of the
         last layer + final norm + logits).  The attention calls stay ordinary launches between the replays - the
         cache's state (residual length, block count) changes from token to token and is passed by value.  After this,
-        `step` replays: ~35 torch launches per layer become one graph launch, which is what the step was bound by."""
+        `step` replays: the eight launches of a layer's dense parts become one graph launch."""
         assert self.attention == "alignedkv", "only the AlignedKV path is split into graphs"
         cfg, B, dev = self.cfg, self.B, self.device
         H, D, n = cfg.num_attention_heads, cfg.head_dim, cfg.num_hidden_layers
