@@ -113,3 +113,33 @@ def test_overlapped_steps_leave_the_same(akv_lib, B, H, G, P, T, mode, packed, m
     for a, b in zip(*seen):
         assert torch.equal(a, b) and bool(a.count_nonzero() or not a.numel())
     assert akv_lib.akv_device_error_flag() == 0
+
+
+@pytest.mark.parametrize("B,H,G,D,P", [(2, 3, 1, 128, 640), (1, 4, 1, 64, 192), (1, 2, 2, 128, 320), (2, 4, 4, 128, 3968), (40, 4, 4, 128, 1088),
+                                       (1, 3, 4, 256, 64), (2, 2, 8, 128, 448), (1, 2, 1, 256, 320)])
+@pytest.mark.parametrize("append", [True, False])
+def test_own_alignment_inputs(akv_lib, B, H, G, D, P, append):
+    """A step whose q.K^T makes its alignment inputs from query, exponent maxima and new token, against one that takes the append
+    kernel's: K planes off a 16-byte boundary go to the kernel that has no form of its own for them."""
+    from alignedkv_b200.decode import DecodeLayer
+    g = torch.Generator(device="cuda").manual_seed(P + D)
+    r = lambda *s: torch.randn(*s, D, device="cuda", generator=g)  # noqa: E731
+    spread = 2.0 ** torch.randint(-7, 3, (H, D), device="cuda", generator=g)
+    k, v, v1 = (r(B, P, H) * spread).half(), r(B, P, H).half(), r(B, 1, H).half()
+    k1 = (r(B, 1, H) * spread * 2.0 ** torch.randint(-6, 7, (B, 1, H, D), device="cuda", generator=g)).half()   # some maxima are the token's
+    q = (r(B, 1, H * G) * 2.0 ** torch.randint(-5, 3, (B, 1, H * G, D), device="cuda", generator=g)).half()
+    outs = []
+    for off in (0, 8):
+        layer = DecodeLayer(B, P + 64, H, D, "cuda:0", n_q_heads=H * G)
+        layer.prefill(k, v)
+        if off:
+            for name in ("k_first_8", "k_mid_4", "k_last_4"):
+                t = getattr(layer, name)
+                at = torch.empty(t.numel() + off, dtype=torch.uint8, device="cuda")[off:].view(t.shape)
+                setattr(layer, name, at.copy_(t))
+                assert at.data_ptr() % 16 == off
+        o = layer.decode(q, k1, v1) if append else layer.decode(q, append=False)
+        outs.append([o, layer.k_exp_max, layer.v_exp_max])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    assert bool(outs[0][0].count_nonzero())
