@@ -23,8 +23,9 @@
 // integer pipe and 16 FMAs for four heads; parking the low bytes of each code in shared memory and fetching them back per
 // head, which this replaces, took 80 instructions: groups of eight 253 against
 // 177 us at batch 64 x 4 KV heads x 8192 tokens, of two 56 against 46 at batch 16 x 16 x 4096, of four 41.5 against 35.5 at
-// batch 8 x 8 x 8192 but 228 against 223 at batch 64, where the copies are what is left (a stage's issue stalls for 450 to
-// 770 cycles on the load unit; neither bulk copies nor TMA boxes, built and bit-exact, moved these pieces faster).
+// batch 8 x 8 x 8192 but 228 against 223 at batch 64 (198 since the head size is known at compile time, see the kernel), where the
+// copies are what is left (a stage's issue stalls for 450 to 770 cycles on the load unit; neither bulk copies nor TMA boxes, built
+// and bit-exact, moved these pieces faster).
 // With G == 1 the producer writes the constants into the skipped rows' slots instead.
 // In a decode step that flushes no block the kernel makes its alignment inputs itself and runs beside the append kernel in front of
 // it (KParams::k_exp): batch 8 x 32 heads x 4096 tokens 80.5 -> 78.7 us per step, 16 x 32 x 1000 56.6 -> 53.0, one sequence of
